@@ -11,7 +11,7 @@
 
 namespace sw2d {
 
-cudaError_t prepare_step(int th, int tw, float) {
+cudaError_t prepare_step(int th, int tw) {
     if (th == 16 && tw == 32) return detail::step_prepare<float, 16, 32, 256>();
     if (th == 32 && tw == 32) return detail::step_prepare<float, 32, 32, 256>();
     if (th == 16 && tw == 64) return detail::step_prepare<float, 16, 64, 256>();

@@ -1,35 +1,82 @@
-// step_f64.cu -- FP64 instantiations.  Compiled with --fmad=false: every
+// step_f64.cu -- FP64 kernels.  Compiled with --fmad=false: every
 // multiply and add rounds separately, as in the serial oracle and in the
 // reference built without contraction, which makes the FP64 path
 // bit-reproducible against them wherever no transcendental is involved.
 #define SW2D_REAL double
 #include "sw2d_launch_impl.cuh"
+#include "sw2d_step64.cuh"
 
 namespace sw2d {
 
 // Fills this translation unit's tables of the deterministic log/exp (on the
 // legacy stream, waited for: the handles' own streams do not order with it).
 cudaError_t init_det_tables() {
-    det_tables_kernel<<<1, 128>>>();
+    pow_tables_kernel<<<2 * kPowN / 256, 256>>>();
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     return cudaStreamSynchronize(0);
 }
 
-cudaError_t prepare_step(int th, int tw, double) {
+// Builds of the step kernel: (tile rows, tile columns, threads, minimum
+// resident CTAs per SM).  16 x 32 with 384 threads and two CTAs per SM: 526 us
+// per iteration on a 1013 x 900 catchment, against 557 with 256 threads (the
+// integer stages run at too few warps), 525 with 512, and 550 with a 32 x 32
+// tile (less halo, but one CTA per SM idles at its barriers).
+#define SW2D_STEP64_TILES(X) X(16, 32, 384, 2) X(8, 32, 256, 3)
+
+cudaError_t prepare_step64(int th, int tw) {
     const cudaError_t e = init_det_tables();
     if (e != cudaSuccess) return e;
-    if (th == 16 && tw == 32) return detail::step_prepare<double, 16, 32, 256>();
-    if (th == 8 && tw == 32) return detail::step_prepare<double, 8, 32, 128>();
+#define SW2D_P64(h, w, nt, mb)                                                                                  \
+    if (th == h && tw == w) {                                                                                   \
+        const cudaError_t e2 = cudaFuncSetAttribute(step64_kernel<h, w, nt, mb>,                                \
+                                                    cudaFuncAttributeMaxDynamicSharedMemorySize,                \
+                                                    (int)Step64Shape<h, w>::kSmem);                            \
+        if (e2 != cudaSuccess) return e2;                                                                       \
+        return cudaFuncSetAttribute(step64_kernel<h, w, nt, mb>, cudaFuncAttributePreferredSharedMemoryCarveout, \
+                                    (int)cudaSharedmemCarveoutMaxShared);                                       \
+    }
+    SW2D_STEP64_TILES(SW2D_P64)
+#undef SW2D_P64
     return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_step(int th, int tw, int nblocks, const GridDesc &G, const ForcingDesc &F,
-                        const StateBufs<double> &S, const Thr<double> &T, Clock *clk, const Control *ctl, int slot,
-                        cudaStream_t st) {
-    if (th == 16 && tw == 32) return detail::step_launch<double, 16, 32, 256>(nblocks, G, F, S, T, clk, ctl, slot, st);
-    if (th == 8 && tw == 32) return detail::step_launch<double, 8, 32, 128>(nblocks, G, F, S, T, clk, ctl, slot, st);
+cudaError_t launch_step64(int th, int tw, int nblocks, int sms, const GridDesc &G, const ForcingDesc &F,
+                          const StateBufs<double> &S, const Thr<double> &T, const double *gnx, const double *gny,
+                          Clock *clk, const Control *ctl, int slot, cudaStream_t st) {
+    Step64Extra X;
+    X.gnx = gnx;
+    X.gny = gny;
+    X.gn = G.sd.g * G.sd.manning * G.sd.manning;
+    X.rdx = G.sd.rdx;
+    X.rdy = G.sd.rdy;
+    // a programmatic dependent of the launch before it (step64_kernel, stage 0)
+    // where one CTA per SM holds the grid: 53.5 against 55.9 us on 64 x 64.  With
+    // more, the early CTAs crowd the SMs that drain first (256 CTAs of 8 x 32:
+    // 91 against 72 us).
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = nblocks <= sms ? 1 : 0;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(nblocks);
+    lc.stream = st;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+#define SW2D_L64(h, w, nt, mb)                                                                             \
+    if (th == h && tw == w) {                                                                              \
+        lc.blockDim = dim3(nt);                                                                            \
+        lc.dynamicSmemBytes = Step64Shape<h, w>::kSmem;                                                    \
+        return cudaLaunchKernelEx(&lc, step64_kernel<h, w, nt, mb>, G, F, S, T, X, clk, ctl, slot);        \
+    }
+    SW2D_STEP64_TILES(SW2D_L64)
+#undef SW2D_L64
     return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_pack_gn(const double *n, int rows, int cols, int pitch, double g, double *gnx, double *gny,
+                           cudaStream_t st) {
+    pack_gn_kernel<<<detail::grid_for((long long)rows * cols, 256), 256, 0, st>>>(n, rows, cols, pitch, g, gnx, gny);
+    return cudaGetLastError();
 }
 
 }  // namespace sw2d

@@ -39,12 +39,14 @@ struct sw2d_handle {
     size_t plane = 0;   // elements per allocated array, frame included
     size_t origin = 0;  // element offset of cell (0,0) in an allocation
     int tile_h = 16, tile_w = 32, nblocks = 0;
+    int sms = 152;
     bool stream_kernel = false;  // FP32 warp-streaming kernel instead of the tile kernel
     int strip_h = 0, stream_tiles_w = 0, stream_units = 0, variant = 0;
     int strip_skew = 0;  // percent by which strip heights fall from the first strip to the last
     cudaStream_t stream = nullptr;
     void *h[2] = {nullptr, nullptr}, *um[2] = {nullptr, nullptr}, *vn[2] = {nullptr, nullptr};
-    void *z = nullptr, *nman = nullptr;
+    void *z = nullptr, *nman = nullptr;  // nman: FP32 only
+    double *gnx = nullptr, *gny = nullptr;  // g n^2 per face (FP64 with a Manning raster; one allocation, gnx first)
     uint8_t *mask = nullptr;
     void *rainw = nullptr;  // spatial rain factors (allocated on first use)
     void *dzx = nullptr, *dzy = nullptr;  // bed differences across faces (streaming kernel)
@@ -97,6 +99,10 @@ int cuda_fail(sw2d_handle *h, cudaError_t e, const char *what) {
         cudaError_t e_ = (expr);                                \
         if (e_ != cudaSuccess) return cuda_fail((h), e_, #expr); \
     } while (0)
+
+// One-iteration launches of every kernel but the FP32 tile kernel defer the
+// budget fold.
+bool defers_fold(const sw2d_handle *h) { return h->stream_kernel || h->cfg.precision == SW2D_PREC_F64; }
 
 bool is_f64(const sw2d_handle *h) { return h->cfg.precision == SW2D_PREC_F64; }
 
@@ -153,8 +159,9 @@ cudaError_t launch_one(sw2d_handle *h, int slot) {
                                   h->strip_skew, h->G, h->F,
                                   make_bufs<float>(h), make_thr<float>(h->cfg), h->d_clk, h->d_ctl, slot, h->stream);
     if (is_f64(h))
-        return launch_step(h->tile_h, h->tile_w, h->nblocks, h->G, h->F, make_bufs<double>(h),
-                           make_thr<double>(h->cfg), h->d_clk, h->d_ctl, slot, h->stream);
+        return launch_step64(h->tile_h, h->tile_w, h->nblocks, h->sms, h->G, h->F, make_bufs<double>(h),
+                             make_thr<double>(h->cfg), h->has_nraster ? h->gnx : nullptr,
+                             h->has_nraster ? h->gny : nullptr, h->d_clk, h->d_ctl, slot, h->stream);
     return launch_step(h->tile_h, h->tile_w, h->nblocks, h->G, h->F, make_bufs<float>(h),
                        make_thr<float>(h->cfg), h->d_clk, h->d_ctl, slot, h->stream);
 }
@@ -204,10 +211,10 @@ void grid_shape(const sw2d_config *c, int *pitch, size_t *plane, int *th, int *t
 
 int read_clock(sw2d_handle *h) {
     const int slot = (int)(h->launches % 3);
-    // the streaming kernel leaves the budget fold of the slot its last
-    // launch wrote to the next launch (finish_cta_deferred_warp): fold it
+    // the streaming and FP64 kernels leave the budget fold of the slot their
+    // last launch wrote to the next launch (finish_cta_deferred_warp): fold it
     // here (a fold is idempotent)
-    if (h->stream_kernel && h->fold_needed && h->have_state) {
+    if (defers_fold(h) && h->fold_needed && h->have_state) {
         fold_kernel<<<1, 32, 0, h->stream>>>(h->d_clk, slot, (slot + 2) % 3);
         CK(h, cudaGetLastError());
         h->kernels++;
@@ -356,7 +363,9 @@ int sw2d_device_bytes(const sw2d_config *c, int64_t *bytes) {
     grid_shape(c, &pitch, &plane, &th, &tw);
     const size_t rs = c->precision == SW2D_PREC_F64 ? 8 : 4;
     const bool stream = c->precision == SW2D_PREC_F32 && c->kernel != SW2D_KERNEL_TILE;
-    size_t total = plane * rs * (stream ? 12 : 8);  // 2x(h, um, vn) + z + n (+ dzx, dzy, 2x remainder), frame included
+    // 2x(h, um, vn) + z, frame included, and: n (FP32), dzx, dzy, 2x remainder (streaming kernel), g n^2 of the
+    // two faces (FP64)
+    size_t total = plane * rs * (stream ? 12 : (rs == 8 ? 9 : 8));
     total += plane;                 // mask
     total += 2 * (size_t)(c->rows + 1) * (c->cols + 1) * sizeof(double);  // staging
     total += kVolumeBlocks * sizeof(double) + 3 * sizeof(Clock) + sizeof(Control);
@@ -382,6 +391,8 @@ int sw2d_create(const sw2d_config *cfg, sw2d_handle **out) {
     cudaError_t e = cudaSetDevice(cfg->device);
     if (e != cudaSuccess) return bail(SW2D_ERR_CUDA);
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(SW2D_ERR_CUDA);
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg->device) == cudaSuccess && sms > 0) h->sms = sms;
     const size_t fb = h->plane * h->real_size;
     // allocate with the zero frame, keep pointers at cell (0,0)
     auto alloc_field = [&](void **p, size_t esz) -> bool {
@@ -396,9 +407,8 @@ int sw2d_create(const sw2d_config *cfg, sw2d_handle **out) {
         for (void **a : arrs)
             if (!alloc_field(a, h->real_size)) return bail(SW2D_ERR_OOM);
     }
-    if (!alloc_field(&h->z, h->real_size) || !alloc_field(&h->nman, h->real_size) ||
-        !alloc_field((void **)&h->mask, 1))
-        return bail(SW2D_ERR_OOM);
+    if (!alloc_field(&h->z, h->real_size) || !alloc_field((void **)&h->mask, 1)) return bail(SW2D_ERR_OOM);
+    if (!is_f64(h) && !alloc_field(&h->nman, h->real_size)) return bail(SW2D_ERR_OOM);
     (void)fb;
     h->stage_elems = (size_t)(cfg->rows + 1) * (cfg->cols + 1);
     if (cudaMalloc((void **)&h->stage, h->stage_elems * sizeof(double)) != cudaSuccess) return bail(SW2D_ERR_OOM);
@@ -418,7 +428,7 @@ int sw2d_create(const sw2d_config *cfg, sw2d_handle **out) {
     if (h->stream_kernel) {
         e = prepare_stream_step(h->variant);
     } else {
-        e = is_f64(h) ? prepare_step(h->tile_h, h->tile_w, 0.0) : prepare_step(h->tile_h, h->tile_w, 0.0f);
+        e = is_f64(h) ? prepare_step64(h->tile_h, h->tile_w) : prepare_step(h->tile_h, h->tile_w);
     }
     if (e != cudaSuccess) return bail(SW2D_ERR_CUDA);
 
@@ -521,6 +531,7 @@ int sw2d_destroy(sw2d_handle *h) {
     }
     free_field(h->z, h->real_size);
     free_field(h->nman, h->real_size);
+    free_field(h->gnx, h->real_size);  // and gny
     free_field(h->mask, 1);
     free_field(h->rainw, h->real_size);
     free_field(h->dzx, h->real_size);
@@ -554,10 +565,17 @@ int sw2d_set_static(sw2d_handle *h, const double *z, const double *manning) {
         CK(h, cudaMemcpyAsync(h->stage2, manning, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
         dn = h->stage2;
     }
-    if (is_f64(h))
-        CK(h, launch_pack_static(h->stage, dn, rows, cols, h->pitch, h->cfg.nodata, (double *)h->z,
-                                 dn ? (double *)h->nman : nullptr, h->mask, h->stream));
-    else
+    if (is_f64(h)) {
+        CK(h, launch_pack_static(h->stage, dn, rows, cols, h->pitch, h->cfg.nodata, (double *)h->z, (double *)nullptr,
+                                 h->mask, h->stream));
+        if (dn && !h->gnx) {
+            void *p = nullptr;
+            CK(h, cudaMalloc(&p, 2 * h->plane * sizeof(double)));
+            h->gnx = static_cast<double *>(p) + h->origin;
+            h->gny = h->gnx + h->plane;
+        }
+        if (dn) CK(h, launch_pack_gn(dn, rows, cols, h->pitch, h->cfg.g, h->gnx, h->gny, h->stream));
+    } else
         CK(h, launch_pack_static(h->stage, dn, rows, cols, h->pitch, h->cfg.nodata, (float *)h->z,
                                  dn ? (float *)h->nman : nullptr, h->mask, h->stream));
     if (h->stream_kernel)
@@ -799,14 +817,14 @@ int sw2d_advance(sw2d_handle *h, int64_t max_steps, double t_end, int64_t *steps
             CK(h, cudaGraphLaunch(h->graph, h->stream));
             h->launches += kChunk;
             h->kernels += kChunk;
-            h->fold_needed = h->stream_kernel;
+            h->fold_needed = defers_fold(h);
         } else {
             const long long n = ((remaining + 2) / 3) * 3;
             for (long long m = 0; m < n; m++) {
                 CK(h, launch_one(h, (int)((h->launches) % 3)));
                 h->launches++;
                 h->kernels++;
-                h->fold_needed = h->stream_kernel;
+                h->fold_needed = defers_fold(h);
             }
         }
         int rc = read_clock(h);

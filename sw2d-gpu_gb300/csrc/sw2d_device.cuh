@@ -28,10 +28,9 @@
 // ends and the next launch can pick its time step without a grid-wide
 // synchronisation.
 //
-// The same template serves FP64 (compiled without FMA contraction, so that
-// every operation rounds exactly as in the serial oracle and the reference
-// built with --fmad=false) and FP32 (fast math).  Threshold tests are
-// written as `x >= c` against host-computed constants so that the FP32 path
+// It is instantiated for FP32 (fast math, SW2D_KERNEL_TILE); the FP64 path's
+// kernel, with the same decomposition, is step64_kernel (sw2d_step64.cuh).
+// Threshold tests are written as `x >= c` against host-computed constants so that the FP32 path
 // decides wet/dry exactly as an FP64 comparison with th = 1e-4 would.
 #pragma once
 
@@ -620,7 +619,7 @@ static __global__ void fold_kernel(Clock *__restrict__ clk, const int slot, cons
 // cu:312).  The update uses the table-driven forms: log with 1/c and ln c for
 // c = 1 + k/128 (k = the top 7 bits of the mantissa) and the series of
 // ln(1+r) to r^8/8; exp with a reduction by ln2/64, the series of e^r to
-// r^6/6! and 2^(j/64).  The tables are built by det_tables_kernel from the
+// r^6/6! and 2^(j/64).  The tables are built by det_tables_entry from the
 // series forms (log: atanh series on [1/sqrt2, sqrt2) to s^21/21; exp:
 // Cody-Waite by ln2, Taylor to r^13/13!) in each translation unit that uses
 // them (init_det_tables).
@@ -673,11 +672,11 @@ __device__ __forceinline__ double det_exp_series(double y) {
 }
 
 // [0,128): 1/c_k, [128,256): ln c_k, [256,320): 2^(j/64); one copy per
-// translation unit, filled by det_tables_kernel before the first use
+// translation unit, filled (det_tables_entry) before the first use
 static __device__ double g_det_tab[320];
 
-static __global__ void det_tables_kernel() {
-    const int t = threadIdx.x;
+// Entry t of each table (t < 128); every table entry is written by one thread.
+__device__ __forceinline__ void det_tables_entry(const int t) {
     if (t < 128) {
         const double c = 1.0 + (double)t * 0.0078125;
         g_det_tab[t] = 1.0 / c;
@@ -729,14 +728,6 @@ __device__ __forceinline__ double det_exp(double y) {
 // ---------------------------------------------------------------------------
 template <class Real>
 struct RT;
-
-template <>
-struct RT<double> {
-    static __device__ __forceinline__ double sqrt_(double x) { return sqrt(x); }
-    static __device__ __forceinline__ double pow_(double x) { return det_exp(1.3333330 * det_log(x)); }  // cu:195
-    static __device__ __forceinline__ double exp_(double x) { return det_exp(x); }
-    static __device__ __forceinline__ bool finite_(double x) { return isfinite(x); }
-};
 
 template <>
 struct RT<float> {

@@ -30,11 +30,21 @@ inline bool plane_fits_int32(int rows, int cols) {
 bool tile_supported(int precision, int th, int tw);
 void default_tile(int precision, int *th, int *tw);
 
+// FP32 tile kernel (step_f32.cu)
+cudaError_t prepare_step(int th, int tw);
+cudaError_t launch_step(int th, int tw, int nblocks, const GridDesc &G, const ForcingDesc &F,
+                        const StateBufs<float> &S, const Thr<float> &T, Clock *clk, const Control *ctl, int slot,
+                        cudaStream_t st);
+
+// FP64 step kernel (step_f64.cu); sms: the device's SM count; gnx, gny: g n^2 per face (launch_pack_gn), or nullptr with a scalar n
+cudaError_t prepare_step64(int th, int tw);
+cudaError_t launch_step64(int th, int tw, int nblocks, int sms, const GridDesc &G, const ForcingDesc &F,
+                          const StateBufs<double> &S, const Thr<double> &T, const double *gnx, const double *gny,
+                          Clock *clk, const Control *ctl, int slot, cudaStream_t st);
+cudaError_t launch_pack_gn(const double *n, int rows, int cols, int pitch, double g, double *gnx, double *gny,
+                           cudaStream_t st);
+
 #define SW2D_DECLARE_LAUNCHERS(Real)                                                                          \
-    cudaError_t prepare_step(int th, int tw, Real tag);                                                      \
-    cudaError_t launch_step(int th, int tw, int nblocks, const GridDesc &G, const ForcingDesc &F,             \
-                            const StateBufs<Real> &S, const Thr<Real> &T, Clock *clk, const Control *ctl,    \
-                            int slot, cudaStream_t st);                                                      \
     cudaError_t launch_pack_static(const double *z, const double *n, int rows, int cols, int pitch,         \
                                    double nodata, Real *zout, Real *nout, uint8_t *mask, cudaStream_t st);   \
     cudaError_t launch_pack_dz(const double *z, int rows, int cols, int pitch, const uint8_t *mask, Real *dzx, \

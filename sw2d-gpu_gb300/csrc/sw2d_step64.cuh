@@ -1,0 +1,667 @@
+// sw2d_step64.cuh -- the FP64 step kernel: one iteration of the reference
+// loop (SW2D-GPU_linux/src/SW2D-GPU.cu:1256-1336) on a TH x TW tile per CTA.
+//
+// Same decomposition, halo and clock bookkeeping as step_kernel
+// (sw2d_device.cuh: 4 halo cells north and west, 3 south and east, the CFL
+// bound of the new state known when the launch ends), and the same bits as the
+// serial oracle: every product, sum, quotient and root below is the correctly
+// rounded one of the reference's expression.  What differs is what it costs.
+// The kernel is bound by the FP64 pipe (2 results per SM and cycle, 1/64 of
+// FP32; 83 % busy in step_kernel, about 520 FP64 instructions per cell), so
+// work is taken off that pipe:
+//
+//   * an upwinded flux is formed once and read by the two faces it separates
+//     (step_kernel formed it for each), the bed+depth sum once per cell, and
+//     g n^2 of a face once per handle (the planes gnx, gny);
+//   * halves and quarters ride on exact powers of two folded into dt2/dx,
+//     dt2/dy and dt2 (the scaled product rounds as the unscaled one);
+//   * divisions and roots are the short correctly rounded forms of
+//     sw2d_f64math.cuh, divisions by dx and dy multiply by the rounded
+//     reciprocal and correct, the friction power leaves its exact steps to
+//     integer instructions and tables;
+//   * threshold and sign tests, clamps and maxima are integer comparisons of
+//     the bits;
+//   * the CFL bound is a maximum: an FP32 estimate of every face's wave speed
+//     finds the few faces that can hold the CTA's maximum, and only those are
+//     evaluated in FP64;
+//   * rain and evaporation are counted per cell and multiplied once per CTA
+//     where they are uniform; sums that are zero in a whole warp are skipped.
+//
+// The last scaling differs from the unscaled expression only where a product
+// leaves the normal range (below 1e-300).
+#pragma once
+
+#include "sw2d_device.cuh"
+#include "sw2d_f64math.cuh"
+
+namespace sw2d {
+
+// Tables of the friction power, filled by pow_tables_kernel (with those of the
+// plain det_log / det_exp) before the first use (init_det_tables).
+static __device__ PowTables g_pow_tab;
+
+static __global__ void pow_tables_kernel() {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    det_tables_entry(t);
+    if (t < 128) {
+        const double c = 1.0 + (double)t * 0.0078125;
+        g_pow_tab.inv[t] = 1.0 / c;
+        g_pow_tab.logc[t] = det_log_series(c);
+    }
+    if (t < 64)
+        g_pow_tab.exp2j[t] =
+            det_exp_series((double)t * (0x1.62e42p-1 / 64.0) + (double)t * (0x1.fdf473de6af28p-22 / 64.0));
+    if (t < 2 * kPowE) {
+        const double e = (double)(t - kPowE);
+        g_pow_tab.ehi[t] = e * 0x1.62e42p-1;
+        g_pow_tab.elo[t] = e * 0x1.fdf473de6af28p-22;
+    }
+    if (t < 2 * kPowN) {
+        const double n = (double)(t - kPowN);
+        g_pow_tab.nhi[t] = n * (0x1.62e42p-1 / 64.0);
+        g_pow_tab.nlo[t] = n * (0x1.fdf473de6af28p-22 / 64.0);
+    }
+}
+
+static __device__ __noinline__ double pow43_plain(double x) { return det_exp(1.3333330 * det_log(x)); }
+
+__device__ __forceinline__ double pow43(double x) {
+    bool ok;
+    const double r = d_pow43_fast(x, &g_pow_tab, &ok);
+    return ok ? r : pow43_plain(x);
+}
+
+// g n^2 of every face from the Manning raster, with the face's n the mean of its
+// two cells' (the order of g * rn * rn in cu:196, cu:313); faces at the domain
+// edge are never read.
+static __global__ void pack_gn_kernel(const double *__restrict__ n, int rows, int cols, int pitch, double g,
+                                      double *__restrict__ gnx, double *__restrict__ gny) {
+    const long long total = (long long)rows * cols;
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < total;
+         k += (long long)gridDim.x * blockDim.x) {
+        const int i = (int)(k / cols), j = (int)(k - (k / cols) * cols);
+        const size_t gp = (size_t)i * pitch + j;
+        const double rx = 0.5 * (n[k] + (i > 0 ? n[k - cols] : n[k])), ry = 0.5 * (n[k] + (j > 0 ? n[k - 1] : n[k]));
+        gnx[gp] = g * rx * rx;
+        gny[gp] = g * ry * ry;
+    }
+}
+
+// FP64 planes of the step kernel that step_kernel does not have: g n^2 of the
+// x-face north of a cell and of the y-face west of it (nullptr: scalar n).
+struct Step64Extra {
+    const double *gnx, *gny;
+    double gn;          // g n^2 of the scalar n
+    double rdx, rdy;    // 1/dx, 1/dy rounded
+};
+
+constexpr int kStep64Arrays = 13;
+
+// Work lists of one CTA: the faces (new discharges) and the fluxes they read.
+template <int TH, int TW>
+struct Step64Shape {
+    static constexpr int kFaces = 2 * (TH + 4) * (TW + 4);
+    static constexpr int kFluxes = 2 * (TH + 5) * (TW + 4) + 2 * (TH + 4) * (TW + 5);
+    static constexpr size_t kSmem = (size_t)(TH + 7) * (TW + 7) * (kStep64Arrays * sizeof(double) + 3) +
+                                    (size_t)(kFaces + kFluxes) * sizeof(uint16_t) + 16;
+};
+
+// Appends `item` of the lanes with `keep` to a list in shared memory (one
+// atomic per warp); every lane of a converged warp calls it.
+__device__ __forceinline__ void append(uint16_t *list, int *count, bool keep, unsigned item, int lane) {
+    const unsigned bal = __ballot_sync(0xffffffffu, keep);
+    if (!bal) return;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(count, __popc(bal));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (keep) list[base + __popc(bal & ((1u << lane) - 1u))] = (uint16_t)item;
+}
+
+template <int TH, int TW, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB)
+    step64_kernel(const GridDesc G, const ForcingDesc F, const StateBufs<double> S, const Thr<double> T,
+                  const Step64Extra X, Clock *__restrict__ clk, const Control *__restrict__ ctl, const int slot) {
+    constexpr int HN = 4;
+    constexpr int RH = TH + 7, RW = TW + 7, RN = RH * RW;
+    constexpr int NW = NT / 32;
+
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double *s_h = reinterpret_cast<double *>(smem_raw);
+    double *s_z = s_h + RN;
+    double *s_eta = s_z + RN;   // depth + bed
+    double *s_umo = s_eta + RN;  // old um, later the corrected new um
+    double *s_vno = s_umo + RN;
+    double *s_uu = s_vno + RN;   // face velocities; s_uu later holds the provisional depth
+    double *s_vv = s_uu + RN;
+    double *s_fx = s_vv + RN;    // upwinded fluxes (times 4): of um through the cell, ...
+    double *s_cu = s_fx + RN;    // ... of um through the corner west of the x-face,
+    double *s_cv = s_cu + RN;    // of vn through the corner north of the y-face,
+    double *s_fy = s_cv + RN;    // of vn through the cell
+    double *s_rum = s_fy + RN;   // new um before the dry-cell fix
+    double *s_rvn = s_rum + RN;
+    constexpr int kFaces = Step64Shape<TH, TW>::kFaces, kFluxes = Step64Shape<TH, TW>::kFluxes;
+    static_assert(kFaces < (1 << 14) && kFluxes < (1 << 16), "list entries are 16 bits wide");
+    uint16_t *s_face = reinterpret_cast<uint16_t *>(s_rvn + RN);  // momentum faces from the front, weir faces from the back
+    uint16_t *s_flux = s_face + kFaces;
+    uint8_t *s_m = reinterpret_cast<uint8_t *>(s_flux + kFluxes);
+    uint8_t *s_tx = s_m + RN, *s_ty = s_tx + RN;  // 1: the x- / y-face takes the momentum equation
+    double *s_hs = s_uu;
+
+    __shared__ double s_red[NW][B_N];
+    __shared__ int s_cnt[NW][2];
+    __shared__ int s_n[3];  // lengths of the lists: momentum faces, weir faces, fluxes
+    __shared__ unsigned s_est;
+    __shared__ unsigned long long s_cm;
+    __shared__ int s_nloc;
+    __shared__ int s_srcp[kMaxLocalSources];
+    __shared__ double s_srcq0[kMaxLocalSources], s_srcq1[kMaxLocalSources];
+    __shared__ int s_wcnt[NW];
+
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int slot_out = slot == 2 ? 0 : slot + 1;
+    const int slot_nx = slot == 0 ? 2 : slot - 1;
+    const int rows = G.rows, cols = G.cols, pitch = G.pitch;
+    const int ti = blockIdx.x / G.tiles_w, tj = blockIdx.x - ti * G.tiles_w;
+    const int I0 = ti * TH - HN, J0 = tj * TW - HN;  // global index of smem (0,0)
+
+    // ---- stage 0: stage the tile + halo in shared memory --------------------
+    // Launched as a programmatic dependent of the previous iteration: the
+    // static fields are read while that one drains, then its completion (and
+    // the visibility of its writes) is waited for
+    for (int idx = tid; idx < RN; idx += NT) {
+        const int r = idx / RW, c = idx - (idx / RW) * RW;
+        const int gi = I0 + r, gj = J0 + c;
+        const bool in = (unsigned)gi < (unsigned)rows && (unsigned)gj < (unsigned)cols;
+        const size_t gp = (size_t)gi * pitch + gj;
+        s_z[idx] = in ? S.z[gp] : 0.0;
+        s_m[idx] = in ? S.mask[gp] : (uint8_t)0;
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const Clock &ci = clk[slot];
+    const Plan &pl = ci.plan;
+
+    if (!pl.run) {  // nothing to do: carry the state's clock forward
+        if (blockIdx.x == 0 && wid == 0) carry_slot_deferred_warp(lane, clk, slot, slot_out, slot_nx);
+        return;
+    }
+
+    const int buf = ci.buf;
+    const double *__restrict__ Hin = S.h[buf];
+    const double *__restrict__ Uin = S.um[buf];
+    const double *__restrict__ Vin = S.vn[buf];
+    double *__restrict__ Hout = S.h[1 - buf];
+    double *__restrict__ Uout = S.um[1 - buf];
+    double *__restrict__ Vout = S.vn[1 - buf];
+
+    const LaunchScalars<double> LS = pl.d;
+    const double dt2 = LS.dt2;
+    const double dx = G.sd.dx, dy = G.sd.dy, g = G.sd.g;
+    const unsigned long long gt_th = d_bits(T.gt_th), ge_th = d_bits(T.ge_th);
+    const unsigned long long gt_ev = d_bits(T.gt_evmin > 0.0 ? T.gt_evmin : 0.0);
+
+    for (int idx = tid; idx < RN; idx += NT) {
+        const int r = idx / RW, c = idx - (idx / RW) * RW;
+        const int gi = I0 + r, gj = J0 + c;
+        const bool in_r = (unsigned)gi < (unsigned)rows, in_c = (unsigned)gj < (unsigned)cols;
+        const size_t gp = (size_t)gi * pitch + gj;
+        s_h[idx] = in_r && in_c ? Hin[gp] : 0.0;
+        s_umo[idx] = ((unsigned)gi <= (unsigned)rows && in_c) ? Uin[gp] : 0.0;
+        s_vno[idx] = (in_r && (unsigned)gj <= (unsigned)cols) ? Vin[gp] : 0.0;
+    }
+    if (tid == 0) {
+        s_nloc = 0;
+        s_n[0] = s_n[1] = s_n[2] = 0;
+        s_est = 0u;
+        s_cm = 0ull;
+    }
+    // point sources inside this tile's provisional-depth region, kept in
+    // list order so that a later source on the same cell wins (cu:545)
+    if (G.n_src > 0) {
+        __syncthreads();
+        const double area = G.dx * G.dy;
+        for (int base = 0; base < G.n_src; base += NT) {
+            const int s = base + tid;
+            bool in = false;
+            int p = 0;
+            if (s < G.n_src) {
+                const int cell = F.src_cell[s];
+                const int gi = cell / cols, gj = cell - (cell / cols) * cols;
+                const int r = gi - I0, c = gj - J0;
+                in = (r >= 2 && r < TH + 5 && c >= 2 && c < TW + 5);
+                p = r * RW + c;
+            }
+            const unsigned bal = __ballot_sync(0xffffffffu, in);
+            if (lane == 0) s_wcnt[wid] = __popc(bal);
+            __syncthreads();
+            if (in) {
+                int off = s_nloc;
+                for (int w = 0; w < wid; w++) off += s_wcnt[w];
+                off += __popc(bal & ((1u << lane) - 1u));
+                if (off < kMaxLocalSources) {
+                    s_srcp[off] = p;
+                    s_srcq0[off] = source_rate(F, G.n_src, s, pl.t0, area);
+                    s_srcq1[off] = source_rate(F, G.n_src, s, pl.t1, area);
+                } else {
+                    atomicOr(&clk[slot_out].status, (unsigned)ST_TOO_MANY_LOCAL_SOURCES);
+                }
+            }
+            __syncthreads();
+            if (tid == 0) {
+                int tot = s_nloc;
+                for (int w = 0; w < NW; w++) tot += s_wcnt[w];
+                s_nloc = tot < kMaxLocalSources ? tot : kMaxLocalSources;
+            }
+            __syncthreads();  // s_wcnt is rewritten by the next chunk
+        }
+    }
+    __syncthreads();
+
+    const double *__restrict__ W = S.rainw;  // spatial rain factors (extension) or nullptr
+    const int nloc = s_nloc;
+    const double pct_hi = G.sd.pct_hi, pct_lo = G.sd.pct_lo;
+    const bool storm = F.rain_kind == RAIN_STORM;
+
+    // ---- stage 1: face velocities (cu:363-453) and surface elevations ------
+    for (int idx = tid; idx < RN; idx += NT) {
+        const int r = idx / RW, c = idx - (idx / RW) * RW;
+        const int gi = I0 + r, gj = J0 + c;
+        const double h = s_h[idx];
+        s_eta[idx] = h + s_z[idx];
+        if (r >= 1) {
+            double hm;
+            if (gi == rows) hm = s_h[idx - RW];
+            else if (gi == 0) hm = h;
+            else hm = d_half(h + s_h[idx - RW]);
+            s_uu[idx] = d_ge_pos(hm, ge_th) ? d_div(s_umo[idx], hm) : 0.0;
+        }
+        if (c >= 1) {
+            double hn;
+            if (gj == cols) hn = s_h[idx - 1];
+            else if (gj == 0) hn = h;
+            else hn = d_half(h + s_h[idx - 1]);
+            s_vv[idx] = d_ge_pos(hn, ge_th) ? d_div(s_vno[idx], hn) : 0.0;
+        }
+    }
+    __syncthreads();
+
+    // ---- stage 1a: what each face does (cu:116-165, cu:232-282) --------------
+    // A warp's FP64 instruction costs the same for 1 as for 32 lanes, and on a
+    // thin film over steep ground dry-bed rules and momentum alternate from face
+    // to face, so the faces are sorted into a list for each first.
+    constexpr int FH = TH + 4, FW = TW + 4, FN = FH * FW;  // faces: rows/cols [2, TH+6) x [2, TW+6)
+    for (int b0 = wid * 32; b0 < kFaces; b0 += NT) {
+        const int k0 = b0 + lane;
+        int rule = 0;  // 1, 2, 3: dry-bed rules, 4: momentum, 0: no flow
+        if (k0 < kFaces) {
+            const bool isx = k0 < FN;
+            const int k = isx ? k0 : k0 - FN;
+            const int r = 2 + k / FW, c = 2 + (k - (k / FW) * FW);
+            const int p = r * RW + c;
+            const int gi = I0 + r, gj = J0 + c;
+            const int pa = isx ? p - RW : p - 1;  // cell "a" (north / west) of the face; p is "b"
+            const bool inner = isx ? (gi > 0 && gi < rows && (unsigned)gj < (unsigned)cols)
+                                   : ((unsigned)gi < (unsigned)rows && gj > 0 && gj < cols);
+            if (inner) {
+                const double ha = s_h[pa], hb = s_h[p];
+                const bool a_wet = d_ge_pos(ha, gt_th), b_wet = d_ge_pos(hb, gt_th);
+                if (s_m[p] && s_m[pa] && (a_wet || b_wet)) {
+                    rule = 4;
+                    if (d_lt(s_eta[p], s_z[pa])) {  // cu:130: b's surface below a's bed
+                        rule = a_wet ? 1 : 0;
+                    } else if (d_lt(s_eta[pa], s_z[p])) {  // cu:138
+                        rule = b_wet ? 2 : 0;
+                    } else {
+                        // cu:149: exactly one side strictly wet; false for NaN
+                        const bool a_dry = !d_ge_pos(ha, ge_th) && !d_is_nan(ha);
+                        const bool b_dry = !d_ge_pos(hb, ge_th) && !d_is_nan(hb);
+                        if ((b_wet && a_dry) || (b_dry && a_wet)) rule = 3;
+                    }
+                }
+            } else if (isx && gi == rows && (unsigned)gj < (unsigned)cols && G.south_open) {
+                // free outfall (extension): the weir formula of rule 1
+                rule = (s_m[pa] && d_ge_pos(s_h[pa], gt_th)) ? 1 : 0;
+            }
+            (isx ? s_tx : s_ty)[p] = rule == 4;
+            if (rule == 0) (isx ? s_rum : s_rvn)[p] = 0.0;
+        }
+        append(s_face, &s_n[0], rule == 4, k0, lane);
+        const unsigned bal = __ballot_sync(0xffffffffu, rule >= 1 && rule <= 3);
+        if (bal) {
+            int base = 0;
+            if (lane == 0) base = atomicAdd(&s_n[1], __popc(bal));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (rule >= 1 && rule <= 3)
+                s_face[kFaces - 1 - (base + __popc(bal & ((1u << lane) - 1u)))] = (uint16_t)(k0 | (rule << 14));
+        }
+    }
+    __syncthreads();
+
+    // ---- stage 1b: upwinded fluxes (cu:172-190, cu:289-307), each once ------
+    // vel (o + s) / 2 + |vel| (s - o) / 2 with vel = (v + w) / 2 is a quarter of
+    // (v + w) (o + s) + |v + w| (s - o); for every flux the second factor is
+    // (lower-index value) - (higher-index value) of the discharge.
+    //   fx[p], of um through cell p, between the x-faces p and p + RW
+    //   cv[p], of vn through the corner between the y-faces p - RW and p
+    //   cu[p], of um through the corner between the x-faces p - 1 and p
+    //   fy[p], of vn through cell p, between the y-faces p and p + 1
+    constexpr int NA = (FH + 1) * FW, NB = FH * (FW + 1);
+    // item -> kind, element of the flux and of the higher-index face it reads
+    auto flux_item = [&](int k, int &kind, int &po, int &e) {
+        if (k < 2 * NA) {
+            kind = k >= NA ? 1 : 0;  // fx, cv
+            k -= kind ? NA : 0;
+            po = (1 + k / FW) * RW + 2 + (k - (k / FW) * FW);
+            e = po + RW;
+            if (kind) po = e;
+        } else {
+            k -= 2 * NA;
+            kind = k >= NB ? 3 : 2;  // cu, fy
+            k -= kind == 3 ? NB : 0;
+            po = (2 + k / (FW + 1)) * RW + 1 + (k - (k / (FW + 1)) * (FW + 1));
+            e = po + 1;
+            if (kind == 2) po = e;
+        }
+    };
+    for (int b0 = wid * 32; b0 < kFluxes; b0 += NT) {
+        const int k = b0 + lane;
+        bool need = false;
+        if (k < kFluxes) {
+            int kind, po, e;
+            flux_item(k, kind, po, e);
+            const bool of_um = kind == 0 || kind == 2;
+            const int oq = kind < 2 ? -RW : -1;
+            // read by momentum faces of its own direction on either side
+            const uint8_t *t = of_um ? s_tx : s_ty;
+            // (a face outside rows/cols [2, TH+6) x [2, TW+6) reads nothing)
+            const int r0 = (e + oq) / RW, c0 = (e + oq) - r0 * RW, r1 = e / RW, c1 = e - r1 * RW;
+            const bool in0 = r0 >= 2 && c0 >= 2, in1 = r1 < TH + 6 && c1 < TW + 6;
+            const double *q = of_um ? s_umo : s_vno;
+            if ((in0 && t[e + oq]) || (in1 && t[e])) {
+                need = !(d_is_zero(q[e]) && d_is_zero(q[e + oq]));
+                if (!need) (kind == 0 ? s_fx : kind == 1 ? s_cv : kind == 2 ? s_cu : s_fy)[po] = 0.0;
+            }
+        }
+        append(s_flux, &s_n[2], need, k, lane);
+    }
+    __syncthreads();
+    for (int i = tid; i < s_n[2]; i += NT) {
+        int kind, po, e;
+        flux_item(s_flux[i], kind, po, e);
+        const int oq = kind < 2 ? -RW : -1, ov = kind == 0 || kind == 2 ? -RW : -1;
+        const double *v = kind < 2 ? s_uu : s_vv, *q = kind == 0 || kind == 2 ? s_umo : s_vno;
+        const double qb = q[e], qa = q[e + oq], vel = v[e] + v[e + ov];
+        (kind == 0 ? s_fx : kind == 1 ? s_cv : kind == 2 ? s_cu : s_fy)[po] = vel * (qa + qb) + fabs(vel) * (qa - qb);
+    }
+    __syncthreads();
+
+    // ---- stage 2: new face discharges (cu:98-354) ---------------------------
+    const double qdx = 0.25 * LS.dt2dx, qdy = 0.25 * LS.dt2dy;  // with the fluxes' quarters
+    const double hdx = 0.5 * LS.dt2dx, hdy = 0.5 * LS.dt2dy, hdt2 = 0.5 * dt2;
+    const int n_mom = s_n[0], n_weir = s_n[1];
+    const int mom_chunks = (n_mom + 31) / 32, chunks = mom_chunks + (n_weir + 31) / 32;
+    for (int ch = wid; ch < chunks; ch += NW) {
+        if (ch < mom_chunks) {
+            const int i = ch * 32 + lane;
+            if (i >= n_mom) continue;
+            const int k0 = s_face[i];
+            const bool isx = k0 < FN;
+            const int k = isx ? k0 : k0 - FN;
+            const int r = 2 + k / FW, c = 2 + (k - (k / FW) * FW);
+            const int p = r * RW + c, pa = isx ? p - RW : p - 1;
+            const int gi = I0 + r, gj = J0 + c;
+            const double ha = s_h[pa], hb = s_h[p], za = s_z[pa], eb = s_eta[p];
+            const double mo = isx ? s_umo[p] : s_vno[p];
+            const double hsum = hb + ha, hm = d_half(hsum);
+            // gravity (cu:166, cu:283): g hm (dt2/dx) (hb + zb - ha - za)
+            const double u13 = g * hsum * (isx ? hdx : hdy) * (eb - ha - za);
+            // convection along i and along j (cu:172-190, cu:289-307)
+            const double *f1 = isx ? s_fx + p : s_cv + p + RW;
+            const double *f2 = isx ? s_cu + p + 1 : s_fy + p;
+            double a1 = qdx * (f1[0] - f1[-RW]), a2 = qdy * (f2[0] - f2[-1]);
+            if (!isx && gi == 0) a1 = 0.0;  // cu:289-291
+            if (isx && gj == 0) a2 = 0.0;   // cu:178-180
+            const double rest = -a1 - a2 - u13;
+            // friction (cu:194-199, cu:311-316): zero only when hm <= th or n == 0
+            const double gn = X.gnx ? (isx ? X.gnx : X.gny)[(size_t)gi * pitch + gj] : X.gn;
+            double q;
+            if ((d_ge_pos(hm, gt_th) || d_is_nan(hm)) && !d_is_zero(gn)) {
+                const double *t = isx ? s_vv + p : s_uu + p;
+                const int o1 = isx ? 1 : RW, o2 = isx ? -RW : -1;
+                const double t4 = t[0] + t[o1] + t[o2] + t[o1 + o2];  // 4 times vva / uua
+                const double own = isx ? s_uu[p] : s_vv[p];
+                const double speed = d_sqrt(d_fma(t4 * t4, 0.0625, own * own));
+                const double x = hdt2 * d_div(gn * speed, pow43(hm));
+                q = d_div((1.00 - x) * mo + rest, 1.00 + x);  // cu:203, cu:320
+            } else {
+                q = mo + rest;
+            }
+            (isx ? s_rum : s_rvn)[p] = q;
+        } else {
+            // dry-bed rules (cu:130-159, cu:247-276) and the outfall: a
+            // coefficient times depth times sqrt(g depth) or sqrt(2 g depth)
+            const int i = (ch - mom_chunks) * 32 + lane;
+            if (i >= n_weir) continue;
+            const int it = s_face[kFaces - 1 - i], rule = it >> 14, k0 = it & 0x3fff;
+            const bool isx = k0 < FN;
+            const int k = isx ? k0 : k0 - FN;
+            const int p = (2 + k / FW) * RW + 2 + (k - (k / FW) * FW), pa = isx ? p - RW : p - 1;
+            const double ha = s_h[pa], hb = s_h[p];
+            double d = rule == 1 ? ha : hb, w = rule == 1 ? 0.5440 : -0.544;
+            if (rule == 3) {
+                const double ea = s_eta[pa], eb = s_eta[p], za = s_z[pa], zb = s_z[p];
+                d = fmax(eb, ea) - fmax(zb, za);
+                w = d_ge_pos(hb, gt_th) ? -0.350 : 0.350;  // cu:151-154
+            }
+            (isx ? s_rum : s_rvn)[p] = w * d * d_sqrt((rule == 3 ? 2.00 * g : g) * d);
+        }
+    }
+    __syncthreads();
+
+    // storm rain at a cell centre; the centre (sx, sy) is per launch
+    const double storm_amp = G.sd.storm_amp, storm_2s2 = G.sd.storm_2s2;
+    auto storm_rate = [&](int gi, int gj, bool on, double sx, double sy) -> double {
+        if (!on) return 0.0;
+        const double x = ((double)gj + 0.5) * dx - sx;
+        const double y = ((double)gi + 0.5) * dy - sy;
+        return storm_amp * det_exp(-(x * x + y * y) / storm_2s2);
+    };
+    // ho - dt2 ((us - un) / dx + (ve - vw) / dy - ql - rr pct + evapo) (cu:654),
+    // the terms that are zero everywhere left out; rp = rr pct
+    const bool any_ev0 = !d_is_zero(LS.ev0), any_ev1 = !d_is_zero(LS.ev1);
+    auto balance = [&](double ho, double un, double us, double vw, double ve, double ql, double rp, double evapo,
+                       bool any_ev) -> double {
+        double s = d_div_const(us - un, dx, X.rdx) + d_div_const(ve - vw, dy, X.rdy);
+        if (nloc) s = s - ql;
+        s = s - rp;
+        if (any_ev) s = s + evapo;
+        return ho - dt2 * s;
+    };
+    const bool uniform = !storm && !W;
+
+    // ---- stage 3: provisional depth with forcing at t (cu:1278-1288) -------
+    const double rp0_hi = LS.rr0 * pct_hi, rp0_lo = LS.rr0 * pct_lo;
+    constexpr int PH = TH + 3, PW = TW + 3;  // rows/cols [2, TH+5) x [2, TW+5)
+    for (int k = tid; k < PH * PW; k += NT) {
+        const int r = 2 + k / PW, c = 2 + (k - (k / PW) * PW);
+        const int p = r * RW + c;
+        double hv = 0.0;
+        if (s_m[p]) {
+            const double ho = s_h[p];
+            const bool hi = d_ge_pos(ho, gt_ev);
+            double ql = 0.0;
+            for (int q = 0; q < nloc; q++)
+                if (s_srcp[q] == p) ql = s_srcq0[q];
+            double rp = hi ? rp0_hi : rp0_lo;
+            if (!uniform) {
+                double rr = storm ? storm_rate(I0 + r, J0 + c, pl.storm_on0, LS.sx0, LS.sy0) : LS.rr0;
+                if (W) rr = rr * W[(size_t)(I0 + r) * pitch + (J0 + c)];
+                rp = rr * (hi ? pct_hi : pct_lo);
+            }
+            hv = d_clamp0(balance(ho, s_rum[p], s_rum[p + RW], s_rvn[p], s_rvn[p + 1], ql, rp, hi ? LS.ev0 : 0.0,
+                                  any_ev0));  // cu:657
+        }
+        s_hs[p] = hv;
+    }
+    __syncthreads();
+
+    // ---- stage 4: dry-cell fix per face (cu:695-725) + final depth ----------
+    // corrected face at p (a: the other cell's element): zero if it drains a dry cell
+    auto fix = [&](double q, int p, int a) -> double {
+        if (d_gt_zero(q) && s_m[a] && !d_ge_pos(s_hs[a], ge_th)) return 0.0;
+        if (d_lt_zero(q) && s_m[p] && !d_ge_pos(s_hs[p], ge_th)) return 0.0;
+        return q;
+    };
+    const double rp1_hi = LS.rr1 * pct_hi, rp1_lo = LS.rr1 * pct_lo;
+    int n_hi = 0, n_lo = 0;  // active owned cells above / not above EV_WL_min
+    double b_rain = 0.0, b_src = 0.0, b_out = 0.0, b_clamp = 0.0;
+    bool bad = false;
+    constexpr int OH = TH + 1, OW = TW + 1;  // rows/cols [3, TH+4) x [3, TW+4)
+    for (int k = tid; k < OH * OW; k += NT) {
+        const int r = 3 + k / OW, c = 3 + (k - (k / OW) * OW);
+        const int p = r * RW + c;
+        const int gi = I0 + r, gj = J0 + c;
+        const double un = fix(s_rum[p], p, p - RW), us = fix(s_rum[p + RW], p + RW, p);
+        const double vw = fix(s_rvn[p], p, p - 1), ve = fix(s_rvn[p + 1], p + 1, p);
+        double hv = 0.0, hraw = 0.0;
+        const bool act = s_m[p] != 0;
+        bool hi = false;
+        double ql = 0.0, rp = 0.0;
+        if (act) {
+            const double ho = s_h[p];
+            hi = d_ge_pos(ho, gt_ev);
+            for (int q = 0; q < nloc; q++)
+                if (s_srcp[q] == p) ql = s_srcq1[q];
+            rp = hi ? rp1_hi : rp1_lo;
+            if (!uniform) {
+                double rr = storm ? storm_rate(gi, gj, pl.storm_on1, LS.sx1, LS.sy1) : LS.rr1;
+                if (W) rr = rr * W[(size_t)gi * pitch + gj];
+                rp = rr * (hi ? pct_hi : pct_lo);
+            }
+            hraw = balance(ho, un, us, vw, ve, ql, rp, hi ? LS.ev1 : 0.0, any_ev1);
+            hv = d_clamp0(hraw);
+        }
+        s_h[p] = hv;  // the new depth; only this thread reads s_h[p] in this stage
+        s_umo[p] = un;
+        s_vno[p] = vw;
+        if (r == TH + 3) s_umo[p + RW] = us;
+        if (c == TW + 3) s_vno[p + 1] = ve;
+        const bool core = r >= HN && c >= HN && r < TH + HN && c < TW + HN && gi < rows && gj < cols;
+        if (core) {
+            const size_t gp = (size_t)gi * pitch + gj;
+            Hout[gp] = hv;
+            Uout[gp] = un;
+            Vout[gp] = vw;
+            if (gi == rows - 1) {
+                Uout[gp + pitch] = us;
+                b_out += us;
+            }
+            if (act) {
+                if (hi) n_hi++;
+                else n_lo++;
+                if (!uniform) b_rain += rp;
+                if (nloc) b_src += ql;
+                if (d_lt_zero(hraw)) b_clamp -= hraw;
+            }
+            if (!d_is_finite(hv) || !d_is_finite(un) || !d_is_finite(vw)) bad = true;
+        }
+    }
+    __syncthreads();
+
+    // ---- stage 5: CFL bound of the new state over the owned faces ----------
+    // An FP32 estimate of |q / h| + sqrt(g h), within 2^-18 of the FP64 value,
+    // is formed for every owned face between active cells (and the open south
+    // faces).  The CTA's largest estimate among the faces certainly deeper than
+    // th, less that margin, is a bar below the exact maximum: only faces whose
+    // estimate reaches it are evaluated in FP64.
+    const float gf = (float)g, thf = (float)T.ge_th;
+    auto faces = [&](auto &&visit) {
+        for (int k = tid; k < TH * TW; k += NT) {
+            const int r = HN + k / TW, c = HN + (k - (k / TW) * TW);
+            const int p = r * RW + c;
+            const int gi = I0 + r, gj = J0 + c;
+            if (gi >= rows || gj >= cols || !s_m[p]) continue;
+            const double h = s_h[p];
+            if (gi > 0 && s_m[p - RW]) visit(s_umo[p], h, s_h[p - RW]);
+            if (gi == rows - 1 && G.south_open) visit(s_umo[p + RW], h, h);
+            if (gj > 0 && s_m[p - 1]) visit(s_vno[p], h, s_h[p - 1]);
+        }
+    };
+    auto estimate = [&](double q, double h0, double h1, float &hm) -> float {
+        hm = 0.5f * (d_abs_float(h0) + d_abs_float(h1));
+        return d_abs_float(q) / hm + sqrtf(gf * hm);
+    };
+    constexpr float kMargin = 1.f / 131072.f;
+    float sure = 0.f, est = 0.f;  // over faces certainly / possibly deeper than th
+    faces([&](double q, double h0, double h1) {
+        float hm;
+        const float e = estimate(q, h0, h1, hm);
+        if (hm >= thf * (1.f + kMargin)) sure = fmaxf(sure, e);
+        if (hm >= thf * (1.f - kMargin)) est = fmaxf(est, e);
+    });
+    const unsigned wmax = __reduce_max_sync(0xffffffffu, __float_as_uint(sure));
+    if (lane == 0 && wmax) atomicMax(&s_est, wmax);
+    const bool any_bad = __syncthreads_or(bad);
+    const float bar = __uint_as_float(s_est) * (1.f - kMargin);
+    if (est >= bar) {
+        unsigned long long cm = 0ull;
+        faces([&](double q, double h0, double h1) {
+            float hf;
+            const float e = estimate(q, h0, h1, hf);
+            if (!(e >= bar) || !(hf >= thf * (1.f - kMargin))) return;
+            const double hm = 0.50 * (h0 + h1);
+            if (!d_ge_pos(hm, ge_th)) return;
+            const double v = fabs(d_div(q, hm)) + d_sqrt(g * hm);
+            if (!d_is_nan(v)) cm = d_bits(v) > cm ? d_bits(v) : cm;
+        });
+        if (cm) atomicMax(&s_cm, cm);
+    }
+
+    // ---- block reductions, one atomic per quantity --------------------------
+    n_hi = __reduce_add_sync(0xffffffffu, n_hi);
+    n_lo = __reduce_add_sync(0xffffffffu, n_lo);
+    double vals[4] = {b_rain, b_src, b_out, b_clamp};
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        double v = vals[q];
+        if (__any_sync(0xffffffffu, !d_is_zero(v))) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        }
+        vals[q] = v;
+    }
+    if (lane == 0) {
+        s_red[wid][0] = vals[0];
+        s_red[wid][1] = vals[1];
+        s_red[wid][2] = vals[2];
+        s_red[wid][3] = vals[3];
+        s_cnt[wid][0] = n_hi;
+        s_cnt[wid][1] = n_lo;
+    }
+    __syncthreads();
+    if (tid >= 32) return;
+    if (tid == 0) {
+        double acc[4] = {0.0, 0.0, 0.0, 0.0};
+        int c_hi = 0, c_lo = 0;
+        for (int w = 0; w < NW; w++) {
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (!d_is_zero(s_red[w][q])) acc[q] += s_red[w][q];
+            c_hi += s_cnt[w][0];
+            c_lo += s_cnt[w][1];
+        }
+        if (uniform) acc[0] = rp1_hi * (double)c_hi + rp1_lo * (double)c_lo;
+        const double area = G.dx * G.dy;
+        const double scale = pl.d.dt2 * area;
+        double v[B_N];
+        v[B_RAIN] = acc[0] * scale;
+        v[B_SRC] = acc[1] * scale;
+        v[B_EV] = LS.ev1 * (double)c_hi * scale;
+        v[B_OUT] = acc[2] * pl.d.dt2 * G.dy;
+        v[B_CLAMP] = acc[3] * area;
+        accumulate_slot(clk[slot_out], blockIdx.x % kBuckets, v, d_from_bits(s_cm), any_bad);
+    }
+    finish_cta_deferred_warp(lane, clk, slot, slot_out, slot_nx, pl, *ctl, G, F);
+}
+
+}  // namespace sw2d
