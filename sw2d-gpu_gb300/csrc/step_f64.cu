@@ -22,7 +22,39 @@ cudaError_t init_det_tables() {
 // per iteration on a 1013 x 900 catchment, against 557 with 256 threads (the
 // integer stages run at too few warps), 525 with 512, and 550 with a 32 x 32
 // tile (less halo, but one CTA per SM idles at its barriers).
-#define SW2D_STEP64_TILES(X) X(16, 32, 384, 2) X(8, 32, 256, 3)
+//
+// The smaller tiles are for grids that would leave SMs without a CTA: a tile's
+// work runs on one SM's FP64 pipe, so a grid is cut into the smallest tiles that
+// still give one CTA per SM (step64_tile).  Measured, us per iteration, tiles
+// 4x8 / 4x16 / 8x16 / 8x32 / 16x32: 64 x 64 23.8 / 27.0 / 30.3 / 42.3 / 53.5;
+// 117 x 131 48.8 / 42.8 / 34.5 / 47.5 / 60.2; 256 x 256 159 / 106 / 79 / 72 /
+// 69.5; 512 x 512 593 / 327 / 261 / 225 / 185 (the halo costs 2.3 times the
+// faces of the tile at 4 x 8, 1.4 at 16 x 32).
+#define SW2D_STEP64_TILES(X) \
+    X(16, 32, 384, 2) X(8, 32, 256, 3) X(8, 16, 256, 2) X(4, 16, 192, 2) X(4, 8, 192, 2)
+
+bool step64_tile_supported(int th, int tw) {
+#define SW2D_S64(h, w, nt, mb) \
+    if (th == h && tw == w) return true;
+    SW2D_STEP64_TILES(SW2D_S64)
+#undef SW2D_S64
+    return false;
+}
+
+// The smallest tile with at most one CTA per SM, 16 x 32 beyond.
+void step64_tile(int rows, int cols, int sms, int *th, int *tw) {
+    *th = 16;
+    *tw = 32;
+    long long best = 16 * 32;
+#define SW2D_D64(h, w, nt, mb)                                                                       \
+    if (h * w < best && (long long)((rows + h - 1) / h) * ((cols + w - 1) / w) <= sms) {             \
+        best = h * w;                                                                                \
+        *th = h;                                                                                     \
+        *tw = w;                                                                                     \
+    }
+    SW2D_STEP64_TILES(SW2D_D64)
+#undef SW2D_D64
+}
 
 cudaError_t prepare_step64(int th, int tw) {
     const cudaError_t e = init_det_tables();

@@ -200,13 +200,23 @@ int validate(const sw2d_config *c, std::string *why) {
     return 1;
 }
 
-void grid_shape(const sw2d_config *c, int *pitch, size_t *plane, int *th, int *tw) {
+void grid_shape(const sw2d_config *c, int *pitch, size_t *plane) {
     *pitch = pitch_for(c->cols);
     *plane = plane_for(c->rows, *pitch);
-    int a = c->tile_h, b = c->tile_w;
-    if (a <= 0 || b <= 0 || !tile_supported(c->precision, a, b)) default_tile(c->precision, &a, &b);
-    *th = a;
-    *tw = b;
+}
+
+// The tile of the FP64 and FP32 tile kernels: the caller's where there is a
+// build of it, the library's otherwise.
+void pick_tile(const sw2d_config *c, int sms, int *th, int *tw) {
+    *th = c->tile_h;
+    *tw = c->tile_w;
+    if (*th > 0 && *tw > 0 && tile_supported(c->precision, *th, *tw)) return;
+    if (c->precision == SW2D_PREC_F64) {
+        step64_tile(c->rows, c->cols, sms, th, tw);
+    } else {
+        *th = 32;
+        *tw = 32;
+    }
 }
 
 int read_clock(sw2d_handle *h) {
@@ -326,13 +336,8 @@ int pipe_strip(int rows, int tiles_w, long long resident) {
 namespace sw2d {
 
 bool tile_supported(int precision, int th, int tw) {
-    if (precision == SW2D_PREC_F64) return (th == 16 && tw == 32) || (th == 8 && tw == 32);
+    if (precision == SW2D_PREC_F64) return step64_tile_supported(th, tw);
     return (th == 16 && tw == 32) || (th == 32 && tw == 32) || (th == 16 && tw == 64);
-}
-
-void default_tile(int precision, int *th, int *tw) {
-    *th = precision == SW2D_PREC_F64 ? 16 : 32;
-    *tw = 32;
 }
 
 }  // namespace sw2d
@@ -358,9 +363,9 @@ int sw2d_config_init(sw2d_config *c) {
 int sw2d_device_bytes(const sw2d_config *c, int64_t *bytes) {
     std::string why;
     if (!bytes || !validate(c, &why)) return SW2D_ERR_INVALID_ARG;
-    int pitch, th, tw;
+    int pitch;
     size_t plane;
-    grid_shape(c, &pitch, &plane, &th, &tw);
+    grid_shape(c, &pitch, &plane);
     const size_t rs = c->precision == SW2D_PREC_F64 ? 8 : 4;
     const bool stream = c->precision == SW2D_PREC_F32 && c->kernel != SW2D_KERNEL_TILE;
     // 2x(h, um, vn) + z, frame included, and: n (FP32), dzx, dzy, 2x remainder (streaming kernel), g n^2 of the
@@ -382,7 +387,7 @@ int sw2d_create(const sw2d_config *cfg, sw2d_handle **out) {
     if (!h) return SW2D_ERR_OOM;
     h->cfg = *cfg;
     h->real_size = cfg->precision == SW2D_PREC_F64 ? 8 : 4;
-    grid_shape(cfg, &h->pitch, &h->plane, &h->tile_h, &h->tile_w);
+    grid_shape(cfg, &h->pitch, &h->plane);
     h->origin = origin_for(h->pitch);
     auto bail = [&](int code) {
         sw2d_destroy(h);
@@ -393,6 +398,7 @@ int sw2d_create(const sw2d_config *cfg, sw2d_handle **out) {
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(SW2D_ERR_CUDA);
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg->device) == cudaSuccess && sms > 0) h->sms = sms;
+    pick_tile(cfg, h->sms, &h->tile_h, &h->tile_w);
     const size_t fb = h->plane * h->real_size;
     // allocate with the zero frame, keep pointers at cell (0,0)
     auto alloc_field = [&](void **p, size_t esz) -> bool {

@@ -28,7 +28,6 @@ inline bool plane_fits_int32(int rows, int cols) {
 
 // Core tiles supported by the step kernel instantiations.
 bool tile_supported(int precision, int th, int tw);
-void default_tile(int precision, int *th, int *tw);
 
 // FP32 tile kernel (step_f32.cu)
 cudaError_t prepare_step(int th, int tw);
@@ -38,6 +37,8 @@ cudaError_t launch_step(int th, int tw, int nblocks, const GridDesc &G, const Fo
 
 // FP64 step kernel (step_f64.cu); sms: the device's SM count; gnx, gny: g n^2 per face (launch_pack_gn), or nullptr with a scalar n
 cudaError_t prepare_step64(int th, int tw);
+bool step64_tile_supported(int th, int tw);
+void step64_tile(int rows, int cols, int sms, int *th, int *tw);  // the library's tile for a grid
 cudaError_t launch_step64(int th, int tw, int nblocks, int sms, const GridDesc &G, const ForcingDesc &F,
                           const StateBufs<double> &S, const Thr<double> &T, const double *gnx, const double *gny,
                           Clock *clk, const Control *ctl, int slot, cudaStream_t st);

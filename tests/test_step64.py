@@ -123,7 +123,7 @@ def test_f64_helpers_give_the_plain_bits(oracle_mod, tmp_path):
     assert r.returncode == 0, r.stdout
 
 
-TILES = [(16, 32), (8, 32)]
+TILES = [(16, 32), (8, 32), (8, 16), (4, 16), (4, 8)]
 
 
 def _film(rows, cols, seed, holes):
@@ -168,3 +168,13 @@ def test_step64_tiles_match_the_oracle(oracle_mod, sw2d_mod, tile, shape):
         for k in ("rain_in", "source_in", "evap_out", "outflow", "clamp_gain"):
             assert bg[k] == pytest.approx(bo[k], rel=1e-12, abs=1e-14), k  # sums in another order
         g.close()
+
+
+@pytest.mark.gpu
+def test_step64_tile_rule(sw2d_mod):
+    """The smallest tile that gives at most one CTA per SM; a caller's tile is
+    kept."""
+    for rows, cols, kw, name in ((64, 64, {}, "4,8"), (117, 131, {}, "8,16"), (512, 512, {}, "16,32"),
+                                 (64, 64, dict(tile_h=8, tile_w=32), "8,32")):
+        with sw2d_mod.Solver(rows=rows, cols=cols, dx=1.0, dy=1.0, **kw) as g:
+            assert g.describe().startswith("step_kernel<double,%s>" % name), g.describe()
