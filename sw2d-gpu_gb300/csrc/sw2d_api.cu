@@ -289,11 +289,10 @@ int upload_table(sw2d_handle *h, DevBuf &b, const T *src, size_t n) {
 }
 
 // Strip height of the FP32 streaming kernel when the caller leaves it to the
-// library.  Units (column tile x strip) are sized so that a whole number of
-// waves of resident warps covers the grid -- a partial last wave leaves SMs
-// idle -- using the fewest waves whose strips are at most kMaxAutoStrip rows
-// (longer strips measured slower on GB300 at 4096^2 and up), and at least 16
-// rows, since each strip recomputes 7 halo rows.
+// library: what one wave of resident warps runs fastest (one_wave_strip), and
+// for grids whose one-wave strips would exceed kMaxAutoStrip rows (longer
+// strips measured slower on GB300 at 4096^2 and up) the fewest whole waves --
+// a partial last wave leaves SMs idle -- whose strips do not.
 constexpr long long kMaxAutoStrip = 160;
 
 // Longest one-wave strip for which the library picks several iterations per
@@ -305,11 +304,44 @@ constexpr int kAutoPipeMaxStrip = 32;
 // 80.7 / 80.6 / 79.4 / 84.0 us per iteration.
 constexpr int kStripSkew = 20;
 
-int auto_strip(int rows, int tiles_w, int variant, int device) {
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const int per_sm = stream_ctas_per_sm(variant);
-    const long long resident = (long long)(sms > 0 ? sms : 152) * (per_sm > 0 ? per_sm : 1) * stream_warps(variant);
+// Time of a row step of the streaming unit by the warps sharing an SM, relative
+// to a lightly loaded one (0.73-0.79 us for the uniform form): measured over
+// 2 .. 20 warps per SM and strips of 2, 8 and 16 rows it stays there up to 8
+// warps, is 0.86 us at 10, and 1.1-1.25 us from 12 on.  The storm and
+// rain-factor forms take 1.2 times as long at every load.
+int row_cost(long long warps_per_sm) { return warps_per_sm <= 8 ? 100 : (warps_per_sm <= 10 ? 112 : 150); }
+
+// The strip height of at least `least` rows that makes one wave of warps
+// finish first: a warp runs its rows plus 7 warm-up rows at row_cost, so a grid
+// that does not fill the GPU is cut into short strips (more warm-up rows in
+// all, but on warps that would otherwise be idle), down to one row.  us per
+// iteration, strips of 16 rows against the choice: 96 x 128 26.1 -> 14.1,
+// 256 x 256 26.2 -> 15.7, 512 x 512 25.3 -> 19.7.  0 when no height fits one
+// wave.
+int one_wave_strip(int rows, int tiles_w, long long sms, int ctas_per_sm, int warps, int least) {
+    const long long tw = tiles_w > 0 ? tiles_w : 1, nw = warps;
+    long long best = 0;
+    int best_sh = 0;
+    for (int sh = least; sh <= kMaxAutoStrip; sh++) {
+        const long long strips = (rows + sh - 1) / sh, ctas = (tw * strips + nw - 1) / nw;
+        if (tw * strips > sms * ctas_per_sm * nw || (strips > 1 && rows / strips < least)) continue;
+        const long long cost = ((rows + strips - 1) / strips + 7) * row_cost((ctas + sms - 1) / sms * nw);
+        if (!best_sh || cost < best) {
+            best = cost;
+            best_sh = sh;
+        }
+        if (sh >= rows) break;
+    }
+    return best_sh;
+}
+
+// least: 1, or under the fixed time step the pipelined launches' shortest
+// strip, so that a run's FP32 budget sums do not depend on steps_per_launch.
+int auto_strip(int rows, int tiles_w, int variant, int sms, int least) {
+    const int per_sm = stream_ctas_per_sm(variant) > 0 ? stream_ctas_per_sm(variant) : 1;
+    const int one = one_wave_strip(rows, tiles_w, sms, per_sm, stream_warps(variant), least);
+    if (one > 0) return one;
+    const long long resident = (long long)sms * per_sm * stream_warps(variant);
     const long long tw = tiles_w > 0 ? tiles_w : 1;
     if (resident < tw) return 64;
     long long sh = rows;
@@ -320,15 +352,16 @@ int auto_strip(int rows, int tiles_w, int variant, int device) {
     return (int)(sh < 16 ? 16 : sh);
 }
 
-// Strip height of the pipelined launches: every unit must be resident at
-// once (one wave), so strips are the shortest that fit one wave, at least 16
-// rows.  0 when even one-row strips would not fit.
-int pipe_strip(int rows, int tiles_w, long long resident) {
+// Strip height of the pipelined launches: every unit must be resident at once
+// (one wave), in strips of at least the rows their neighbour set needs; the
+// shortest that fit when they are longer than one_wave_strip looks at.  0 when
+// even one-row strips would not fit.
+int pipe_strip(int rows, int tiles_w, long long sms, int ctas_per_sm, int warps) {
     const long long tw = tiles_w > 0 ? tiles_w : 1;
-    const long long per_tile = resident / tw;  // strips per column tile that one wave holds
+    const long long per_tile = sms * ctas_per_sm * warps / tw;  // strips per column tile that one wave holds
     if (per_tile < 1) return 0;
-    const long long sh = (rows + per_tile - 1) / per_tile;
-    return (int)(sh < 16 ? 16 : sh);
+    const int one = one_wave_strip(rows, tiles_w, sms, ctas_per_sm, warps, stream_pipe_min_strip());
+    return one > 0 ? one : (int)((rows + per_tile - 1) / per_tile);
 }
 
 }  // namespace
@@ -453,10 +486,9 @@ int sw2d_create(const sw2d_config *cfg, sw2d_handle **out) {
         // several iterations per launch under the fixed time step, when every
         // unit fits one wave of resident warps (asked for: an error otherwise)
         if (cfg->dt_mode == SW2D_DT_FIXED && cfg->steps_per_launch != 1) {
-            int sms = 0;
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg->device);
-            const long long resident = (long long)sms * stream_pipe_ctas_per_sm(h->variant) * nw;
-            const int psh = sh > 0 ? sh : pipe_strip(cfg->rows, h->stream_tiles_w, resident);
+            const int per_sm = stream_pipe_ctas_per_sm(h->variant);
+            const long long resident = (long long)h->sms * per_sm * nw;
+            const int psh = sh > 0 ? sh : pipe_strip(cfg->rows, h->stream_tiles_w, h->sms, per_sm, nw);
             const long long strips = psh > 0 ? (cfg->rows + psh - 1) / psh : 0;
             const long long units = (long long)h->stream_tiles_w * strips;
             // strips split the rows evenly: the shortest has rows / strips rows
@@ -476,7 +508,8 @@ int sw2d_create(const sw2d_config *cfg, sw2d_handle **out) {
                 return bail(SW2D_ERR_INVALID_ARG);
             }
         }
-        if (sh <= 0) sh = auto_strip(cfg->rows, h->stream_tiles_w, h->variant, cfg->device);
+        if (sh <= 0) sh = auto_strip(cfg->rows, h->stream_tiles_w, h->variant, h->sms,
+                            cfg->dt_mode == SW2D_DT_FIXED ? stream_pipe_min_strip() : 1);
         h->strip_h = sh;
         h->stream_units = h->stream_tiles_w * ((cfg->rows + sh - 1) / sh);
         h->nblocks = (h->stream_units + nw - 1) / nw;
@@ -484,9 +517,7 @@ int sw2d_create(const sw2d_config *cfg, sw2d_handle **out) {
             // one launch per iteration filling one wave of resident warps: the
             // warp scheduler favours the CTAs launched first, so their strips
             // get more rows (measured at 2048^2: 79.4 against 80.7 us)
-            int sms = 0;
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg->device);
-            const long long resident = (long long)sms * stream_ctas_per_sm(h->variant) * nw;
+            const long long resident = (long long)h->sms * stream_ctas_per_sm(h->variant) * nw;
             const int strips = (cfg->rows + sh - 1) / sh;
             if (h->stream_units <= resident && 10LL * h->stream_units >= 9 * resident && cfg->rows / strips >= 16)
                 h->strip_skew = kStripSkew;

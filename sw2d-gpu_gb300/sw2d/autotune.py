@@ -29,7 +29,7 @@ from typing import Callable, Optional
 
 import numpy as np
 
-STRIPS = (16, 24, 32, 48, 64, 96, 128)
+STRIPS = (1, 2, 4, 8, 16, 24, 32, 48, 64, 96, 128)
 VARIANTS = (0, 1, 2, 3, 4, 5)
 CHUNKS = (12, 24, 48, 96)
 OUT_COLS = 27            # output columns of one streaming warp
@@ -38,7 +38,7 @@ RESIDENT_WARPS_PER_SM = (16, 20, 24)  # resident warps per SM of the kernel buil
 
 # Variant ids index the kernel builds of the library; a cache written for
 # another table of builds is not reused.
-TABLE_VERSION = "stream-v5"
+TABLE_VERSION = "stream-v6"
 
 
 def wave_strips(rows: int, cols: int, sms: int = 152, waves=(1, 2, 3, 4), warps_per_sm=RESIDENT_WARPS_PER_SM):
