@@ -29,6 +29,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
 UNITS = {
     "step_f64.cu": ["--fmad=false"],
     "step_f32.cu": ["--use_fast_math"],
+    "pipe_f32.cu": ["--use_fast_math"],  # same flags as step_f32.cu: the same bits
     # the one device function here (the per-launch plan) must round like the
     # oracle: no contraction in device or host code
     "sw2d_api.cu": ["--fmad=false", "-Xcompiler", "-ffp-contract=off"],

@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(NWARP * 32, MINB) batch_step_kernel(const Batc
             // batched scenarios take neither a storm nor point sources nor rain
             // factors (sw2d_batch_add accepts none), so the uniform-forcing unit
             const int r0 = rs * S.strip_h;
-            stream_unit<UNR, false, false>(V, ct, r0, min(r0 + S.strip_h, V.rows), lane, s_sr[wid], s_sc[wid],
+            stream_unit<UNR, false, kFormUniform>(V, ct, r0, min(r0 + S.strip_h, V.rows), lane, s_sr[wid], s_sc[wid],
                                            s_q0[wid], s_q1[wid], A);
             warp_reduce_acc(A);
             if (lane == 0) {

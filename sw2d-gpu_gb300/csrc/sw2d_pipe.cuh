@@ -136,7 +136,7 @@ static __global__ void pipe_plan_kernel(const GridDesc G, const ForcingDesc F, c
     if (j == 0) words[0] = (unsigned)s_count;
 }
 
-template <int NWARP, int MINB, int UNR, bool RAINW, bool GEN>
+template <int NWARP, int MINB, int UNR, bool RAINW, int FORM>
 __global__ void __launch_bounds__(NWARP * 32, MINB)
     stream_pipe_kernel(const GridDesc G, const ForcingDesc F, const StateBufs<float> S, const Thr<float> T,
                        Clock *__restrict__ clk, const Control *__restrict__ ctl, const int slot,
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(NWARP * 32, MINB)
             StreamAcc A;
             A.rain = A.src = A.ev = A.out = A.clamp = A.cm = 0.f;
             A.bad = A.too_many_sources = false;
-            stream_unit<UNR, RAINW, GEN, false, true>(V, ct, r0, r1, lane, s_sr[wid], s_sc[wid], s_q0[wid],
+            stream_unit<UNR, RAINW, FORM, false, true>(V, ct, r0, r1, lane, s_sr[wid], s_sc[wid], s_q0[wid],
                                                       s_q1[wid], A, nullptr, 0, nullptr, nullptr,
                                                       P.flags + SH.units + unit, (unsigned)(j + 1));
             warp_reduce_acc(A);
