@@ -125,21 +125,20 @@ __global__ void __launch_bounds__(NWARP * 32, MINB) batch_step_kernel(const Batc
             V.dx = S.G.dx;
             V.dy = S.G.dy;
             StreamAcc A;
-            A.rain = A.src = A.ev = A.out = A.clamp = A.cm = 0.f;
-            A.bad = A.too_many_sources = false;
+            acc_clear(A);
             const int ct = ue.y % S.tiles_w, rs = ue.y / S.tiles_w;
             // batched scenarios take neither a storm nor point sources nor rain
             // factors (sw2d_batch_add accepts none), so the uniform-forcing unit
             const int r0 = rs * S.strip_h;
             stream_unit<UNR, false, kFormUniform>(V, ct, r0, min(r0 + S.strip_h, V.rows), lane, s_sr[wid], s_sc[wid],
                                            s_q0[wid], s_q1[wid], A);
-            warp_reduce_acc(A);
+            warp_reduce_acc<true>(A);
             if (lane == 0) {
                 const double area = S.G.dx * S.G.dy, scale = ci.plan.d.dt2 * area;
                 double v[B_N];
-                v[B_RAIN] = (double)A.rain * scale;
+                v[B_RAIN] = acc_rain((double)A.rain, A.n_act, A.n_hi, ci.plan.f, S.G.sf) * scale;
                 v[B_SRC] = (double)A.src * scale;
-                v[B_EV] = (double)A.ev * scale;
+                v[B_EV] = acc_ev((double)A.ev, A.n_hi, ci.plan.f) * scale;
                 v[B_OUT] = (double)A.out * ci.plan.d.dt2 * S.G.dy;
                 v[B_CLAMP] = (double)A.clamp * area;
                 accumulate_slot(S.clk[slot_out], ue.y % kBuckets, v, (double)A.cm, A.bad);

@@ -424,13 +424,20 @@ __device__ inline void carry_slot(const Clock &ci, Clock &co, Clock &cn) {
     clear_slot_accumulators(cn);
 }
 
-// One CTA's contribution (one thread calls it): budget sums [m^3 already
-// scaled], CFL bound, non-finite flag.
-__device__ inline void accumulate_slot(Clock &co, int bucket, const double v[B_N], double cmax, bool bad) {
-    for (int k = 0; k < B_N; k++)
-        if (v[k] != 0.0) atomicAdd(&co.stepb[k][bucket], v[k]);
+// One CTA's contribution (one thread calls each): CFL bound and flags, which
+// the launch's last CTA reads, and budget sums [m^3 already scaled], which with
+// the deferred fold only the next launch reads.
+__device__ __forceinline__ void accumulate_cmax(Clock &co, int bucket, double cmax, bool bad) {
     if (cmax > 0.0) atomicMax(&co.cmaxb[bucket], (unsigned long long)__double_as_longlong(cmax));
     if (bad) atomicOr(&co.nonfinite, 1u);
+}
+__device__ __forceinline__ void accumulate_budgets(Clock &co, int bucket, const double v[B_N]) {
+    for (int k = 0; k < B_N; k++)
+        if (v[k] != 0.0) atomicAdd(&co.stepb[k][bucket], v[k]);
+}
+__device__ inline void accumulate_slot(Clock &co, int bucket, const double v[B_N], double cmax, bool bad) {
+    accumulate_budgets(co, bucket, v);
+    accumulate_cmax(co, bucket, cmax, bad);
 }
 
 // Finalises slot `co` once every contribution of the launch is in: sums the
@@ -581,7 +588,9 @@ __device__ inline void finalize_slot_deferred_warp(const int lane, const Clock &
 // finish_cta_warp with the deferred fold: the first CTA to finish folds the
 // slot this launch read (written by the previous launch), the last
 // finalises the slot this launch wrote.  clk, and the three slot indices as
-// in the step kernels.
+// in the step kernels.  Called after accumulate_cmax; another warp adds the
+// CTA's budgets meanwhile (accumulate_budgets: FP64 arithmetic and atomics that
+// need not lie on the path to the last CTA's ticket).
 __device__ inline void finish_cta_deferred_warp(const int lane, Clock *clk, const int slot, const int slot_out,
                                                 const int slot_nx, const Plan &pl, const Control &ctl,
                                                 const GridDesc &G, const ForcingDesc &F) {

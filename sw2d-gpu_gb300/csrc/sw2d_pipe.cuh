@@ -233,17 +233,16 @@ __global__ void __launch_bounds__(NWARP * 32, MINB)
             V.dx = G.dx;
             V.dy = G.dy;
             StreamAcc A;
-            A.rain = A.src = A.ev = A.out = A.clamp = A.cm = 0.f;
-            A.bad = A.too_many_sources = false;
+            acc_clear(A);
             stream_unit<UNR, RAINW, FORM, false, true>(V, ct, r0, r1, lane, s_sr[wid], s_sc[wid], s_q0[wid],
                                                       s_q1[wid], A, nullptr, 0, nullptr, nullptr,
                                                       P.flags + SH.units + unit, (unsigned)(j + 1));
-            warp_reduce_acc(A);
+            warp_reduce_acc<!RAINW && FORM == kFormUniform>(A);
             if (lane == 0) {
                 const double scale = pl.d.dt2 * area;
-                s_acc[wid][B_RAIN] += (double)A.rain * scale;
+                s_acc[wid][B_RAIN] += acc_rain((double)A.rain, A.n_act, A.n_hi, pl.f, G.sf) * scale;
                 s_acc[wid][B_SRC] += (double)A.src * scale;
-                s_acc[wid][B_EV] += (double)A.ev * scale;
+                s_acc[wid][B_EV] += acc_ev((double)A.ev, A.n_hi, pl.f) * scale;
                 s_acc[wid][B_OUT] += (double)A.out * pl.d.dt2 * G.dy;
                 s_acc[wid][B_CLAMP] += (double)A.clamp * area;
                 s_cm[wid] = A.cm;  // the CFL bound of the launch's final state

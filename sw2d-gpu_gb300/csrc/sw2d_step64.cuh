@@ -639,8 +639,12 @@ __global__ void __launch_bounds__(NT, MINB)
         s_cnt[wid][1] = n_lo;
     }
     __syncthreads();
-    if (tid >= 32) return;
-    if (tid == 0) {
+    // warp 0 takes what the last CTA of the launch needs to its ticket, warp 1
+    // the budgets, which only the next launch reads
+    if (wid == 0) {
+        if (lane == 0) accumulate_cmax(clk[slot_out], blockIdx.x % kBuckets, d_from_bits(s_cm), any_bad);
+        finish_cta_deferred_warp(lane, clk, slot, slot_out, slot_nx, pl, *ctl, G, F);
+    } else if (tid == 32) {
         double acc[4] = {0.0, 0.0, 0.0, 0.0};
         int c_hi = 0, c_lo = 0;
         for (int w = 0; w < NW; w++) {
@@ -659,9 +663,8 @@ __global__ void __launch_bounds__(NT, MINB)
         v[B_EV] = LS.ev1 * (double)c_hi * scale;
         v[B_OUT] = acc[2] * pl.d.dt2 * G.dy;
         v[B_CLAMP] = acc[3] * area;
-        accumulate_slot(clk[slot_out], blockIdx.x % kBuckets, v, d_from_bits(s_cm), any_bad);
+        accumulate_budgets(clk[slot_out], blockIdx.x % kBuckets, v);
     }
-    finish_cta_deferred_warp(lane, clk, slot, slot_out, slot_nx, pl, *ctl, G, F);
 }
 
 }  // namespace sw2d

@@ -165,12 +165,30 @@ __device__ __forceinline__ T *wuni(T *p) {
     return reinterpret_cast<T *>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(p), 0));
 }
 
-// Per-warp results of a strip (per lane until reduced).
+// Per-warp results of a strip (per lane until reduced).  Under uniform forcing
+// rain and evaporation are two values per launch, by whether the old depth is
+// above EV_WL_min, so the unit counts cells (n_act active, n_hi of them above)
+// instead of adding FP32 rates: exact, whatever the strips are.
 struct StreamAcc {
     float rain, src, ev, out, clamp, cm;
+    int n_act, n_hi;
     bool bad;
     bool too_many_sources;
 };
+__device__ __forceinline__ void acc_clear(StreamAcc &A) {
+    A.rain = A.src = A.ev = A.out = A.clamp = A.cm = 0.f;
+    A.n_act = A.n_hi = 0;
+    A.bad = A.too_many_sources = false;
+}
+// The rain and evaporation rates summed over cells, from the reduced counts and
+// sums, with the FP32 rates the unit applied.
+__device__ __forceinline__ double acc_rain(double sum, int n_act, int n_hi, const LaunchScalars<float> &LS,
+                                           const GridScalars<float> &GS) {
+    return sum + (double)n_hi * (double)(LS.rr1 * GS.pct_hi) + (double)(n_act - n_hi) * (double)(LS.rr1 * GS.pct_lo);
+}
+__device__ __forceinline__ double acc_ev(double sum, int n_hi, const LaunchScalars<float> &LS) {
+    return sum + (double)n_hi * (double)LS.ev1;
+}
 
 // Advances column tile `ct`, rows r0 .. r1-1 (a strip) of the
 // scenario in V.  s_sr/s_sc/s_q0/s_q1 are this warp's slots for local point
@@ -593,9 +611,14 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
                 A.out += us;
             }
             if (m3) {
-                A.rain += rr1 * pct1;
-                A.src += ql1;
-                A.ev += ev1;
+                if constexpr (FORM == kFormUniform && !RAINW) {
+                    A.n_act++;
+                    A.n_hi += h3 >= gt_ev ? 1 : 0;
+                } else {
+                    A.rain += rr1 * pct1;
+                    A.src += ql1;
+                    A.ev += ev1;
+                }
                 A.clamp += clampv;
                 // CFL bound of the new state on the owned faces (extension)
                 if (m4) {
@@ -635,12 +658,20 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
 }
 
 // Warp reduction of a StreamAcc: sums / max / any into lane 0's return.
+// UNIFORM: the uniform-forcing form's counts instead of the rate sums.
+template <bool UNIFORM>
 __device__ __forceinline__ void warp_reduce_acc(StreamAcc &A) {
+    if constexpr (UNIFORM) {
+        A.n_act = __reduce_add_sync(0xffffffffu, A.n_act);
+        A.n_hi = __reduce_add_sync(0xffffffffu, A.n_hi);
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        A.rain += __shfl_xor_sync(0xffffffffu, A.rain, o);
-        A.src += __shfl_xor_sync(0xffffffffu, A.src, o);
-        A.ev += __shfl_xor_sync(0xffffffffu, A.ev, o);
+        if constexpr (!UNIFORM) {
+            A.rain += __shfl_xor_sync(0xffffffffu, A.rain, o);
+            A.src += __shfl_xor_sync(0xffffffffu, A.src, o);
+            A.ev += __shfl_xor_sync(0xffffffffu, A.ev, o);
+        }
         A.out += __shfl_xor_sync(0xffffffffu, A.out, o);
         A.clamp += __shfl_xor_sync(0xffffffffu, A.clamp, o);
         A.cm = fmaxf(A.cm, __shfl_xor_sync(0xffffffffu, A.cm, o));
