@@ -65,33 +65,41 @@ __device__ inline void write_status(const Clock &c, ScenarioStatus *st) {
     st->status = c.status;
 }
 
+// Reads the cache lines of a scenario's descriptor into L1 (one line per lane).
+__device__ __forceinline__ void prefetch_scenario(const ScenarioDev *S, int lane) {
+    if (lane * 128 < (int)sizeof(ScenarioDev))
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char *>(S) + lane * 128));
+}
+
 template <int NWARP, int MINB, int UNR>
 __global__ void __launch_bounds__(NWARP * 32, MINB) batch_step_kernel(const BatchDev B, const int slot) {
-    // Launched as a programmatic dependent of the previous iteration: wait
-    // until that grid has completed and its writes are visible (the queue
-    // head, every scenario's state and clock), then let the next iteration's
-    // grid be scheduled; its CTAs wait here the same way
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    __shared__ int s_sr[NWARP][kStreamMaxSrc], s_sc[NWARP][kStreamMaxSrc];
-    __shared__ float s_q0[NWARP][kStreamMaxSrc], s_q1[NWARP][kStreamMaxSrc];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int slot_out = slot == 2 ? 0 : slot + 1;
     const int slot_nx = slot == 0 ? 2 : slot - 1;
+    // Every warp starts on a unit of its own and pulls further ones from the
+    // queue.  With at most one unit per warp the units are dealt out across the
+    // CTAs first, so that they spread over the SMs.
+    const int warps = (int)gridDim.x * NWARP, n_units = B.hdr->n_units;
+    unsigned u = n_units <= warps ? wid * gridDim.x + blockIdx.x : blockIdx.x * NWARP + wid;
+    int2 ue = make_int2(0, 0);
+    if (u < (unsigned)n_units) {
+        ue = B.units[u];
+        prefetch_scenario(B.scen + ue.x, lane);
+    }
+    // Launched as a programmatic dependent of the previous iteration: the unit
+    // table and the descriptors are the host's, but the queue head, every
+    // scenario's state and clock are that grid's, so wait until it has completed
+    // and its writes are visible, then let the next iteration's grid be
+    // scheduled; its CTAs wait here the same way
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (blockIdx.x == 0 && threadIdx.x == 0) B.hdr->head[slot_out] = 0u;  // queue of the next launch
-    const int n_units = B.hdr->n_units;
-    // with fewer units than warps, the warps past the unit count would only
-    // find the queue empty: the first n_units warps pull every unit
-    if ((int)blockIdx.x * NWARP + wid >= n_units) return;
-    for (;;) {
-        unsigned u = 0;
-        if (lane == 0) u = atomicAdd(&B.hdr->head[slot], 1u);
-        u = __shfl_sync(0xffffffffu, u, 0);
-        if (u >= (unsigned)n_units) break;
-        const int2 ue = B.units[u];
+    while (u < (unsigned)n_units) {
         const ScenarioDev &S = B.scen[ue.x];
         const Clock &ci = S.clk[slot];
         const int run = ci.plan.run;
+        StreamAcc A;
+        acc_clear(A);
         if (run) {
             StreamView V;
             const int b = ci.buf;
@@ -124,40 +132,51 @@ __global__ void __launch_bounds__(NWARP * 32, MINB) batch_step_kernel(const Batc
             V.t1 = ci.plan.t1;
             V.dx = S.G.dx;
             V.dy = S.G.dy;
-            StreamAcc A;
-            acc_clear(A);
             const int ct = ue.y % S.tiles_w, rs = ue.y / S.tiles_w;
             // batched scenarios take neither a storm nor point sources nor rain
             // factors (sw2d_batch_add accepts none), so the uniform-forcing unit
             const int r0 = rs * S.strip_h;
-            stream_unit<UNR, false, kFormUniform>(V, ct, r0, min(r0 + S.strip_h, V.rows), lane, s_sr[wid], s_sc[wid],
-                                           s_q0[wid], s_q1[wid], A);
+            stream_unit<UNR, false, kFormUniform>(V, ct, r0, min(r0 + S.strip_h, V.rows), lane, nullptr, nullptr,
+                                                  nullptr, nullptr, A);
             warp_reduce_acc<true>(A);
-            if (lane == 0) {
-                const double area = S.G.dx * S.G.dy, scale = ci.plan.d.dt2 * area;
-                double v[B_N];
-                v[B_RAIN] = acc_rain((double)A.rain, A.n_act, A.n_hi, ci.plan.f, S.G.sf) * scale;
-                v[B_SRC] = (double)A.src * scale;
-                v[B_EV] = acc_ev((double)A.ev, A.n_hi, ci.plan.f) * scale;
-                v[B_OUT] = (double)A.out * ci.plan.d.dt2 * S.G.dy;
-                v[B_CLAMP] = (double)A.clamp * area;
-                accumulate_slot(S.clk[slot_out], ue.y % kBuckets, v, (double)A.cm, A.bad);
-                if (A.too_many_sources) atomicOr(&S.clk[slot_out].status, (unsigned)ST_TOO_MANY_LOCAL_SOURCES);
+            if (lane == 0) accumulate_cmax(S.clk[slot_out], ue.y % kBuckets, (double)A.cm, A.bad);
+            // the budgets, one per lane (B_RAIN .. B_CLAMP; no sources here): FP64
+            // operations have long latencies and this warp is on the way to its ticket
+            if (lane < B_N && lane != B_SRC) {
+                const LaunchScalars<float> &L = ci.plan.f;
+                const double area = S.G.dx * S.G.dy, dt2 = ci.plan.d.dt2;
+                const float rate = lane == B_RAIN ? L.rr1 * S.G.sf.pct_hi : (lane == B_EV ? L.ev1 : 0.f);
+                const float rate_lo = lane == B_RAIN ? L.rr1 * S.G.sf.pct_lo : 0.f;
+                const float sum = lane == B_OUT ? A.out : (lane == B_CLAMP ? A.clamp : 0.f);
+                const double per = lane == B_CLAMP ? area : dt2 * (lane == B_OUT ? S.G.dy : area);
+                const double v = (double)sum + (double)A.n_hi * (double)rate + (double)(A.n_act - A.n_hi) * (double)rate_lo;
+                if (v != 0.0) atomicAdd(&S.clk[slot_out].stepb[lane][ue.y % kBuckets], v * per);
             }
         }
+        // the scenario's first unit to finish folds the budgets of the previous
+        // iteration, its last finalises this one (finish_cta_deferred_warp)
         unsigned ticket = 0u;
         if (lane == 0) {
             __threadfence();
             ticket = atomicAdd(&S.clk[slot_out].done_blocks, 1u);
         }
         ticket = __shfl_sync(0xffffffffu, ticket, 0);
-        if (ticket == (unsigned)S.nunits - 1u) {  // the scenario's last unit: the whole warp finalises
+        if (run && ticket == 0u) fold_slot_warp(lane, S.clk[slot_nx], S.clk[slot]);
+        if (ticket == (unsigned)S.nunits - 1u) {
             __threadfence();
-            if (run) finalize_slot_warp(lane, ci, S.clk[slot_out], S.clk[slot_nx], ci.plan, S.ctl, S.G, S.F);
-            else if (lane == 0) carry_slot(ci, S.clk[slot_out], S.clk[slot_nx]);
+            if (run)
+                finalize_slot_deferred_warp(lane, ci, S.clk[slot_out], S.clk[slot_nx], ci.plan, S.ctl, S.G, S.F);
+            else
+                carry_slot_deferred_warp(lane, S.clk, slot, slot_out, slot_nx);
             __syncwarp();
             if (lane == 0) write_status(S.clk[slot_out], S.status);
         }
+        // the next unit: the queue starts behind the warps' own
+        if (n_units <= warps) break;
+        unsigned k = 0;
+        if (lane == 0) k = atomicAdd(&B.hdr->head[slot], 1u);
+        u = (unsigned)warps + __shfl_sync(0xffffffffu, k, 0);
+        if (u < (unsigned)n_units) ue = B.units[u];
         __syncwarp();
     }
 }
