@@ -273,14 +273,16 @@ __global__ void __launch_bounds__(NT, MINB)
             if (gi == rows) hm = s_h[idx - RW];
             else if (gi == 0) hm = h;
             else hm = d_half(h + s_h[idx - RW]);
-            s_uu[idx] = d_ge_pos(hm, ge_th) ? d_div(s_umo[idx], hm) : 0.0;
+            const double q = s_umo[idx];  // (at rest the division is left out)
+            s_uu[idx] = d_ge_pos(hm, ge_th) && !d_is_zero(q) ? d_div(q, hm) : 0.0;
         }
         if (c >= 1) {
             double hn;
             if (gj == cols) hn = s_h[idx - 1];
             else if (gj == 0) hn = h;
             else hn = d_half(h + s_h[idx - 1]);
-            s_vv[idx] = d_ge_pos(hn, ge_th) ? d_div(s_vno[idx], hn) : 0.0;
+            const double q = s_vno[idx];
+            s_vv[idx] = d_ge_pos(hn, ge_th) && !d_is_zero(q) ? d_div(q, hn) : 0.0;
         }
     }
     __syncthreads();
@@ -604,14 +606,20 @@ __global__ void __launch_bounds__(NT, MINB)
     const bool any_bad = __syncthreads_or(bad);
     const float bar = __uint_as_float(s_est) * (1.f - kMargin);
     if (est >= bar) {
-        unsigned long long cm = 0ull;
+        // a face with the values of the thread's last one (still water of one
+        // depth) is not evaluated again
+        unsigned long long cm = 0ull, seen_q = 1ull, seen_0 = 0ull, seen_1 = 0ull;
         faces([&](double q, double h0, double h1) {
             float hf;
             const float e = estimate(q, h0, h1, hf);
             if (!(e >= bar) || !(hf >= thf * (1.f - kMargin))) return;
+            if ((d_bits(q) << 1) == seen_q && d_bits(h0) == seen_0 && d_bits(h1) == seen_1) return;
+            seen_q = d_bits(q) << 1;
+            seen_0 = d_bits(h0);
+            seen_1 = d_bits(h1);
             const double hm = 0.50 * (h0 + h1);
             if (!d_ge_pos(hm, ge_th)) return;
-            const double v = fabs(d_div(q, hm)) + d_sqrt(g * hm);
+            const double v = (d_is_zero(q) ? 0.0 : fabs(d_div(q, hm))) + d_sqrt(g * hm);
             if (!d_is_nan(v)) cm = d_bits(v) > cm ? d_bits(v) : cm;
         });
         if (cm) atomicMax(&s_cm, cm);
