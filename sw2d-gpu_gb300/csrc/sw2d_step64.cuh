@@ -105,6 +105,9 @@ struct Step64Shape {
     static constexpr size_t kSmem = (size_t)(TH + 7) * (TW + 7) * (kStep64Arrays * sizeof(double) + 3) +
                                     (size_t)(kFaces + kFluxes) * sizeof(uint16_t) + 16;
 };
+// List entries: the element of the tile, and for a face its direction and rule,
+// for a flux its kind.
+constexpr unsigned kItemY = 1u << 13, kItemRule = 14, kItemKind = 14, kItemElem = kItemY - 1;
 
 // Appends `item` of the lanes with `keep` to a list in shared memory (one
 // atomic per warp); every lane of a converged warp calls it.
@@ -115,6 +118,16 @@ __device__ __forceinline__ void append(uint16_t *list, int *count, bool keep, un
     if (lane == 0) base = atomicAdd(count, __popc(bal));
     base = __shfl_sync(0xffffffffu, base, 0);
     if (keep) list[base + __popc(bal & ((1u << lane) - 1u))] = (uint16_t)item;
+}
+
+// The same downwards from `end`.
+__device__ __forceinline__ void append_back(uint16_t *end, int *count, bool keep, unsigned item, int lane) {
+    const unsigned bal = __ballot_sync(0xffffffffu, keep);
+    if (!bal) return;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(count, __popc(bal));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (keep) *(end - (base + __popc(bal & ((1u << lane) - 1u)))) = (uint16_t)item;
 }
 
 template <int TH, int TW, int NT, int MINB>
@@ -140,11 +153,12 @@ __global__ void __launch_bounds__(NT, MINB)
     double *s_rum = s_fy + RN;   // new um before the dry-cell fix
     double *s_rvn = s_rum + RN;
     constexpr int kFaces = Step64Shape<TH, TW>::kFaces, kFluxes = Step64Shape<TH, TW>::kFluxes;
-    static_assert(kFaces < (1 << 14) && kFluxes < (1 << 16), "list entries are 16 bits wide");
+    static_assert(RN <= (int)kItemElem, "list entries are 16 bits wide");
     uint16_t *s_face = reinterpret_cast<uint16_t *>(s_rvn + RN);  // momentum faces from the front, weir faces from the back
     uint16_t *s_flux = s_face + kFaces;
     uint8_t *s_m = reinterpret_cast<uint8_t *>(s_flux + kFluxes);
     uint8_t *s_tx = s_m + RN, *s_ty = s_tx + RN;  // 1: the x- / y-face takes the momentum equation
+    uint8_t *s_dry = s_tx;  // after stage 2: the cell is active and dry after the provisional update
     double *s_hs = s_uu;
 
     __shared__ double s_red[NW][B_N];
@@ -175,6 +189,7 @@ __global__ void __launch_bounds__(NT, MINB)
         const size_t gp = (size_t)gi * pitch + gj;
         s_z[idx] = in ? S.z[gp] : 0.0;
         s_m[idx] = in ? S.mask[gp] : (uint8_t)0;
+        s_tx[idx] = s_ty[idx] = 0;
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -292,50 +307,43 @@ __global__ void __launch_bounds__(NT, MINB)
     // thin film over steep ground dry-bed rules and momentum alternate from face
     // to face, so the faces are sorted into a list for each first.
     constexpr int FH = TH + 4, FW = TW + 4, FN = FH * FW;  // faces: rows/cols [2, TH+6) x [2, TW+6)
-    for (int b0 = wid * 32; b0 < kFaces; b0 += NT) {
-        const int k0 = b0 + lane;
-        int rule = 0;  // 1, 2, 3: dry-bed rules, 4: momentum, 0: no flow
-        if (k0 < kFaces) {
-            const bool isx = k0 < FN;
-            const int k = isx ? k0 : k0 - FN;
-            const int r = 2 + k / FW, c = 2 + (k - (k / FW) * FW);
-            const int p = r * RW + c;
-            const int gi = I0 + r, gj = J0 + c;
-            const int pa = isx ? p - RW : p - 1;  // cell "a" (north / west) of the face; p is "b"
-            const bool inner = isx ? (gi > 0 && gi < rows && (unsigned)gj < (unsigned)cols)
-                                   : ((unsigned)gi < (unsigned)rows && gj > 0 && gj < cols);
-            if (inner) {
-                const double ha = s_h[pa], hb = s_h[p];
-                const bool a_wet = d_ge_pos(ha, gt_th), b_wet = d_ge_pos(hb, gt_th);
-                if (s_m[p] && s_m[pa] && (a_wet || b_wet)) {
-                    rule = 4;
-                    if (d_lt(s_eta[p], s_z[pa])) {  // cu:130: b's surface below a's bed
-                        rule = a_wet ? 1 : 0;
-                    } else if (d_lt(s_eta[pa], s_z[p])) {  // cu:138
-                        rule = b_wet ? 2 : 0;
-                    } else {
-                        // cu:149: exactly one side strictly wet; false for NaN
-                        const bool a_dry = !d_ge_pos(ha, ge_th) && !d_is_nan(ha);
-                        const bool b_dry = !d_ge_pos(hb, ge_th) && !d_is_nan(hb);
-                        if ((b_wet && a_dry) || (b_dry && a_wet)) rule = 3;
-                    }
-                }
-            } else if (isx && gi == rows && (unsigned)gj < (unsigned)cols && G.south_open) {
-                // free outfall (extension): the weir formula of rule 1
-                rule = (s_m[pa] && d_ge_pos(s_h[pa], gt_th)) ? 1 : 0;
-            }
-            (isx ? s_tx : s_ty)[p] = rule == 4;
-            if (rule == 0) (isx ? s_rum : s_rvn)[p] = 0.0;
+    for (int b0 = wid * 32; b0 < FN; b0 += NT) {
+        const int k = b0 + lane;
+        const int r = 2 + k / FW, c = 2 + (k - (k / FW) * FW);
+        const int p = r * RW + c;
+        const int gi = I0 + r, gj = J0 + c;
+        int rule_x = 0, rule_y = 0;  // 1, 2, 3: dry-bed rules, 4: momentum, 0: no flow
+        const bool in = k < FN && (unsigned)gi <= (unsigned)rows && (unsigned)gj < (unsigned)cols;
+        if (in) {
+            const double hb = s_h[p], zb = s_z[p], eb = s_eta[p];
+            const bool b_act = s_m[p] != 0, b_wet = d_ge_pos(hb, gt_th), b_ge = d_ge_pos(hb, ge_th);
+            // cell "a" (north / west) of the face; p is "b"
+            auto rule_of = [&](int pa) -> int {
+                const double ha = s_h[pa];
+                const bool a_wet = d_ge_pos(ha, gt_th);
+                if (!(b_act && s_m[pa] && (a_wet || b_wet))) return 0;
+                if (d_lt(eb, s_z[pa])) return a_wet ? 1 : 0;   // cu:130: b's surface below a's bed
+                if (d_lt(s_eta[pa], zb)) return b_wet ? 2 : 0;  // cu:138
+                // cu:149: exactly one side strictly wet; false for NaN
+                const bool a_dry = !d_ge_pos(ha, ge_th) && !d_is_nan(ha);
+                const bool b_dry = !b_ge && !d_is_nan(hb);
+                return (b_wet && a_dry) || (b_dry && a_wet) ? 3 : 4;
+            };
+            if (gi > 0 && gi < rows) rule_x = rule_of(p - RW);
+            // free outfall (extension): the weir formula of rule 1
+            else if (gi == rows && G.south_open && s_m[p - RW] && d_ge_pos(s_h[p - RW], gt_th)) rule_x = 1;
+            if (gj > 0 && gi < rows) rule_y = rule_of(p - 1);
         }
-        append(s_face, &s_n[0], rule == 4, k0, lane);
-        const unsigned bal = __ballot_sync(0xffffffffu, rule >= 1 && rule <= 3);
-        if (bal) {
-            int base = 0;
-            if (lane == 0) base = atomicAdd(&s_n[1], __popc(bal));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (rule >= 1 && rule <= 3)
-                s_face[kFaces - 1 - (base + __popc(bal & ((1u << lane) - 1u)))] = (uint16_t)(k0 | (rule << 14));
+        if (k < FN) {
+            s_tx[p] = rule_x == 4;
+            s_ty[p] = rule_y == 4;
+            if (rule_x == 0) s_rum[p] = 0.0;
+            if (rule_y == 0) s_rvn[p] = 0.0;
         }
+        append(s_face, &s_n[0], rule_x == 4, p, lane);
+        append(s_face, &s_n[0], rule_y == 4, p | kItemY, lane);
+        append_back(s_face + kFaces - 1, &s_n[1], rule_x >= 1 && rule_x <= 3, p | (rule_x << kItemRule), lane);
+        append_back(s_face + kFaces - 1, &s_n[1], rule_y >= 1 && rule_y <= 3, p | kItemY | (rule_y << kItemRule), lane);
     }
     __syncthreads();
 
@@ -343,57 +351,39 @@ __global__ void __launch_bounds__(NT, MINB)
     // vel (o + s) / 2 + |vel| (s - o) / 2 with vel = (v + w) / 2 is a quarter of
     // (v + w) (o + s) + |v + w| (s - o); for every flux the second factor is
     // (lower-index value) - (higher-index value) of the discharge.
-    //   fx[p], of um through cell p, between the x-faces p and p + RW
-    //   cv[p], of vn through the corner between the y-faces p - RW and p
-    //   cu[p], of um through the corner between the x-faces p - 1 and p
-    //   fy[p], of vn through cell p, between the y-faces p and p + 1
-    constexpr int NA = (FH + 1) * FW, NB = FH * (FW + 1);
-    // item -> kind, element of the flux and of the higher-index face it reads
-    auto flux_item = [&](int k, int &kind, int &po, int &e) {
-        if (k < 2 * NA) {
-            kind = k >= NA ? 1 : 0;  // fx, cv
-            k -= kind ? NA : 0;
-            po = (1 + k / FW) * RW + 2 + (k - (k / FW) * FW);
-            e = po + RW;
-            if (kind) po = e;
-        } else {
-            k -= 2 * NA;
-            kind = k >= NB ? 3 : 2;  // cu, fy
-            k -= kind == 3 ? NB : 0;
-            po = (2 + k / (FW + 1)) * RW + 1 + (k - (k / (FW + 1)) * (FW + 1));
-            e = po + 1;
-            if (kind == 2) po = e;
+    //   kind 0: fx[p], of um through cell p, between the x-faces p and p + RW
+    //   kind 1: cv[p], of vn through the corner between the y-faces p - RW and p
+    //   kind 2: cu[p], of um through the corner between the x-faces p - 1 and p
+    //   kind 3: fy[p], of vn through cell p, between the y-faces p and p + 1
+    // each read by the two faces it lies between where they take the momentum
+    // equation (s_tx and s_ty are 0 outside the faces above).
+    constexpr int EW = TW + 5, EN = (TH + 5) * EW;  // higher-index faces: rows/cols [2, TH+7) x [2, TW+7)
+    for (int b0 = wid * 32; b0 < EN; b0 += NT) {
+        const int k = b0 + lane, e = (2 + k / EW) * RW + 2 + (k - (k / EW) * EW);
+        bool need[4] = {false, false, false, false};
+        if (k < EN) {
+            const bool x = s_tx[e] != 0, y = s_ty[e] != 0;
+            need[0] = x || s_tx[e - RW];
+            need[1] = y || s_ty[e - RW];
+            need[2] = x || s_tx[e - 1];
+            need[3] = y || s_ty[e - 1];
+            const bool u0 = d_is_zero(s_umo[e]), v0 = d_is_zero(s_vno[e]);
+            if (need[0] && u0 && d_is_zero(s_umo[e - RW])) s_fx[e - RW] = 0.0, need[0] = false;
+            if (need[1] && v0 && d_is_zero(s_vno[e - RW])) s_cv[e] = 0.0, need[1] = false;
+            if (need[2] && u0 && d_is_zero(s_umo[e - 1])) s_cu[e] = 0.0, need[2] = false;
+            if (need[3] && v0 && d_is_zero(s_vno[e - 1])) s_fy[e - 1] = 0.0, need[3] = false;
         }
-    };
-    for (int b0 = wid * 32; b0 < kFluxes; b0 += NT) {
-        const int k = b0 + lane;
-        bool need = false;
-        if (k < kFluxes) {
-            int kind, po, e;
-            flux_item(k, kind, po, e);
-            const bool of_um = kind == 0 || kind == 2;
-            const int oq = kind < 2 ? -RW : -1;
-            // read by momentum faces of its own direction on either side
-            const uint8_t *t = of_um ? s_tx : s_ty;
-            // (a face outside rows/cols [2, TH+6) x [2, TW+6) reads nothing)
-            const int r0 = (e + oq) / RW, c0 = (e + oq) - r0 * RW, r1 = e / RW, c1 = e - r1 * RW;
-            const bool in0 = r0 >= 2 && c0 >= 2, in1 = r1 < TH + 6 && c1 < TW + 6;
-            const double *q = of_um ? s_umo : s_vno;
-            if ((in0 && t[e + oq]) || (in1 && t[e])) {
-                need = !(d_is_zero(q[e]) && d_is_zero(q[e + oq]));
-                if (!need) (kind == 0 ? s_fx : kind == 1 ? s_cv : kind == 2 ? s_cu : s_fy)[po] = 0.0;
-            }
-        }
-        append(s_flux, &s_n[2], need, k, lane);
+#pragma unroll
+        for (int q = 0; q < 4; q++) append(s_flux, &s_n[2], need[q], (unsigned)e | (q << kItemKind), lane);
     }
     __syncthreads();
     for (int i = tid; i < s_n[2]; i += NT) {
-        int kind, po, e;
-        flux_item(s_flux[i], kind, po, e);
+        const int it = s_flux[i], kind = it >> kItemKind, e = it & ((1 << kItemKind) - 1);
         const int oq = kind < 2 ? -RW : -1, ov = kind == 0 || kind == 2 ? -RW : -1;
         const double *v = kind < 2 ? s_uu : s_vv, *q = kind == 0 || kind == 2 ? s_umo : s_vno;
+        double *out = kind == 0 ? s_fx - RW : kind == 1 ? s_cv : kind == 2 ? s_cu : s_fy - 1;
         const double qb = q[e], qa = q[e + oq], vel = v[e] + v[e + ov];
-        (kind == 0 ? s_fx : kind == 1 ? s_cv : kind == 2 ? s_cu : s_fy)[po] = vel * (qa + qb) + fabs(vel) * (qa - qb);
+        out[e] = vel * (qa + qb) + fabs(vel) * (qa - qb);
     }
     __syncthreads();
 
@@ -406,12 +396,10 @@ __global__ void __launch_bounds__(NT, MINB)
         if (ch < mom_chunks) {
             const int i = ch * 32 + lane;
             if (i >= n_mom) continue;
-            const int k0 = s_face[i];
-            const bool isx = k0 < FN;
-            const int k = isx ? k0 : k0 - FN;
-            const int r = 2 + k / FW, c = 2 + (k - (k / FW) * FW);
-            const int p = r * RW + c, pa = isx ? p - RW : p - 1;
-            const int gi = I0 + r, gj = J0 + c;
+            const int it = s_face[i], p = it & kItemElem;
+            const bool isx = !(it & kItemY);
+            const int r = p / RW, pa = isx ? p - RW : p - 1;
+            const int gi = I0 + r, gj = J0 + p - r * RW;
             const double ha = s_h[pa], hb = s_h[p], za = s_z[pa], eb = s_eta[p];
             const double mo = isx ? s_umo[p] : s_vno[p];
             const double hsum = hb + ha, hm = d_half(hsum);
@@ -444,10 +432,9 @@ __global__ void __launch_bounds__(NT, MINB)
             // coefficient times depth times sqrt(g depth) or sqrt(2 g depth)
             const int i = (ch - mom_chunks) * 32 + lane;
             if (i >= n_weir) continue;
-            const int it = s_face[kFaces - 1 - i], rule = it >> 14, k0 = it & 0x3fff;
-            const bool isx = k0 < FN;
-            const int k = isx ? k0 : k0 - FN;
-            const int p = (2 + k / FW) * RW + 2 + (k - (k / FW) * FW), pa = isx ? p - RW : p - 1;
+            const int it = s_face[kFaces - 1 - i], rule = it >> kItemRule, p = it & kItemElem;
+            const bool isx = !(it & kItemY);
+            const int pa = isx ? p - RW : p - 1;
             const double ha = s_h[pa], hb = s_h[p];
             double d = rule == 1 ? ha : hb, w = rule == 1 ? 0.5440 : -0.544;
             if (rule == 3) {
@@ -487,7 +474,8 @@ __global__ void __launch_bounds__(NT, MINB)
     for (int k = tid; k < PH * PW; k += NT) {
         const int r = 2 + k / PW, c = 2 + (k - (k / PW) * PW);
         const int p = r * RW + c;
-        double hv = 0.0;
+        double hraw = 0.0;
+        bool dry = false;
         if (s_m[p]) {
             const double ho = s_h[p];
             const bool hi = d_ge_pos(ho, gt_ev);
@@ -500,21 +488,28 @@ __global__ void __launch_bounds__(NT, MINB)
                 if (W) rr = rr * W[(size_t)(I0 + r) * pitch + (J0 + c)];
                 rp = rr * (hi ? pct_hi : pct_lo);
             }
-            hv = d_clamp0(balance(ho, s_rum[p], s_rum[p + RW], s_rvn[p], s_rvn[p + 1], ql, rp, hi ? LS.ev0 : 0.0,
-                                  any_ev0));  // cu:657
+            hraw = balance(ho, s_rum[p], s_rum[p + RW], s_rvn[p], s_rvn[p + 1], ql, rp, hi ? LS.ev0 : 0.0, any_ev0);
+            dry = !d_ge_pos(d_clamp0(hraw), ge_th);  // cu:657
         }
-        s_hs[p] = hv;
+        s_hs[p] = hraw;
+        s_dry[p] = dry;
     }
     __syncthreads();
 
     // ---- stage 4: dry-cell fix per face (cu:695-725) + final depth ----------
-    // corrected face at p (a: the other cell's element): zero if it drains a dry cell
-    auto fix = [&](double q, int p, int a) -> double {
-        if (d_gt_zero(q) && s_m[a] && !d_ge_pos(s_hs[a], ge_th)) return 0.0;
-        if (d_lt_zero(q) && s_m[p] && !d_ge_pos(s_hs[p], ge_th)) return 0.0;
-        return q;
+    // corrected face at p (a: the other cell's element): zero if it drains a dry
+    // cell (a zero stays one, a NaN too); hit: a face of the cell was corrected
+    auto fix = [&](double q, int p, int a, bool &hit) -> double {
+        const bool drains = s_dry[(int)d_hi(q) < 0 ? p : a] != 0;
+        if (!drains || d_is_zero(q) || d_is_nan(q)) return q;
+        hit = true;
+        return 0.0;
     };
+    // With the same forcing at t and t + dt and none of its faces corrected, a
+    // cell's final depth is the provisional one: the same operands.
+    const bool steady = uniform && nloc == 0 && d_bits(LS.rr0) == d_bits(LS.rr1) && d_bits(LS.ev0) == d_bits(LS.ev1);
     const double rp1_hi = LS.rr1 * pct_hi, rp1_lo = LS.rr1 * pct_lo;
+    float *s_hf = reinterpret_cast<float *>(s_fx);  // the fluxes are done with: FP32 depths for stage 5
     int n_hi = 0, n_lo = 0;  // active owned cells above / not above EV_WL_min
     double b_rain = 0.0, b_src = 0.0, b_out = 0.0, b_clamp = 0.0;
     bool bad = false;
@@ -523,8 +518,9 @@ __global__ void __launch_bounds__(NT, MINB)
         const int r = 3 + k / OW, c = 3 + (k - (k / OW) * OW);
         const int p = r * RW + c;
         const int gi = I0 + r, gj = J0 + c;
-        const double un = fix(s_rum[p], p, p - RW), us = fix(s_rum[p + RW], p + RW, p);
-        const double vw = fix(s_rvn[p], p, p - 1), ve = fix(s_rvn[p + 1], p + 1, p);
+        bool hit = false;
+        const double un = fix(s_rum[p], p, p - RW, hit), us = fix(s_rum[p + RW], p + RW, p, hit);
+        const double vw = fix(s_rvn[p], p, p - 1, hit), ve = fix(s_rvn[p + 1], p + 1, p, hit);
         double hv = 0.0, hraw = 0.0;
         const bool act = s_m[p] != 0;
         bool hi = false;
@@ -540,7 +536,8 @@ __global__ void __launch_bounds__(NT, MINB)
                 if (W) rr = rr * W[(size_t)gi * pitch + gj];
                 rp = rr * (hi ? pct_hi : pct_lo);
             }
-            hraw = balance(ho, un, us, vw, ve, ql, rp, hi ? LS.ev1 : 0.0, any_ev1);
+            if (steady && !hit) hraw = s_hs[p];
+            else hraw = balance(ho, un, us, vw, ve, ql, rp, hi ? LS.ev1 : 0.0, any_ev1);
             hv = d_clamp0(hraw);
         }
         s_h[p] = hv;  // the new depth; only this thread reads s_h[p] in this stage
@@ -548,6 +545,7 @@ __global__ void __launch_bounds__(NT, MINB)
         s_vno[p] = vw;
         if (r == TH + 3) s_umo[p + RW] = us;
         if (c == TW + 3) s_vno[p + 1] = ve;
+        s_hf[p] = d_abs_float(hv);
         const bool core = r >= HN && c >= HN && r < TH + HN && c < TW + HN && gi < rows && gj < cols;
         if (core) {
             const size_t gp = (size_t)gi * pitch + gj;
@@ -583,21 +581,20 @@ __global__ void __launch_bounds__(NT, MINB)
             const int p = r * RW + c;
             const int gi = I0 + r, gj = J0 + c;
             if (gi >= rows || gj >= cols || !s_m[p]) continue;
-            const double h = s_h[p];
-            if (gi > 0 && s_m[p - RW]) visit(s_umo[p], h, s_h[p - RW]);
-            if (gi == rows - 1 && G.south_open) visit(s_umo[p + RW], h, h);
-            if (gj > 0 && s_m[p - 1]) visit(s_vno[p], h, s_h[p - 1]);
+            if (gi > 0 && s_m[p - RW]) visit(s_umo[p], p, p - RW);
+            if (gi == rows - 1 && G.south_open) visit(s_umo[p + RW], p, p);
+            if (gj > 0 && s_m[p - 1]) visit(s_vno[p], p, p - 1);
         }
     };
-    auto estimate = [&](double q, double h0, double h1, float &hm) -> float {
-        hm = 0.5f * (d_abs_float(h0) + d_abs_float(h1));
-        return d_abs_float(q) / hm + sqrtf(gf * hm);
+    auto estimate = [&](double q, int p0, int p1, float &hm) -> float {
+        hm = 0.5f * (s_hf[p0] + s_hf[p1]);
+        return __fdividef(d_abs_float(q), hm) + __fsqrt_rn(gf * hm);
     };
     constexpr float kMargin = 1.f / 131072.f;
     float sure = 0.f, est = 0.f;  // over faces certainly / possibly deeper than th
-    faces([&](double q, double h0, double h1) {
+    faces([&](double q, int p0, int p1) {
         float hm;
-        const float e = estimate(q, h0, h1, hm);
+        const float e = estimate(q, p0, p1, hm);
         if (hm >= thf * (1.f + kMargin)) sure = fmaxf(sure, e);
         if (hm >= thf * (1.f - kMargin)) est = fmaxf(est, e);
     });
@@ -609,10 +606,11 @@ __global__ void __launch_bounds__(NT, MINB)
         // a face with the values of the thread's last one (still water of one
         // depth) is not evaluated again
         unsigned long long cm = 0ull, seen_q = 1ull, seen_0 = 0ull, seen_1 = 0ull;
-        faces([&](double q, double h0, double h1) {
+        faces([&](double q, int p0, int p1) {
             float hf;
-            const float e = estimate(q, h0, h1, hf);
+            const float e = estimate(q, p0, p1, hf);
             if (!(e >= bar) || !(hf >= thf * (1.f - kMargin))) return;
+            const double h0 = s_h[p0], h1 = s_h[p1];
             if ((d_bits(q) << 1) == seen_q && d_bits(h0) == seen_0 && d_bits(h1) == seen_1) return;
             seen_q = d_bits(q) << 1;
             seen_0 = d_bits(h0);
