@@ -80,8 +80,8 @@ cudaError_t launch_step64(int th, int tw, int nblocks, int sms, const GridDesc &
     X.gnx = gnx;
     X.gny = gny;
     X.gn = G.sd.g * G.sd.manning * G.sd.manning;
-    X.rdx = G.sd.rdx;
-    X.rdy = G.sd.rdy;
+    X.dx = known_divisor(G.sd.dx);
+    X.dy = known_divisor(G.sd.dy);
     // a programmatic dependent of the launch before it (step64_kernel, stage 0)
     // where one CTA per SM holds the grid: 53.5 against 55.9 us on 64 x 64.  With
     // more, the early CTAs crowd the SMs that drain first (256 CTAs of 8 x 32:

@@ -46,7 +46,7 @@ struct sw2d_handle {
     cudaStream_t stream = nullptr;
     void *h[2] = {nullptr, nullptr}, *um[2] = {nullptr, nullptr}, *vn[2] = {nullptr, nullptr};
     void *z = nullptr, *nman = nullptr;  // nman: FP32 only
-    double *gnx = nullptr, *gny = nullptr;  // g n^2 per face (FP64 with a Manning raster; one allocation, gnx first)
+    double *gnx = nullptr, *gny = nullptr;  // g n^2 per face (FP64 only; one allocation, gnx first)
     uint8_t *mask = nullptr;
     void *rainw = nullptr;  // spatial rain factors (allocated on first use)
     void *dzx = nullptr, *dzy = nullptr;  // bed differences across faces (streaming kernel)
@@ -447,7 +447,14 @@ int sw2d_create(const sw2d_config *cfg, sw2d_handle **out) {
             if (!alloc_field(a, h->real_size)) return bail(SW2D_ERR_OOM);
     }
     if (!alloc_field(&h->z, h->real_size) || !alloc_field((void **)&h->mask, 1)) return bail(SW2D_ERR_OOM);
-    if (!is_f64(h) && !alloc_field(&h->nman, h->real_size)) return bail(SW2D_ERR_OOM);
+    if (is_f64(h)) {
+        void *p = nullptr;  // one allocation for both planes, filled by set_static before anything reads it
+        if (cudaMalloc(&p, 2 * h->plane * sizeof(double)) != cudaSuccess) return bail(SW2D_ERR_OOM);
+        h->gnx = static_cast<double *>(p) + h->origin;
+        h->gny = h->gnx + h->plane;
+    } else if (!alloc_field(&h->nman, h->real_size)) {
+        return bail(SW2D_ERR_OOM);
+    }
     (void)fb;
     h->stage_elems = (size_t)(cfg->rows + 1) * (cfg->cols + 1);
     if (cudaMalloc((void **)&h->stage, h->stage_elems * sizeof(double)) != cudaSuccess) return bail(SW2D_ERR_OOM);
@@ -605,12 +612,6 @@ int sw2d_set_static(sw2d_handle *h, const double *z, const double *manning) {
     if (is_f64(h)) {
         CK(h, launch_pack_static(h->stage, dn, rows, cols, h->pitch, h->cfg.nodata, (double *)h->z, (double *)nullptr,
                                  h->mask, h->stream));
-        if (dn && !h->gnx) {
-            void *p = nullptr;
-            CK(h, cudaMalloc(&p, 2 * h->plane * sizeof(double)));
-            h->gnx = static_cast<double *>(p) + h->origin;
-            h->gny = h->gnx + h->plane;
-        }
         if (dn) CK(h, launch_pack_gn(dn, rows, cols, h->pitch, h->cfg.g, h->gnx, h->gny, h->stream));
     } else
         CK(h, launch_pack_static(h->stage, dn, rows, cols, h->pitch, h->cfg.nodata, (float *)h->z,

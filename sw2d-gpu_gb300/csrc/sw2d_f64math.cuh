@@ -7,7 +7,7 @@
 // friction term); it only takes fewer FP64 instructions for them.  What a
 // helper's fast form does not cover (subnormals, infinities, NaN, operands
 // near the ends of the exponent range) falls through to the plain expression.
-// The forms with host equivalents compile on the host too, where the tests
+// They compile on the host too, where the tests
 // compare them with the plain expressions.
 #pragma once
 
@@ -72,14 +72,18 @@ SW2D_HD unsigned f_bits(float x) {
 #endif
 }
 // FP32 seeds: 1/x and 1/sqrt(x) to about 22 bits (any approximation that good
-// gives the same final bits; see the users)
+// gives the same final bits; see the users).  On the host SW2D_SEED_ULPS puts
+// them off by that many FP32 ulps, so that a test covers the device's.
+#ifndef SW2D_SEED_ULPS
+#define SW2D_SEED_ULPS 0
+#endif
 SW2D_HD float f_rcp_seed(float x) {
 #ifdef __CUDA_ARCH__
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 #else
-    return 1.0f / x;
+    return f_from_bits(f_bits(1.0f / x) + (SW2D_SEED_ULPS));
 #endif
 }
 SW2D_HD float f_rsqrt_seed(float x) {
@@ -88,7 +92,7 @@ SW2D_HD float f_rsqrt_seed(float x) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 #else
-    return 1.0f / std::sqrt(x);
+    return f_from_bits(f_bits(1.0f / std::sqrt(x)) + (SW2D_SEED_ULPS));
 #endif
 }
 
@@ -125,87 +129,151 @@ SW2D_HD double d_half(double x) {
 // fast forms below compute.
 SW2D_HD bool d_mid(double x) { return (d_hi(x) & 0x7ff00000u) - (200u << 20) < (1600u << 20); }
 
-// ---- division ---------------------------------------------------------------
-
-// a / b, correctly rounded.  The reciprocal comes from an FP32 seed of b's
-// mantissa by one third-order Newton step (three FMAs), and the quotient from
-// Markstein's correction q + (a - b q) y (P. Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
-// Dev. 34, 1990): six FP64 instructions.  With a seed error of 2^-22 the
-// reciprocal is off by half an ulp plus 2^-13 ulp at most, and the rounding of
-// the corrected quotient can differ from that of a / b only for a quotient
-// within 2^-53 ulp of a midpoint between two doubles that also meets that
-// excess, about one in 2^60 operand pairs.
-SW2D_HD double d_div_fast(double a, double b) {
-    const unsigned bh = d_hi(b), bl = d_lo(b);
-    const float m = f_from_bits(0x3f800000u | ((bh & 0x000fffffu) << 3) | (bl >> 29));
-    const unsigned s = f_bits(f_rcp_seed(m));
-    // the seed as a double times 2^-exponent(b); b's sign is the caller's: +
-    const double y0 = d_make((s >> 3) + 0x38000000u - ((bh & 0x7ff00000u) - 0x3ff00000u), s << 29);
-    const double e = d_fma(-b, y0, 1.0);
-    const double y = d_fma(y0, d_fma(e, e, e), y0);
-    const double q = a * y;
-    return d_fma(d_fma(-b, q, a), y, q);
-}
-
 #ifdef __CUDACC__
 static __host__ __device__ __noinline__ double d_div_plain(double a, double b) { return a / b; }
-#else
-inline double d_div_plain(double a, double b) { return a / b; }
-#endif
-
-// a / b for b >= 0 (or any b: what is not in mid range takes the plain form)
-SW2D_HD double d_div(double a, double b) {
-    if (d_mid(b) && (d_mid(a) || d_is_zero(a)) && (int)d_hi(b) > 0) return d_div_fast(a, b);
-    return d_div_plain(a, b);
-}
-
-// a / d for a divisor known in advance, rd = 1 / d rounded: the multiplication
-// and two FMAs of N. Brisebarre, J.-M. Muller, S. K. Raina, "Accelerating
-// correctly rounded floating-point division when the divisor is known in
-// advance", IEEE Trans. Comput. 53, 2004.
-SW2D_HD double d_div_const(double a, double d, double rd) {
-    if (d_mid(a) || d_is_zero(a)) {
-        const double q = a * rd;
-        return d_fma(d_fma(-q, d, a), rd, q);
-    }
-    return d_div_plain(a, d);
-}
-
-// ---- square root --------------------------------------------------------------
-
-// sqrt(x), correctly rounded: FP32 seed of 1/sqrt of the mantissa (scaled to
-// [1, 4)), one third-order step on g ~ sqrt(x) and h ~ 1 / (2 sqrt(x)) together
-// (Goldschmidt's coupled form), and Markstein's correction g + (x - g g) h:
-// eight FP64 instructions.
-SW2D_HD double d_sqrt_fast(double x) {
-    const unsigned xh = d_hi(x), xl = d_lo(x);
-    const int e = (int)(xh >> 20) - 1023;       // x = m 2^e, e = 2 k + odd
-    const unsigned odd = (unsigned)e & 1u;
-    const int k = (e - (int)odd) / 2;
-    const float m = f_from_bits((0x3f800000u + (odd << 23)) | ((xh & 0x000fffffu) << 3) | (xl >> 29));
-    const unsigned s = f_bits(f_rsqrt_seed(m));  // in (0.5, 1]
-    const unsigned yh = (s >> 3) + 0x38000000u - ((unsigned)k << 20);
-    const double y = d_make(yh, s << 29), h = d_make(yh - 0x00100000u, s << 29);
-    const double g = x * y;
-    const double r = d_fma(-g, h, 0.5);
-    const double t = d_fma(1.5 * r, r, r);
-    const double g1 = d_fma(g, t, g), h1 = d_fma(h, t, h);
-    return d_fma(d_fma(-g1, g1, x), h1, g1);
-}
-
-#ifdef __CUDACC__
 static __host__ __device__ __noinline__ double d_sqrt_plain(double x) { return sqrt(x); }
 #else
+inline double d_div_plain(double a, double b) { return a / b; }
 inline double d_sqrt_plain(double x) { return std::sqrt(x); }
 #endif
 
-// The roots nearest to a midpoint between two doubles are those of the mantissas
-// one unit away from 1 (and from 2): those take the plain form.
+// ---- division and square root on the integer pipes ---------------------------------
+//
+// The quotient of two 53-bit mantissas as integers: a 22-bit FP32 seed of the
+// reciprocal, one third-order Newton step in 64-bit fixed point (2^-61 relative,
+// never above), floor of the quotient to within one by a high product, and the
+// exact remainder, which fixes the floor and rounds to nearest.  About 60 integer
+// instructions where Newton and Markstein steps on the FP64 pipe take six of 64
+// cycles each, and correctly rounded for every operand pair by construction (a quotient of two doubles is never midway between
+// two doubles).
+
+SW2D_HD unsigned long long mul_hi(unsigned long long a, unsigned long long b) {
+#ifdef __CUDA_ARCH__
+    return __umul64hi(a, b);
+#else
+    return (unsigned long long)(((unsigned __int128)a * b) >> 64);
+#endif
+}
+
+// A seed in (or an ulp or two outside) [1/2, 1) as a 32-bit fraction in [1/2, 1).
+SW2D_HD unsigned seed_fraction(float seed) {
+    const unsigned s = f_bits(seed);
+    return s >= 0x3f800000u ? 0xffffffffu : (s < 0x3f000000u ? 0x80000000u : ((s & 0x7fffffu) | 0x800000u) << 8);
+}
+
+// 2^127 / B for B in [2^63, 2^64), as Y <= 2^64 / m with m = B / 2^63, low by
+// less than 2^-60 of it.
+SW2D_HD unsigned long long recip64(unsigned long long B) {
+    typedef unsigned long long u64;
+    typedef long long i64;
+    const unsigned Bh = (unsigned)(B >> 32), Bl = (unsigned)B;
+    const unsigned Y0 = seed_fraction(f_rcp_seed(f_from_bits(0x3f800000u | ((Bh >> 8) & 0x7fffffu))));
+    // e = 1 - m y0 in units of 2^-63 (|e| < 2^42)
+    const u64 prod = (u64)Bh * Y0 + (((u64)Bl * Y0) >> 32);
+    const i64 e = (i64)(0x8000000000000000ull - prod);
+    // t = e + e^2; y0 (1 + t)
+    const i64 eh = e >> 20;  // |eh| < 2^22
+    const i64 t = e + ((eh * eh) >> 23) - 4;
+    const u64 tu = t < 0 ? (u64)-t : (u64)t;
+    const u64 corr = ((u64)(unsigned)(tu >> 32) * Y0 << 1) + (((u64)(unsigned)tu * Y0) >> 31);
+    const u64 base = (u64)Y0 << 32;
+    return t < 0 ? base - corr - 2ull : base + corr;
+}
+
+// The mantissa quotient: A, B in [2^52, 2^53), Y = recip64(B << 11); the quotient
+// rounded to 53 bits in [2^52, 2^53], and *less = 1 where A < B (exponent one less).
+SW2D_HD unsigned long long quotient53(unsigned long long A, unsigned long long B, unsigned long long Y, int *less) {
+    typedef unsigned long long u64;
+    const int l = A < B ? 1 : 0;
+    const u64 A2 = A << l;
+    u64 Q = mul_hi(A2, Y);
+    u64 r = (A2 << 52) - Q * B;  // exact: 0 <= r < 2 B, as Q is the floor or one less
+    if (r >= B) Q++, r -= B;
+    *less = l;
+    return Q + (2 * r > B ? 1ull : 0ull);
+}
+
+SW2D_HD unsigned long long d_mant(double x) {
+    return (d_bits(x) & 0xfffffffffffffull) | 0x10000000000000ull;
+}
+
+// a / b for b in mid range and positive, a in mid range
+SW2D_HD double d_div_fast(double a, double b) {
+    typedef unsigned long long u64;
+    const u64 B = d_mant(b);
+    int less;
+    const u64 Q = quotient53(d_mant(a), B, recip64(B << 11), &less);
+    const int ea = (int)((d_hi(a) >> 20) & 0x7ffu), eb = (int)(d_hi(b) >> 20);
+    return d_from_bits((d_bits(a) & 0x8000000000000000ull) + ((u64)(ea - eb + 1022 - less) << 52) + Q);
+}
+
+SW2D_HD double d_div(double a, double b) {
+    if (d_mid(b) && (int)d_hi(b) > 0) {
+        if (d_mid(a)) return d_div_fast(a, b);
+        if (d_is_zero(a)) return a;
+    }
+    return d_div_plain(a, b);
+}
+
+// a / d for a divisor known in advance (positive, in mid range): its mantissa, its
+// reciprocal (recip64) and its exponent field.
+struct KnownDivisor {
+    double d;
+    unsigned long long B, Y;
+    int e, ok;
+};
+SW2D_HD KnownDivisor known_divisor(double d) {
+    KnownDivisor k;
+    k.d = d;
+    k.ok = d_mid(d) && (int)d_hi(d) > 0;
+    k.B = d_mant(d);
+    k.Y = recip64(k.B << 11);
+    k.e = (int)(d_hi(d) >> 20);
+    return k;
+}
+SW2D_HD double d_div_known(double a, const KnownDivisor &k) {
+    typedef unsigned long long u64;
+    if (d_is_zero(a)) return a;
+    if (!k.ok || !d_mid(a)) return d_div_plain(a, k.d);
+    int less;
+    const u64 Q = quotient53(d_mant(a), k.B, k.Y, &less);
+    const int ea = (int)((d_hi(a) >> 20) & 0x7ffu);
+    return d_from_bits((d_bits(a) & 0x8000000000000000ull) + ((u64)(ea - k.e + 1022 - less) << 52) + Q);
+}
+
+// sqrt(x), x positive in mid range: the integer root of the mantissa scaled to 106
+// or 107 bits, from a 22-bit seed of 1/sqrt and one third-order step, with the
+// exact remainder (a root is never midway between two doubles).
+SW2D_HD double d_sqrt_fast(double x) {
+    typedef unsigned long long u64;
+    typedef long long i64;
+    const unsigned xh = d_hi(x);
+    const int e = (int)(xh >> 20) - 1023;
+    const unsigned odd = (unsigned)e & 1u;
+    const int k = (e - (int)odd) / 2;
+    const u64 M = d_mant(x) << odd;  // m = M / 2^52 in [1, 4)
+    const unsigned Y0 = seed_fraction(
+        f_rsqrt_seed(f_from_bits((0x3f800000u + (odd << 23)) | ((xh & 0x000fffffu) << 3) | (d_lo(x) >> 29))));
+    // e1 = 1 - m y0^2 in units of 2^-62
+    const u64 yy = (u64)Y0 * Y0;                      // y0^2 in 2^-64
+    const u64 prod = mul_hi(yy, M << 10);             // m y0^2 in units of 2^-62
+    const i64 e1 = (i64)(0x4000000000000000ull - prod);  // |e1| < 2^42
+    // y = y0 (1 + e1/2 + 3/8 e1^2); S = m y
+    const i64 eh = e1 >> 20;
+    const i64 t = (e1 >> 1) + ((3 * ((eh * eh) >> 22)) >> 3) - 2;  // in 2^-62
+    const u64 tu = t < 0 ? (u64)-t : (u64)t;
+    const u64 corr = ((u64)(unsigned)(tu >> 32) * Y0 << 2) + (((u64)(unsigned)tu * Y0) >> 30);  // y0 t in 2^-64
+    const u64 base = (u64)Y0 << 32;
+    const u64 y = t < 0 ? base - corr - 4ull : base + corr;
+    u64 S = mul_hi(M << 10, y) >> 10;                 // the root's floor or one less
+    u64 r = (M << 52) - S * S;                        // exact: 0 <= r <= 4 S
+    if (r > 2 * S) r -= 2 * S + 1, S++;
+    S += r > S ? 1ull : 0ull;                         // nearest: (S + 1/2)^2 = S^2 + S + 1/4
+    return d_from_bits(((u64)(1022 + k) << 52) + S);
+}
+
 SW2D_HD double d_sqrt(double x) {
-    const unsigned long long m = d_bits(x) & 0x000fffffffffffffull;
-    const bool hard = m != 0ull && ((m + 8ull) & 0x000fffffffffffffull) < 17ull;
-    if (d_mid(x) && (int)d_hi(x) > 0 && !hard) return d_sqrt_fast(x);
+    if (d_mid(x) && (int)d_hi(x) > 0) return d_sqrt_fast(x);
     return d_is_zero(x) ? x : d_sqrt_plain(x);
 }
 
@@ -295,6 +363,151 @@ SW2D_HD double d_pow43_fast(double x, const PowTables *__restrict__ T, bool *ok)
     const double f = p * T->exp2j[j];
     *ok = true;
     return d_make(d_hi(f) + ((unsigned)q << 20), d_lo(f));
+}
+
+// ---- the same power on the integer pipes ------------------------------------------
+//
+// A Horner step p' = c +- p r rounds twice, after the product and after the sum,
+// and costs two FP64 instructions of 64 pipe cycles each.  The coefficients, the
+// signs and the range of r are known, so the step can be done exactly in 64-bit
+// fixed point in about 36 integer instructions: p as an integer PF = p 2^F (F per
+// step, 2^60 <= PF < 2^64), r as a mantissa R in [2^63, 2^64) and an exponent.
+// The 128-bit product is rounded to 53 bits (to nearest, ties to even, with the
+// lower bits jammed into a sticky bit), aligned, added and rounded again at the
+// sum's last place.
+
+SW2D_HD int u_clz(unsigned x) {
+#ifdef __CUDA_ARCH__
+    return __clz((int)x);
+#else
+    return __builtin_clz(x);
+#endif
+}
+
+// High 64 bits of a b, the lower 64 jammed into the last bit.
+SW2D_HD unsigned long long mul_jam(unsigned long long a, unsigned long long b) {
+    typedef unsigned long long u64;
+    const unsigned al = (unsigned)a, ah = (unsigned)(a >> 32), bl = (unsigned)b, bh = (unsigned)(b >> 32);
+    const u64 p0 = (u64)al * bl;
+    const u64 p1 = (u64)ah * bl + (p0 >> 32);
+    const u64 p2 = (u64)al * bh + (unsigned)p1;
+    const u64 p3 = (u64)ah * bh + (p1 >> 32) + (p2 >> 32);
+    return p3 | (((unsigned)p0 | (unsigned)p2) != 0u ? 1ull : 0ull);
+}
+
+// x (>= 2^53, its last bit sticky) rounded to 53 significant bits; *lz: its
+// leading zeros before rounding.
+SW2D_HD unsigned long long round53(unsigned long long x, int *lz) {
+    const int z = u_clz((unsigned)(x >> 32)), d = 11 - z;  // d bits go
+    const unsigned lo = (unsigned)x, inc = (1u << (d - 1)) - 1u + ((lo >> d) & 1u);
+    *lz = z;
+    const unsigned long long t = x + inc;
+    return t & ~(unsigned long long)((1u << d) - 1u);
+}
+
+// x >> n with the bits lost jammed into the last one, 0 < n < 32
+SW2D_HD unsigned long long shift_jam(unsigned long long x, int n) {
+    return (x >> n) | (((unsigned)x << (32 - n)) != 0u ? 1ull : 0ull);
+}
+
+// v rounded to a multiple of 2^sh, ties to even
+SW2D_HD unsigned long long round_at(unsigned long long v, int sh) {
+    const unsigned inc = (1u << (sh - 1)) - 1u + (((unsigned)v >> sh) & 1u);
+    return (v + inc) & ~(unsigned long long)((1u << sh) - 1u);
+}
+
+// c - p r with p, r >= 0: c and p with F = 63, r = R 2^(-sft - 64), result with
+// its last place at bit `sh`.
+SW2D_HD unsigned long long horner_sub(unsigned long long p, unsigned long long R, int sft, unsigned long long c, int sh) {
+    int lz;
+    return round_at(c - shift_jam(round53(mul_jam(p, R), &lz), sft), sh);
+}
+
+// c + p s for a signed s of mantissa S: `neg` all ones for s < 0.
+SW2D_HD unsigned long long horner_add(unsigned long long p, unsigned long long S, int sft, unsigned long long c,
+                                      unsigned long long neg, int sh) {
+    int lz;
+    const unsigned long long x = shift_jam(round53(mul_jam(p, S), &lz), sft);
+    return round_at(c + ((x ^ neg) - neg), sh);
+}
+
+// c 2^F of a double c, exactly (constants)
+SW2D_HD constexpr unsigned long long fixed_of(double c, int F) {
+    for (int k = 0; k < F; k++) c *= 2.0;
+    return (unsigned long long)c;
+}
+
+// d_pow43_fast with both polynomials and the exact products in integers: 8 FP64
+// instructions instead of 36.  *ok is false for the operands whose reduced
+// argument is 0 or below 2^-28 as well (d_pow43_fast takes those).
+SW2D_HD double d_pow43_int(double x, const PowTables *__restrict__ T, bool *ok) {
+    typedef unsigned long long u64;
+    constexpr u64 c7 = fixed_of(1.0 / 7.0, 63), c6 = fixed_of(1.0 / 6.0, 63), c5 = fixed_of(1.0 / 5.0, 63),
+                  c4 = fixed_of(1.0 / 4.0, 63), c3 = fixed_of(1.0 / 3.0, 63), c2 = fixed_of(0.5, 63),
+                  c1 = fixed_of(1.0, 63);
+    constexpr u64 e720 = fixed_of(1.0 / 720.0, 72), e120 = fixed_of(1.0 / 120.0, 69), e24 = fixed_of(1.0 / 24.0, 67),
+                  e6 = fixed_of(1.0 / 6.0, 65);
+    const u64 b = d_bits(x);
+    const int e = (int)(b >> 52) - 1023;  // x > 0
+    const int k = (int)((b >> 45) & 127);
+    const u64 frac = b & 0x1fffffffffffull;  // m - c = frac 2^-52
+    *ok = false;
+    if ((unsigned)(e + kPowE) >= 2u * kPowE || (frac >> 27) == 0ull) return 0.0;
+    // r = frac 2^-52 / c rounded: R 2^(er - 63)
+    const double inv = T->inv[k];  // in (1/2, 1]: exponent -1 (or 0 for k = 0)
+    const int zf = u_clz((unsigned)(frac >> 13));  // frac < 2^45
+    const u64 M = ((d_bits(inv) & 0xfffffffffffffull) | 0x10000000000000ull) << 11;
+    int lz;
+    u64 R = round53(mul_jam(frac << (19 + zf), M), &lz);
+    // frac << (19 + zf) = (m - c) 2^(71 + zf), M = inv 2^(63 or 64)
+    int er = 63 - (71 + zf + (k ? 64 : 63) - 64);
+    if (lz) R <<= 1, er -= 1;  // (rounding up to 2^64 cannot happen: 1/c and m - c do not both end in ones)
+    if (R >> 63 == 0ull) return 0.0;
+    const int sft = -er - 1;
+    if (sft > 27) return 0.0;
+    u64 p = round_at(c7 - shift_jam(R, sft + 4), 8);
+    p = horner_sub(p, R, sft, c6, 8);
+    p = horner_sub(p, R, sft, c5, 8);
+    p = horner_sub(p, R, sft, c4, 8);
+    p = horner_sub(p, R, sft, c3, 9);
+    p = horner_sub(p, R, sft, c2, 9);
+    p = horner_sub(p, R, sft, c1, 10);
+    const u64 l = round53(mul_jam(p, R), &lz);  // lr = l 2^(er - 62)
+    const int zl = u_clz((unsigned)(l >> 32));
+    const double lr = d_from_bits(((u64)(1023 + er + 1 - zl) << 52) + (((l << zl) >> 11) & 0xfffffffffffffull));
+    const double y = 1.3333330 * (T->ehi[e + kPowE] + (T->elo[e + kPowE] + (T->logc[k] + lr)));
+    const double v = y * (64.0 * 0x1.71547652b82fep+0) + 0.5;
+    const unsigned vh = d_hi(v), vl = d_lo(v);
+    const int ev = (int)((vh >> 20) & 0x7ffu) - 1023;
+    if (ev > 10) return 0.0;  // |v| >= 2048
+    int n;
+    if (ev < 0) {
+        n = ((int)vh < 0 && !d_is_zero(v)) ? -1 : 0;
+    } else {
+        const unsigned m = (vh & 0x000fffffu) | 0x00100000u;
+        const int mag = (int)(m >> (20 - ev));
+        const bool fr = ((m & ((1u << (20 - ev)) - 1u)) | vl) != 0u;
+        n = (int)vh < 0 ? -(mag + (fr ? 1 : 0)) : mag;
+    }
+    const double s = (y - T->nhi[n + kPowN]) - T->nlo[n + kPowN];
+    const u64 sb = d_bits(s);
+    const int es = (int)((sb >> 52) & 0x7ffu) - 1023;
+    if (es < -29 || es > -8) return 0.0;
+    const u64 S = ((sb & 0xfffffffffffffull) | 0x10000000000000ull) << 11, neg = (u64)((long long)sb >> 63);
+    const int q0 = -es - 1, lower = (int)(sb >> 63);  // below 1/2 and 1 the last place is one bit finer
+    p = horner_add(e720, S, q0 + 3, e120, neg, 10);
+    p = horner_add(p, S, q0 + 2, e24, neg, 10);
+    p = horner_add(p, S, q0 + 2, e6, neg, 10);
+    p = horner_add(p, S, q0 + 2, c2, neg, 10 - lower);
+    p = horner_add(p, S, q0, c1, neg, 11 - lower);
+    p = horner_add(p, S, q0, c1, neg, 11 - lower);
+    // times 2^(j/64), in [1, 2), and 2^q
+    const int j = n & 63, q = (n - j) / 64;
+    const u64 E = ((d_bits(T->exp2j[j]) & 0xfffffffffffffull) | 0x10000000000000ull) << 11;
+    const u64 f = round53(mul_jam(p, E), &lz);  // the product times 2^62
+    const int z = u_clz((unsigned)(f >> 32));
+    *ok = true;
+    return d_from_bits(((u64)(1023 + q + 1 - z) << 52) + (((f << z) >> 11) & 0xfffffffffffffull));
 }
 
 }  // namespace sw2d

@@ -63,12 +63,17 @@ static __global__ void pow_tables_kernel() {
     }
 }
 
-static __device__ __noinline__ double pow43_plain(double x) { return det_exp(1.3333330 * det_log(x)); }
+// The friction power for what the integer form does not cover (d_pow43_int).
+static __device__ __noinline__ double pow43_rest(double x) {
+    bool ok;
+    const double r = d_pow43_fast(x, &g_pow_tab, &ok);
+    return ok ? r : det_exp(1.3333330 * det_log(x));
+}
 
 __device__ __forceinline__ double pow43(double x) {
     bool ok;
-    const double r = d_pow43_fast(x, &g_pow_tab, &ok);
-    return ok ? r : pow43_plain(x);
+    const double r = d_pow43_int(x, &g_pow_tab, &ok);
+    return ok ? r : pow43_rest(x);
 }
 
 // g n^2 of every face from the Manning raster, with the face's n the mean of its
@@ -92,7 +97,7 @@ static __global__ void pack_gn_kernel(const double *__restrict__ n, int rows, in
 struct Step64Extra {
     const double *gnx, *gny;
     double gn;          // g n^2 of the scalar n
-    double rdx, rdy;    // 1/dx, 1/dy rounded
+    KnownDivisor dx, dy;
 };
 
 constexpr int kStep64Arrays = 13;
@@ -460,7 +465,7 @@ __global__ void __launch_bounds__(NT, MINB)
     const bool any_ev0 = !d_is_zero(LS.ev0), any_ev1 = !d_is_zero(LS.ev1);
     auto balance = [&](double ho, double un, double us, double vw, double ve, double ql, double rp, double evapo,
                        bool any_ev) -> double {
-        double s = d_div_const(us - un, dx, X.rdx) + d_div_const(ve - vw, dy, X.rdy);
+        double s = d_div_known(us - un, X.dx) + d_div_known(ve - vw, X.dy);
         if (nloc) s = s - ql;
         s = s - rp;
         if (any_ev) s = s + evapo;

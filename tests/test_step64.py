@@ -39,7 +39,7 @@ static double rnd(int lo, int hi) {
     return d_from_bits(((unsigned long long)(lo + (int)(R() % (unsigned)(hi - lo + 1)) + 1023) << 52) | m);
 }
 static bool eq(double a, double b) { return a == b || (a != a && b != b); }
-static long bad = 0;
+static long bad = 0, taken = 0;
 static void expect(bool ok, const char *what, double a, double b) {
     if (!ok && bad++ < 10) printf("%s %a %a\n", what, a, b);
 }
@@ -84,20 +84,23 @@ int main(int, char **argv) {
     for (long i = 0; i < n; i++) {
         const double a = rnd(-40, 40) * ((R() & 1) ? 1 : -1), b = rnd(-20, 20), d = rnd(-8, 8);
         pair(a, b);
-        expect(d_div_const(a, d, 1.0 / d) == a / d, "div_const", a, d);
+        expect(d_div_known(a, known_divisor(d)) == a / d, "div_known", a, d);
         one(a);
         one(std::fabs(a));
         const double m = rnd(0, 0), near = d_fma(b, m, b * 0x1p-53 * m * 0.5);  // a quotient by a midpoint
         for (int t = -1; t <= 1; t++) {
             const double x = d_from_bits(d_bits(near) + (unsigned long long)(long long)t);
             pair(x, b);
-            expect(d_div_const(x, b, 1.0 / b) == x / b, "div_const", x, b);
+            expect(d_div_known(x, known_divisor(b)) == x / b, "div_known", x, b);
         }
         const double s = rnd(-20, 20);
         one(d_from_bits(d_bits(s * s) + R() % 5 - 2));
         bool ok;
         const double h = rnd(-14, 8), pw = d_pow43_fast(h, T, &ok);
         expect(ok && pw == orc_pow43(h), "pow", h, pw);
+        const double pi = d_pow43_int(h, T, &ok);
+        taken += ok;
+        expect(!ok || pi == orc_pow43(h), "pow_int", h, pi);
         expect(std::fabs((double)d_abs_float(a) - std::fabs(a)) <= std::fabs(a) * 0x1p-23, "float", a, 0);
     }
     const double sp[] = {0.0, -0.0, HUGE_VAL, -HUGE_VAL, std::nan(""), 5e-324, -5e-324, 1e-310, 1e-300, 1e300, -1e300,
@@ -106,17 +109,21 @@ int main(int, char **argv) {
         one(a);
         for (double b : sp) pair(a, b);
     }
+    expect(taken > n / 2, "pow_int covers too few", (double)taken, 0);
     printf("bad %ld\n", bad);
     return bad != 0;
 }
 """
 
 
-def test_f64_helpers_give_the_plain_bits(oracle_mod, tmp_path):
+@pytest.mark.parametrize("seed_ulps", [-2, 0, 2])
+def test_f64_helpers_give_the_plain_bits(oracle_mod, tmp_path, seed_ulps):
+    """With exact FP32 seeds and with seeds off by more than the device's
+    approximations are (one ulp)."""
     src, exe = tmp_path / "check.cpp", tmp_path / "check"
     src.write_text(CHECK)
     so = os.path.join(ROOT, "oracle", "_build", "liboracle.so")
-    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-I",
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", f"-DSW2D_SEED_ULPS={seed_ulps}", "-I",
                     os.path.join(ROOT, "sw2d-gpu_gb300", "csrc"), str(src), so, "-Wl,-rpath," + os.path.dirname(so),
                     "-o", str(exe)], check=True)
     r = subprocess.run([str(exe), "200000"], capture_output=True, text=True)
