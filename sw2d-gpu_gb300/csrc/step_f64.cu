@@ -18,20 +18,23 @@ cudaError_t init_det_tables() {
 }
 
 // Builds of the step kernel: (tile rows, tile columns, threads, minimum
-// resident CTAs per SM).  16 x 32 with 384 threads and two CTAs per SM: 526 us
-// per iteration on a 1013 x 900 catchment, against 557 with 256 threads (the
-// integer stages run at too few warps), 525 with 512, and 550 with a 32 x 32
-// tile (less halo, but one CTA per SM idles at its barriers).
+// resident CTAs per SM).  16 x 32 runs two CTAs of 512 threads per SM, whose
+// stages overlap: 313 us per iteration on a 1013 x 900 catchment, 447 with one
+// CTA of 768 (the stages then wait at each other's barriers), 358 with one CTA on
+// a 32 x 32 tile (less halo, same wait); 256 to 448 threads are within 3 %.
 //
 // The smaller tiles are for grids that would leave SMs without a CTA: a tile's
-// work runs on one SM's FP64 pipe, so a grid is cut into the smallest tiles that
-// still give one CTA per SM (step64_tile).  Measured, us per iteration, tiles
-// 4x8 / 4x16 / 8x16 / 8x32 / 16x32: 64 x 64 23.8 / 27.0 / 30.3 / 42.3 / 53.5;
-// 117 x 131 48.8 / 42.8 / 34.5 / 47.5 / 60.2; 256 x 256 159 / 106 / 79 / 72 /
-// 69.5; 512 x 512 593 / 327 / 261 / 225 / 185 (the halo costs 2.3 times the
-// faces of the tile at 4 x 8, 1.4 at 16 x 32).
+// work runs on one SM, so a grid is cut into the smallest tiles that still give
+// one CTA per SM (step64_tile).  Measured with the first form of the kernel, us
+// per iteration, tiles 4x8 / 4x16 / 8x16 / 8x32 / 16x32: 64 x 64 23.8 / 27.0 /
+// 30.3 / 42.3 / 53.5; 117 x 131 48.8 / 42.8 / 34.5 / 47.5 / 60.2; 256 x 256 159 /
+// 106 / 79 / 72 / 69.5; 512 x 512 593 / 327 / 261 / 225 / 185 (the halo costs 2.3
+// times the faces of the tile at 4 x 8, 1.4 at 16 x 32); the final form runs 18.9,
+// 23.2, 43 and 106 on the tile the rule takes.  With one CTA per SM more threads
+// shorten the stages: 8 x 16 23.2 with 512 against 26.9 with 256, 8 x 32 30.6 with
+// 768 against 34.2 with 384.
 #define SW2D_STEP64_TILES(X) \
-    X(16, 32, 384, 2) X(8, 32, 256, 3) X(8, 16, 256, 2) X(4, 16, 192, 2) X(4, 8, 192, 2)
+    X(16, 32, 512, 2) X(8, 32, 768, 1) X(8, 16, 512, 1) X(4, 16, 256, 1) X(4, 8, 256, 1)
 
 bool step64_tile_supported(int th, int tw) {
 #define SW2D_S64(h, w, nt, mb) \
@@ -80,6 +83,7 @@ cudaError_t launch_step64(int th, int tw, int nblocks, int sms, const GridDesc &
     X.gnx = gnx;
     X.gny = gny;
     X.gn = G.sd.g * G.sd.manning * G.sd.manning;
+    X.thf = (float)T.ge_th;
     X.dx = known_divisor(G.sd.dx);
     X.dy = known_divisor(G.sd.dy);
     // a programmatic dependent of the launch before it (step64_kernel, stage 0)

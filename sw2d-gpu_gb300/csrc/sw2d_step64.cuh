@@ -98,6 +98,7 @@ struct Step64Extra {
     const double *gnx, *gny;
     double gn;          // g n^2 of the scalar n
     KnownDivisor dx, dy;
+    float thf;          // T.ge_th in FP32
 };
 
 constexpr int kStep64Arrays = 13;
@@ -168,6 +169,7 @@ __global__ void __launch_bounds__(NT, MINB)
 
     __shared__ double s_red[NW][B_N];
     __shared__ int s_cnt[NW][2];
+    __shared__ double s_k[9];  // dt2/dx and dt2/dy by 4, by 2, dt2 by 2, rr0 and rr1 times pct_hi, pct_lo
     __shared__ int s_n[3];  // lengths of the lists: momentum faces, weir faces, fluxes
     __shared__ unsigned s_est;
     __shared__ unsigned long long s_cm;
@@ -228,6 +230,12 @@ __global__ void __launch_bounds__(NT, MINB)
         s_h[idx] = in_r && in_c ? Hin[gp] : 0.0;
         s_umo[idx] = ((unsigned)gi <= (unsigned)rows && in_c) ? Uin[gp] : 0.0;
         s_vno[idx] = (in_r && (unsigned)gj <= (unsigned)cols) ? Vin[gp] : 0.0;
+    }
+    // per-launch products, one lane each
+    if (wid == NW - 1 && lane < 9) {
+        const double a = lane < 4 ? (lane & 1 ? LS.dt2dy : LS.dt2dx) : (lane == 4 ? dt2 : (lane < 7 ? LS.rr0 : LS.rr1));
+        const double b = lane < 2 ? 0.25 : (lane < 5 ? 0.5 : (lane & 1 ? G.sd.pct_hi : G.sd.pct_lo));
+        s_k[lane] = a * b;
     }
     if (tid == 0) {
         s_nloc = 0;
@@ -393,8 +401,8 @@ __global__ void __launch_bounds__(NT, MINB)
     __syncthreads();
 
     // ---- stage 2: new face discharges (cu:98-354) ---------------------------
-    const double qdx = 0.25 * LS.dt2dx, qdy = 0.25 * LS.dt2dy;  // with the fluxes' quarters
-    const double hdx = 0.5 * LS.dt2dx, hdy = 0.5 * LS.dt2dy, hdt2 = 0.5 * dt2;
+    const double qdx = s_k[0], qdy = s_k[1];  // with the fluxes' quarters
+    const double hdx = s_k[2], hdy = s_k[3], hdt2 = s_k[4];
     const int n_mom = s_n[0], n_weir = s_n[1];
     const int mom_chunks = (n_mom + 31) / 32, chunks = mom_chunks + (n_weir + 31) / 32;
     for (int ch = wid; ch < chunks; ch += NW) {
@@ -474,7 +482,7 @@ __global__ void __launch_bounds__(NT, MINB)
     const bool uniform = !storm && !W;
 
     // ---- stage 3: provisional depth with forcing at t (cu:1278-1288) -------
-    const double rp0_hi = LS.rr0 * pct_hi, rp0_lo = LS.rr0 * pct_lo;
+    const double rp0_hi = s_k[5], rp0_lo = s_k[6];
     constexpr int PH = TH + 3, PW = TW + 3;  // rows/cols [2, TH+5) x [2, TW+5)
     for (int k = tid; k < PH * PW; k += NT) {
         const int r = 2 + k / PW, c = 2 + (k - (k / PW) * PW);
@@ -513,7 +521,7 @@ __global__ void __launch_bounds__(NT, MINB)
     // With the same forcing at t and t + dt and none of its faces corrected, a
     // cell's final depth is the provisional one: the same operands.
     const bool steady = uniform && nloc == 0 && d_bits(LS.rr0) == d_bits(LS.rr1) && d_bits(LS.ev0) == d_bits(LS.ev1);
-    const double rp1_hi = LS.rr1 * pct_hi, rp1_lo = LS.rr1 * pct_lo;
+    const double rp1_hi = s_k[7], rp1_lo = s_k[8];
     float *s_hf = reinterpret_cast<float *>(s_fx);  // the fluxes are done with: FP32 depths for stage 5
     int n_hi = 0, n_lo = 0;  // active owned cells above / not above EV_WL_min
     double b_rain = 0.0, b_src = 0.0, b_out = 0.0, b_clamp = 0.0;
@@ -579,7 +587,7 @@ __global__ void __launch_bounds__(NT, MINB)
     // faces).  The CTA's largest estimate among the faces certainly deeper than
     // th, less that margin, is a bar below the exact maximum: only faces whose
     // estimate reaches it are evaluated in FP64.
-    const float gf = (float)g, thf = (float)T.ge_th;
+    const float gf = G.sf.g, thf = X.thf;
     auto faces = [&](auto &&visit) {
         for (int k = tid; k < TH * TW; k += NT) {
             const int r = HN + k / TW, c = HN + (k - (k / TW) * TW);
