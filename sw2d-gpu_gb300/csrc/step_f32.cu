@@ -53,13 +53,25 @@ cudaError_t prepare_stream_step(int variant) {
         if (e != cudaSuccess) return e;
         variant = 0;  // the build the other forcing forms run
     }
+    // the default build's forms for short strips
+    if (variant == 0) {
+        const void *k[4] = {(const void *)stream_step_kernel<2, 10, 2, false, kFormUniform, true>,
+                            (const void *)stream_step_kernel<2, 10, 2, false, kFormStorm, true>,
+                            (const void *)stream_step_kernel<2, 10, 2, false, kFormAny, true>,
+                            (const void *)stream_step_kernel<2, 10, 2, true, kFormUniform, true>};
+        for (int i = 0; i < 4; i++) {
+            cudaError_t e = cudaFuncSetAttribute(k[i], cudaFuncAttributePreferredSharedMemoryCarveout,
+                                                 kStreamCarveoutPercent);
+            if (e != cudaSuccess) return e;
+        }
+    }
 #define SW2D_P(id, nw, mb, un)                                                                            \
     if (variant == id) {                                                                               \
-        const void *k[5] = {(const void *)stream_step_kernel<nw, mb, un, false, kFormUniform>,         \
-                            (const void *)stream_step_kernel<nw, mb, un, false, kFormStorm>,           \
-                            (const void *)stream_step_kernel<nw, mb, un, false, kFormAny>,             \
-                            (const void *)stream_step_kernel<nw, mb, un, true, kFormUniform>,          \
-                            (const void *)stream_step_kernel<nw, mb, un, true, kFormAny>};             \
+        const void *k[5] = {(const void *)stream_step_kernel<nw, mb, un, false, kFormUniform, false>,         \
+                            (const void *)stream_step_kernel<nw, mb, un, false, kFormStorm, false>,           \
+                            (const void *)stream_step_kernel<nw, mb, un, false, kFormAny, false>,             \
+                            (const void *)stream_step_kernel<nw, mb, un, true, kFormUniform, false>,          \
+                            (const void *)stream_step_kernel<nw, mb, un, true, kFormAny, false>};             \
         for (int i = 0; i < 5; i++) {                                                                  \
             cudaError_t e = cudaFuncSetAttribute(k[i], cudaFuncAttributePreferredSharedMemoryCarveout, \
                                                  kStreamCarveoutPercent);                             \
@@ -90,7 +102,7 @@ int stream_ctas_per_sm(int variant) {
                    : 0;
 #define SW2D_O(id, nw, mb, un)                                                                           \
     if (variant == id &&                                                                                 \
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, stream_step_kernel<nw, mb, un, false, kFormUniform>, nw * 32, 0) != \
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, stream_step_kernel<nw, mb, un, false, kFormUniform, false>, nw * 32, 0) != \
             cudaSuccess)                                                                                 \
         n = 0;
     SW2D_STREAM_VARIANTS(SW2D_O)
@@ -173,16 +185,30 @@ cudaError_t launch_stream_step(int variant, int nblocks, int tiles_w, int strip_
         }
         variant = 0;
     }
-#define SW2D_LK(nw, mb, un, rw, fm) \
-    return cudaLaunchKernelEx(&lc, stream_step_kernel<nw, mb, un, rw, fm>, G, F, S, T, clk, ctl, slot, sh)
-#define SW2D_L(id, nw, mb, un)                                               \
-    if (variant == id) {                                                     \
-        lc.blockDim = dim3(nw * 32);                                         \
-        if (S.rainw && form == kFormAny) SW2D_LK(nw, mb, un, true, kFormAny); \
-        if (S.rainw) SW2D_LK(nw, mb, un, true, kFormUniform);                \
-        if (form == kFormStorm) SW2D_LK(nw, mb, un, false, kFormStorm);      \
-        if (form == kFormAny) SW2D_LK(nw, mb, un, false, kFormAny);          \
-        SW2D_LK(nw, mb, un, false, kFormUniform);                            \
+#define SW2D_LK(nw, mb, un, rw, fm, sk) \
+    return cudaLaunchKernelEx(&lc, stream_step_kernel<nw, mb, un, rw, fm, sk>, G, F, S, T, clk, ctl, slot, sh)
+    // Short strips leave out the warm-up rows' unread stages (SKIP), in the default
+    // build.  us per iteration without / with, rows per strip in brackets: uniform
+    // 13.5 / 12.6 (1), 15.1 / 14.2 (2), 16.7 / 16.2 (4), 17.3 / 17.2 (6), but 18.9 /
+    // 19.0 (8), 21.9 / 22.1 (10), 73.3 / 76.8 (52); storm 13.5 / 12.6 (1), 31.4 / 31.0
+    // (13), 78.2 / 81.4 (52); sources 17.3 / 15.5 (1), 40.2 / 39.4 (13), 93.6 / 95.1
+    // (52); rain factors 14.1 / 13.4 (1), 33.2 / 33.0 (13), 39.2 / 39.6 (16), 98 / 103
+    // (52).
+    if (variant == 0 && strip_h <= (form == kFormUniform && !S.rainw ? 6 : 13)) {
+        lc.blockDim = dim3(64);
+        if (S.rainw && form == kFormUniform) SW2D_LK(2, 10, 2, true, kFormUniform, true);
+        if (!S.rainw && form == kFormStorm) SW2D_LK(2, 10, 2, false, kFormStorm, true);
+        if (!S.rainw && form == kFormAny) SW2D_LK(2, 10, 2, false, kFormAny, true);
+        if (!S.rainw) SW2D_LK(2, 10, 2, false, kFormUniform, true);
+    }
+#define SW2D_L(id, nw, mb, un)                                                      \
+    if (variant == id) {                                                            \
+        lc.blockDim = dim3(nw * 32);                                                \
+        if (S.rainw && form == kFormAny) SW2D_LK(nw, mb, un, true, kFormAny, false); \
+        if (S.rainw) SW2D_LK(nw, mb, un, true, kFormUniform, false);                \
+        if (form == kFormStorm) SW2D_LK(nw, mb, un, false, kFormStorm, false);      \
+        if (form == kFormAny) SW2D_LK(nw, mb, un, false, kFormAny, false);          \
+        SW2D_LK(nw, mb, un, false, kFormUniform, false);                            \
     }
     SW2D_STREAM_VARIANTS(SW2D_L)
 #undef SW2D_L

@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(NWARP * 32, MINB)
             V.dy = G.dy;
             StreamAcc A;
             acc_clear(A);
-            stream_unit<UNR, RAINW, FORM, false, true>(V, ct, r0, r1, lane, s_sr[wid], s_sc[wid], s_q0[wid],
+            stream_unit<UNR, RAINW, FORM, false, true, true>(V, ct, r0, r1, lane, s_sr[wid], s_sc[wid], s_q0[wid],
                                                       s_q1[wid], A, nullptr, 0, nullptr, nullptr,
                                                       P.flags + SH.units + unit, (unsigned)(j + 1));
             warp_reduce_acc<!RAINW && FORM == kFormUniform>(A);

@@ -82,7 +82,7 @@ __device__ __forceinline__ int unit_of_warp(const StreamShape &SH, int w) {
 // and point sources (the launcher picks the build from the handle's
 // forcing); TMA: rows staged in shared memory by TMA (M: the planes' tensor
 // maps, smem: kTmaStages stages per warp).
-template <int NWARP, int MINB, int UNR, bool RAINW, int FORM, bool TMA>
+template <int NWARP, int MINB, int UNR, bool RAINW, int FORM, bool TMA, bool SKIP>
 __device__ __forceinline__ void stream_step_body(const GridDesc &G, const ForcingDesc &F, const StateBufs<float> &S,
                                                  const Thr<float> &T, Clock *__restrict__ clk,
                                                  const Control *__restrict__ ctl, const int slot,
@@ -155,7 +155,7 @@ __device__ __forceinline__ void stream_step_body(const GridDesc &G, const Forcin
         strip_rows(G.rows, SH.strips, SH.skew, unit / SH.tiles_w, r0, r1);
         r0 = __shfl_sync(0xffffffffu, r0, 0);  // the strip's rows, warp-uniform (see above)
         r1 = __shfl_sync(0xffffffffu, r1, 0);
-        stream_unit<UNR, RAINW, FORM, TMA>(V, unit % SH.tiles_w, r0, r1, lane, s_sr[wid],
+        stream_unit<UNR, RAINW, FORM, TMA, false, SKIP>(V, unit % SH.tiles_w, r0, r1, lane, s_sr[wid],
                                            s_sc[wid], s_q0[wid], s_q1[wid], A, M, b,
                                            TMA ? smem + wid * kTmaStages * kTmaStageBytes : nullptr,
                                            TMA ? s_bar[wid] : nullptr);
@@ -219,12 +219,12 @@ __device__ __forceinline__ void stream_step_body(const GridDesc &G, const Forcin
     }
 }
 
-template <int NWARP, int MINB, int UNR, bool RAINW, int FORM>
+template <int NWARP, int MINB, int UNR, bool RAINW, int FORM, bool SKIP>
 __global__ void __launch_bounds__(NWARP * 32, MINB)
     stream_step_kernel(const GridDesc G, const ForcingDesc F, const StateBufs<float> S, const Thr<float> T,
                        Clock *__restrict__ clk, const Control *__restrict__ ctl, const int slot,
                        const StreamShape SH) {
-    stream_step_body<NWARP, MINB, UNR, RAINW, FORM, false>(G, F, S, T, clk, ctl, slot, SH, nullptr, nullptr);
+    stream_step_body<NWARP, MINB, UNR, RAINW, FORM, false, SKIP>(G, F, S, T, clk, ctl, slot, SH, nullptr, nullptr);
 }
 
 // The build that stages rows in shared memory by TMA (uniform forcing only):
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(NWARP * 32, MINB)
                            Clock *__restrict__ clk, const Control *__restrict__ ctl, const int slot,
                            const StreamShape SH, const __grid_constant__ TmaMaps M) {
     extern __shared__ __align__(1024) unsigned char s_stage[];
-    stream_step_body<NWARP, MINB, UNR, false, kFormUniform, true>(G, F, S, T, clk, ctl, slot, SH, &M, s_stage);
+    stream_step_body<NWARP, MINB, UNR, false, kFormUniform, true, false>(G, F, S, T, clk, ctl, slot, SH, &M, s_stage);
 }
 
 }  // namespace sw2d

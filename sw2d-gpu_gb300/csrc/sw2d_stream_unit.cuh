@@ -220,7 +220,13 @@ __device__ __forceinline__ double acc_ev(double sum, int n_hi, const LaunchScala
 // above reads of this iteration) and the rows above the strip have been
 // read (all of the strip above that this iteration reads), lane 0 publishes
 // top_val at *top_flag with a release store.
-template <int UNR, bool RAINW, int FORM, bool TMA = false, bool PIPE = false>
+//
+// SKIP leaves out, in the 7 warm-up rows, the stages whose results no output row
+// reads: fluxes before row R0-2, discharges before R0-1, provisional depths before
+// R0, final depths before R0+2 (warp-uniform branches, same bits).  It pays where
+// warm-up rows are a large part of a short strip (see the launchers) and costs the
+// long ones 4 % in scheduling freedom.
+template <int UNR, bool RAINW, int FORM, bool TMA = false, bool PIPE = false, bool SKIP = false>
 __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, const int r0, const int r1,
                                             const int lane, int *s_sr, int *s_sc, float *s_q0, float *s_q1,
                                             StreamAcc &A, const TmaMaps *M = nullptr, int buf = 0,
@@ -478,24 +484,27 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
 
         // ---- row r-1: new face discharges (cu:98-354) ----
         const int i = r - 1;
-        const float umW = shup(um1);
-        const float vnE = vnE1;
-        // upwinded fluxes shared between neighbouring faces: the flux through
-        // the cell south of x-face i is the one north of face i+1 (kept for the
-        // next row); the corner flux east of a lane is the one west of its east
-        // neighbour (a shuffle); likewise along the rows for the y-faces
-        const float vx = uu_0 + uu_1;
-        const float fx_0 = vx * (vx >= 0.f ? um1 : um0);  // upw(uu_0 + uu_1, um0, um1)
-        const float vw2 = vv_1 + vv_2;
-        const float fw = vw2 * (vw2 >= 0.f ? umW : um1);  // upw_r(vv_1 + vv_2, umW, um1)
-        const float fe = shdn(fw);                        // the east lane's fw (lane 31: a halo lane)
-        const float vc = uu_0 + uuL_0;
-        const float cy_0 = vc * (vc >= 0.f ? vn1 : vn0);  // upw(uu_0 + uuL_0, vn0, vn1)
-        const float ve2 = vvR_1 + vv_1;
-        const float ge = ve2 * (ve2 >= 0.f ? vn1 : vnE);  // upw(vvR_1 + vv_1, vnE, vn1)
-        const float gw = shup(ge);                        // the west lane's ge (lane 0: a halo lane)
+        float fx_0 = 0.f, cy_0 = 0.f, fw = 0.f, fe = 0.f, ge = 0.f, gw = 0.f;
+        if (!SKIP || r >= R0 - 2) {
+            const float umW = shup(um1);
+            const float vnE = vnE1;
+            // upwinded fluxes shared between neighbouring faces: the flux through
+            // the cell south of x-face i is the one north of face i+1 (kept for the
+            // next row); the corner flux east of a lane is the one west of its east
+            // neighbour (a shuffle); likewise along the rows for the y-faces
+            const float vx = uu_0 + uu_1;
+            fx_0 = vx * (vx >= 0.f ? um1 : um0);  // upw(uu_0 + uu_1, um0, um1)
+            const float vw2 = vv_1 + vv_2;
+            fw = vw2 * (vw2 >= 0.f ? umW : um1);  // upw_r(vv_1 + vv_2, umW, um1)
+            fe = shdn(fw);                        // the east lane's fw (lane 31: a halo lane)
+            const float vc = uu_0 + uuL_0;
+            cy_0 = vc * (vc >= 0.f ? vn1 : vn0);  // upw(uu_0 + uuL_0, vn0, vn1)
+            const float ve2 = vvR_1 + vv_1;
+            ge = ve2 * (ve2 >= 0.f ? vn1 : vnE);  // upw(vvR_1 + vv_1, vnE, vn1)
+            gw = shup(ge);                        // the west lane's ge (lane 0: a halo lane)
+        }
         float rum_1 = 0.f;
-        {
+        if (!SKIP || r >= R0 - 1) {
             const float ha = h2, hb = h1, dz = dzx1;
             if (((mb >> 2) & (mb >> 1) & 1u) && ((ha >= gt_th) || (hb >= gt_th))) {
                 if (!dry_bed_dz(T, g, ha, hb, dz, rum_1)) {
@@ -514,7 +523,7 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
             }
         }
         float rvn_1 = 0.f;
-        {
+        if (!SKIP || r >= R0 - 1) {
             const float ha = hL1, hb = h1, dz = dzy1;
             if (((mLb >> 1) & (mb >> 1) & 1u) && ((ha >= gt_th) || (hb >= gt_th))) {
                 if (!dry_bed_dz(T, g, ha, hb, dz, rvn_1)) {
@@ -532,109 +541,114 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
         }
 
         // ---- row r-2: provisional depth, forcing at t (cu:1278-1288) ----
-        const float rvnE_2 = shdn(rvn_2);
         float hs_2 = 0.f;
-        if ((mb >> 2) & 1u) {
-            const float ho = h2;
-            const bool hi = ho >= gt_ev;
-            const float pct = hi ? pct_hi : pct_lo;
-            const float evapo = hi ? u_ev0 : 0.f;
-            const float ql = nsrc ? source_at(r - 2, false) : 0.f;
-            float rr = storm ? storm_rate(r - 2, on0, sx0, sy0) : u_rr0;
-            if (RAINW) rr = rr * Win[(r - 2) * pitch + gj];
-            if constexpr (FORM == kFormUniform && !RAINW) {  // the cell's forcing is one select of per-warp values
-                hs_2 = fmaxf(ho + ((rum_1 - rum_2) * ndx + (rvnE_2 - rvn_2) * ndy) + (hi ? f0_hi : f0_lo), 0.f);
-            } else {
-                hs_2 = fmaxf(ho - dt2 * ((rum_1 - rum_2) * rdx + (rvnE_2 - rvn_2) * rdy - ql - rr * pct + evapo),
-                             0.f);
+        if (!SKIP || r >= R0) {
+            const float rvnE_2 = shdn(rvn_2);
+            if ((mb >> 2) & 1u) {
+                const float ho = h2;
+                const bool hi = ho >= gt_ev;
+                const float pct = hi ? pct_hi : pct_lo;
+                const float evapo = hi ? u_ev0 : 0.f;
+                const float ql = nsrc ? source_at(r - 2, false) : 0.f;
+                float rr = storm ? storm_rate(r - 2, on0, sx0, sy0) : u_rr0;
+                if (RAINW) rr = rr * Win[(r - 2) * pitch + gj];
+                if constexpr (FORM == kFormUniform && !RAINW) {  // the cell's forcing is one select of per-warp values
+                    hs_2 = fmaxf(ho + ((rum_1 - rum_2) * ndx + (rvnE_2 - rvn_2) * ndy) + (hi ? f0_hi : f0_lo), 0.f);
+                } else {
+                    hs_2 = fmaxf(ho - dt2 * ((rum_1 - rum_2) * rdx + (rvnE_2 - rvn_2) * rdy - ql - rr * pct + evapo),
+                                 0.f);
+                }
             }
-        }
 
+        }
         // ---- row r-3: dry-cell fix (cu:695-725) and final depth ----
         // dry-cell fix (cu:695-725): a cell is "dry" when active and h* < th; its
         // flag is kept in a bit ring, so each cell's test is made once
         db = (db << 1) | ((((mb >> 2) & 1u) && hs_2 < ge_th) ? 1u : 0u);
-        const unsigned dbW = __shfl_up_sync(0xffffffffu, db, 1);
-        const bool m3 = (mb >> 3) & 1u, m4 = (mb >> 4) & 1u, mL3 = (mLb >> 3) & 1u;
-        const bool d2 = db & 1u, d3 = (db >> 1) & 1u, d4 = (db >> 2) & 1u, dW3 = (dbW >> 1) & 1u;
-        float un = rum_3;  // x-face north of the row-(r-3) cell
-        if ((un > 0.f && d4) || (un < 0.f && d3)) un = 0.f;
-        float us = rum_2;  // x-face south of it
-        if ((us > 0.f && d3) || (us < 0.f && d2)) us = 0.f;
-        float vw = rvn_3;  // y-face west of it
-        if ((vw > 0.f && dW3) || (vw < 0.f && d3)) vw = 0.f;
-        const float ve = shdn(vw);
-        const int f = r - 3;
-        float hw_3 = 0.f, hres = 0.f, clampv = 0.f, rr1 = 0.f, pct1 = 0.f, ev1 = 0.f, ql1 = 0.f;
-        if (m3) {
-            const float ho = h3;
-            const bool hi = ho >= gt_ev;
-            pct1 = hi ? pct_hi : pct_lo;
-            ev1 = hi ? u_ev1 : 0.f;
-            ql1 = nsrc ? source_at(f, true) : 0.f;
-            rr1 = storm ? storm_rate(f, on1, sx1, sy1) : u_rr1;
-            if (RAINW) rr1 = rr1 * Win[f * pitch + gj];
-            // compensated depth: the state is the FP32 pair h + remainder, and the
-            // update is added with two error-free sums, so that changes below half
-            // an ulp of h (light rain on deep water) accumulate in the remainder
-            // instead of being rounded away, which would leave the FP32 state
-            // behind its FP64 budget.  The fast two-sum is exact here: an update
-            // larger than the depth either drains the cell (clamped below) or
-            // fills it from 0, and the remainder is below an ulp of the depth.
-            float d;
-            if constexpr (FORM == kFormUniform && !RAINW) {
-                d = (us - un) * ndx + (ve - vw) * ndy + (hi ? f1_hi : f1_lo);
-            } else {
-                d = __fmul_rn(-dt2, (us - un) * rdx + (ve - vw) * rdy - ql1 - rr1 * pct1 + ev1);
-            }
-            float s, e, hn, rn;
-            fast_two_sum(ho, d, s, e);
-            fast_two_sum(s, __fadd_rn(res3, e), hn, rn);
-            if (hn < 0.f) {  // fmax(h, 0) (cu:657) of the pair
-                clampv = -__fadd_rn(hn, rn);
-                hn = 0.f;
-                rn = 0.f;
-            }
-            hw_3 = hn;
-            hres = rn;
-        }
-        const float hwW = shup(hw_3);
-        if (out_col && f >= R0) {  // f <= R1 - 1 always
-            const int gp = f * pitch + gj;
-            Hout[gp] = hw_3;
-            Rout[gp] = hres;
-            Uout[gp] = un;
-            Vout[gp] = vw;
-            if (f == rows - 1) {  // south face, and the depth copy below the last row
-                Uout[gp + pitch] = us;
-                Hout[gp + pitch] = hw_3;
-                A.out += us;
-            }
+        float hw_3 = 0.f;
+        if (!SKIP || r >= R0 + 2) {
+            const unsigned dbW = __shfl_up_sync(0xffffffffu, db, 1);
+            const bool m3 = (mb >> 3) & 1u, m4 = (mb >> 4) & 1u, mL3 = (mLb >> 3) & 1u;
+            const bool d2 = db & 1u, d3 = (db >> 1) & 1u, d4 = (db >> 2) & 1u, dW3 = (dbW >> 1) & 1u;
+            float un = rum_3;  // x-face north of the row-(r-3) cell
+            if ((un > 0.f && d4) || (un < 0.f && d3)) un = 0.f;
+            float us = rum_2;  // x-face south of it
+            if ((us > 0.f && d3) || (us < 0.f && d2)) us = 0.f;
+            float vw = rvn_3;  // y-face west of it
+            if ((vw > 0.f && dW3) || (vw < 0.f && d3)) vw = 0.f;
+            const float ve = shdn(vw);
+            const int f = r - 3;
+            float hres = 0.f, clampv = 0.f, rr1 = 0.f, pct1 = 0.f, ev1 = 0.f, ql1 = 0.f;
             if (m3) {
+                const float ho = h3;
+                const bool hi = ho >= gt_ev;
+                pct1 = hi ? pct_hi : pct_lo;
+                ev1 = hi ? u_ev1 : 0.f;
+                ql1 = nsrc ? source_at(f, true) : 0.f;
+                rr1 = storm ? storm_rate(f, on1, sx1, sy1) : u_rr1;
+                if (RAINW) rr1 = rr1 * Win[f * pitch + gj];
+                // compensated depth: the state is the FP32 pair h + remainder, and the
+                // update is added with two error-free sums, so that changes below half
+                // an ulp of h (light rain on deep water) accumulate in the remainder
+                // instead of being rounded away, which would leave the FP32 state
+                // behind its FP64 budget.  The fast two-sum is exact here: an update
+                // larger than the depth either drains the cell (clamped below) or
+                // fills it from 0, and the remainder is below an ulp of the depth.
+                float d;
                 if constexpr (FORM == kFormUniform && !RAINW) {
-                    A.n_act++;
-                    A.n_hi += h3 >= gt_ev ? 1 : 0;
+                    d = (us - un) * ndx + (ve - vw) * ndy + (hi ? f1_hi : f1_lo);
                 } else {
-                    A.rain += rr1 * pct1;
-                    A.src += ql1;
-                    A.ev += ev1;
+                    d = __fmul_rn(-dt2, (us - un) * rdx + (ve - vw) * rdy - ql1 - rr1 * pct1 + ev1);
                 }
-                A.clamp += clampv;
-                // CFL bound of the new state on the owned faces (extension)
-                if (m4) {
-                    const float hm = 0.50f * (hw_3 + hw_4);
-                    if (hm >= ge_th) A.cm = fmaxf(A.cm, wave_speed(un, hm));
+                float s, e, hn, rn;
+                fast_two_sum(ho, d, s, e);
+                fast_two_sum(s, __fadd_rn(res3, e), hn, rn);
+                if (hn < 0.f) {  // fmax(h, 0) (cu:657) of the pair
+                    clampv = -__fadd_rn(hn, rn);
+                    hn = 0.f;
+                    rn = 0.f;
                 }
-                if (f == rows - 1 && south_open && hw_3 >= ge_th)
-                    A.cm = fmaxf(A.cm, wave_speed(us, hw_3));
-                if (mL3) {
-                    const float hn = 0.50f * (hw_3 + hwW);
-                    if (hn >= ge_th) A.cm = fmaxf(A.cm, wave_speed(vw, hn));
-                }
+                hw_3 = hn;
+                hres = rn;
             }
-            if (!isfinite(hw_3 + un + vw)) A.bad = true;  // a NaN or an infinity in any of the three
-        }
+            const float hwW = shup(hw_3);
+            if (out_col && f >= R0) {  // f <= R1 - 1 always
+                const int gp = f * pitch + gj;
+                Hout[gp] = hw_3;
+                Rout[gp] = hres;
+                Uout[gp] = un;
+                Vout[gp] = vw;
+                if (f == rows - 1) {  // south face, and the depth copy below the last row
+                    Uout[gp + pitch] = us;
+                    Hout[gp + pitch] = hw_3;
+                    A.out += us;
+                }
+                if (m3) {
+                    if constexpr (FORM == kFormUniform && !RAINW) {
+                        A.n_act++;
+                        A.n_hi += h3 >= gt_ev ? 1 : 0;
+                    } else {
+                        A.rain += rr1 * pct1;
+                        A.src += ql1;
+                        A.ev += ev1;
+                    }
+                    A.clamp += clampv;
+                    // CFL bound of the new state on the owned faces (extension)
+                    if (m4) {
+                        const float hm = 0.50f * (hw_3 + hw_4);
+                        if (hm >= ge_th) A.cm = fmaxf(A.cm, wave_speed(un, hm));
+                    }
+                    if (f == rows - 1 && south_open && hw_3 >= ge_th)
+                        A.cm = fmaxf(A.cm, wave_speed(us, hw_3));
+                    if (mL3) {
+                        const float hn = 0.50f * (hw_3 + hwW);
+                        if (hn >= ge_th) A.cm = fmaxf(A.cm, wave_speed(vw, hn));
+                    }
+                }
+                if (!isfinite(hw_3 + un + vw)) A.bad = true;  // a NaN or an infinity in any of the three
+            }
 
+        }
         if constexpr (PIPE) {
             if (r == R0 + 5) {  // output rows R0 .. R0+2 written; every row above R0 read
                 __syncwarp();
