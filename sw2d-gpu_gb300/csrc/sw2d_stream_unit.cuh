@@ -344,6 +344,7 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
     // domain, whose zeros are the inactive-cell and wall values, so no load
     // needs a bounds test
     float p_h, p_hw, p_hE, p_vnE, p_dzx, p_dzy, p_n, p_um, p_vn, p_res;
+    float p_w = 0.f, w_3 = 0.f;  // rain factors of rows r-2 (read with row r) and r-3
     unsigned p_m;
     int gp = (R0 - 4) * pitch + gj;  // element offset of the next row to read (fields fit 32-bit offsets)
     const int gp0 = gp;
@@ -356,6 +357,7 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
         p_h = ld_state(Hin + gp);
         p_hw = ld_state(Hin + gp - 1);  // the west neighbour's depth, exact on lane 0 too
         p_res = lrow >= 3 ? ld_state(Rin + gp - 3 * pitch) : 0.f;  // remainder of row lrow-3, used with this row
+        if (RAINW) p_w = lrow >= 2 ? Win[gp - 2 * pitch] : 0.f;     // factor of row lrow-2, likewise
         lrow++;
         p_n = raster ? Nin[gp] : manning;
         p_m = (unsigned)Min[gp];
@@ -454,6 +456,7 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
         const float hE0 = p_hE, vnE0 = p_vnE;
         const float h0 = p_h, hL0 = p_hw, n0 = p_n, um0 = p_um, vn0 = p_vn;
         const float res3 = p_res;  // depth remainder of row r-3
+        const float w_2 = p_w;
         mb = (mb << 1) | p_m;
         const unsigned mL0 = __shfl_up_sync(0xffffffffu, p_m, 1);
         mLb = (mLb << 1) | mL0;
@@ -551,7 +554,7 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
                 const float evapo = hi ? u_ev0 : 0.f;
                 const float ql = nsrc ? source_at(r - 2, false) : 0.f;
                 float rr = storm ? storm_rate(r - 2, on0, sx0, sy0) : u_rr0;
-                if (RAINW) rr = rr * Win[(r - 2) * pitch + gj];
+                if (RAINW) rr = rr * w_2;
                 if constexpr (FORM == kFormUniform && !RAINW) {  // the cell's forcing is one select of per-warp values
                     hs_2 = fmaxf(ho + ((rum_1 - rum_2) * ndx + (rvnE_2 - rvn_2) * ndy) + (hi ? f0_hi : f0_lo), 0.f);
                 } else {
@@ -586,7 +589,7 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
                 ev1 = hi ? u_ev1 : 0.f;
                 ql1 = nsrc ? source_at(f, true) : 0.f;
                 rr1 = storm ? storm_rate(f, on1, sx1, sy1) : u_rr1;
-                if (RAINW) rr1 = rr1 * Win[f * pitch + gj];
+                if (RAINW) rr1 = rr1 * w_3;
                 // compensated depth: the state is the FP32 pair h + remainder, and the
                 // update is added with two error-free sums, so that changes below half
                 // an ulp of h (light rain on deep water) accumulate in the remainder
@@ -666,6 +669,7 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
         vnE1 = vnE0;
         rum_3 = rum_2; rum_2 = rum_1; rvn_3 = rvn_2; rvn_2 = rvn_1;
         hw_4 = hw_3;
+        if (RAINW) w_3 = w_2;
         fx_1 = fx_0; cy_1 = cy_0;
         hmf_1 = hmf; hnf_1 = hnf;
     }
