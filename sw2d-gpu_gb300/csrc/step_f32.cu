@@ -55,11 +55,12 @@ cudaError_t prepare_stream_step(int variant) {
     }
     // the default build's forms for short strips
     if (variant == 0) {
-        const void *k[4] = {(const void *)stream_step_kernel<2, 10, 2, false, kFormUniform, true>,
+        const void *k[5] = {(const void *)stream_step_kernel<2, 10, 2, false, kFormUniform, true>,
                             (const void *)stream_step_kernel<2, 10, 2, false, kFormStorm, true>,
+                            (const void *)stream_step_kernel<2, 10, 2, false, kFormSources, true>,
                             (const void *)stream_step_kernel<2, 10, 2, false, kFormAny, true>,
                             (const void *)stream_step_kernel<2, 10, 2, true, kFormUniform, true>};
-        for (int i = 0; i < 4; i++) {
+        for (int i = 0; i < 5; i++) {
             cudaError_t e = cudaFuncSetAttribute(k[i], cudaFuncAttributePreferredSharedMemoryCarveout,
                                                  kStreamCarveoutPercent);
             if (e != cudaSuccess) return e;
@@ -67,12 +68,13 @@ cudaError_t prepare_stream_step(int variant) {
     }
 #define SW2D_P(id, nw, mb, un)                                                                            \
     if (variant == id) {                                                                               \
-        const void *k[5] = {(const void *)stream_step_kernel<nw, mb, un, false, kFormUniform, false>,         \
+        const void *k[6] = {(const void *)stream_step_kernel<nw, mb, un, false, kFormUniform, false>,         \
                             (const void *)stream_step_kernel<nw, mb, un, false, kFormStorm, false>,           \
+                            (const void *)stream_step_kernel<nw, mb, un, false, kFormSources, false>,         \
                             (const void *)stream_step_kernel<nw, mb, un, false, kFormAny, false>,             \
                             (const void *)stream_step_kernel<nw, mb, un, true, kFormUniform, false>,          \
                             (const void *)stream_step_kernel<nw, mb, un, true, kFormAny, false>};             \
-        for (int i = 0; i < 5; i++) {                                                                  \
+        for (int i = 0; i < 6; i++) {                                                                  \
             cudaError_t e = cudaFuncSetAttribute(k[i], cudaFuncAttributePreferredSharedMemoryCarveout, \
                                                  kStreamCarveoutPercent);                             \
             if (e != cudaSuccess) return e;                                                            \
@@ -155,7 +157,9 @@ cudaError_t launch_stream_step(int variant, int nblocks, int tiles_w, int strip_
     const StreamShape sh = stream_shape(G.rows, tiles_w, strip_h, units, false, skew);
     // the build that carries the forcing that is set and no other
     const bool storm = F.rain_kind == RAIN_STORM;
-    const int form = G.n_src > 0 || (storm && S.rainw) ? kFormAny : (storm ? kFormStorm : kFormUniform);
+    const bool src = G.n_src > 0;
+    const int form = S.rainw ? (src || storm ? kFormAny : kFormUniform)
+                             : (storm ? (src ? kFormAny : kFormStorm) : (src ? kFormSources : kFormUniform));
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -198,6 +202,7 @@ cudaError_t launch_stream_step(int variant, int nblocks, int tiles_w, int strip_
         lc.blockDim = dim3(64);
         if (S.rainw && form == kFormUniform) SW2D_LK(2, 10, 2, true, kFormUniform, true);
         if (!S.rainw && form == kFormStorm) SW2D_LK(2, 10, 2, false, kFormStorm, true);
+        if (!S.rainw && form == kFormSources) SW2D_LK(2, 10, 2, false, kFormSources, true);
         if (!S.rainw && form == kFormAny) SW2D_LK(2, 10, 2, false, kFormAny, true);
         if (!S.rainw) SW2D_LK(2, 10, 2, false, kFormUniform, true);
     }
@@ -207,6 +212,7 @@ cudaError_t launch_stream_step(int variant, int nblocks, int tiles_w, int strip_
         if (S.rainw && form == kFormAny) SW2D_LK(nw, mb, un, true, kFormAny, false); \
         if (S.rainw) SW2D_LK(nw, mb, un, true, kFormUniform, false);                \
         if (form == kFormStorm) SW2D_LK(nw, mb, un, false, kFormStorm, false);      \
+        if (form == kFormSources) SW2D_LK(nw, mb, un, false, kFormSources, false);  \
         if (form == kFormAny) SW2D_LK(nw, mb, un, false, kFormAny, false);          \
         SW2D_LK(nw, mb, un, false, kFormUniform, false);                            \
     }

@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(NWARP * 32, MINB) batch_step_kernel(const Batc
             const int r0 = rs * S.strip_h;
             stream_unit<UNR, false, kFormUniform>(V, ct, r0, min(r0 + S.strip_h, V.rows), lane, nullptr, nullptr,
                                                   nullptr, nullptr, A);
-            warp_reduce_acc<true>(A);
+            warp_reduce_acc<false, kFormUniform>(A);
             if (lane == 0) accumulate_cmax(S.clk[slot_out], ue.y % kBuckets, (double)A.cm, A.bad);
             // the budgets, one per lane (B_RAIN .. B_CLAMP; no sources here): FP64
             // operations have long latencies and this warp is on the way to its ticket

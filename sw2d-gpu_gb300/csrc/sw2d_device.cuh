@@ -37,6 +37,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "sw2d_f64math.cuh"
+
 namespace sw2d {
 
 enum { B_RAIN = 0, B_SRC = 1, B_EV = 2, B_OUT = 3, B_CLAMP = 4, B_N = 5 };
@@ -236,14 +238,14 @@ __device__ inline double source_rate(const ForcingDesc &F, int n_src, int s, dou
     if (t <= 1.00) {
         q = F.src_q[s] * t;
     } else {
-        int it = (int)(t / F.dtoq);
+        int it = (int)d_div(t, F.dtoq);
         int a = it < F.n_qrec ? it : F.n_qrec - 1;
         int b = it + 1 < F.n_qrec ? it + 1 : F.n_qrec - 1;
         double qa = F.src_q[(size_t)a * n_src + s];
         double qb = F.src_q[(size_t)b * n_src + s];
-        q = qa + (qb - qa) / (F.dtoq * __dsub_rn(t, __dmul_rn(F.dtoq, (double)it)));
+        q = qa + d_div(qb - qa, F.dtoq * __dsub_rn(t, __dmul_rn(F.dtoq, (double)it)));
     }
-    return q / area;
+    return d_div(q, area);  // d_div: the plain quotient's bits, without its FP64 latency
 }
 
 // One of the two evaluations a plan needs at time tl: the step over the cell

@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(NWARP * 32, MINB)
             stream_unit<UNR, RAINW, FORM, false, true, true>(V, ct, r0, r1, lane, s_sr[wid], s_sc[wid], s_q0[wid],
                                                       s_q1[wid], A, nullptr, 0, nullptr, nullptr,
                                                       P.flags + SH.units + unit, (unsigned)(j + 1));
-            warp_reduce_acc<!RAINW && FORM == kFormUniform>(A);
+            warp_reduce_acc<RAINW, FORM>(A);
             if (lane == 0) {
                 const double scale = pl.d.dt2 * area;
                 s_acc[wid][B_RAIN] += acc_rain((double)A.rain, A.n_act, A.n_hi, pl.f, G.sf) * scale;

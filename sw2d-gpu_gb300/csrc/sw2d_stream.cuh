@@ -167,7 +167,7 @@ __device__ __forceinline__ void stream_step_body(const GridDesc &G, const Forcin
     }
 
     // ---- warp, then CTA reductions; one thread accumulates and finishes ----
-    warp_reduce_acc<!RAINW && FORM == kFormUniform>(A);
+    warp_reduce_acc<RAINW, FORM>(A);
     if (lane == 0) {
         s_red[wid][B_RAIN] = A.rain;
         s_red[wid][B_SRC] = A.src;

@@ -7,6 +7,8 @@
 // sw2d_stream.cuh for the layout of the pipeline and the halo).
 #pragma once
 
+#include <climits>
+
 #include <cuda.h>
 
 #include "sw2d_device.cuh"
@@ -131,11 +133,15 @@ __device__ __forceinline__ bool dry_bed_dz(const Thr<float> &T, float g, float h
 }
 
 // Forcing forms of the unit: rain uniform over the grid, the moving storm alone,
-// or whichever of storm and point sources the handle has set.  Sources under
-// uniform rain have no form of their own: one without the storm, and warps
-// without local sources in a copy of the loop without them, both measured the
-// same as kFormAny (40.3 us at 701 x 1237).
-enum { kFormUniform = 0, kFormStorm = 1, kFormAny = 2 };
+// point sources under uniform rain, or whichever of storm and sources the handle
+// has set.
+enum { kFormUniform = 0, kFormStorm = 1, kFormSources = 2, kFormAny = 3 };
+
+// Whether a form counts cells instead of adding rain rates (StreamAcc); with
+// sources it measured 1 % slower than the sums.
+__host__ __device__ constexpr bool counts_rain(bool rainw, int form) {
+    return !rainw && form == kFormUniform;
+}
 
 // Everything a warp reads to advance one strip of one scenario.
 struct StreamView {
@@ -232,6 +238,7 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
                                             StreamAcc &A, const TmaMaps *M = nullptr, int buf = 0,
                                             unsigned char *stg = nullptr, unsigned long long *bars = nullptr,
                                             unsigned *top_flag = nullptr, unsigned top_val = 0u) {
+    constexpr bool kSources = FORM == kFormSources || FORM == kFormAny;
     const int rows = wuni(V.rows), cols = wuni(V.cols), pitch = wuni(V.pitch), south_open = wuni(V.south_open);
     const float dt2 = wuni(V.LS.dt2), dt2dx = wuni(V.LS.dt2dx), dt2dy = wuni(V.LS.dt2dy);
     const float u_ev0 = wuni(V.LS.ev0), u_ev1 = wuni(V.LS.ev1), u_rr0 = wuni(V.LS.rr0), u_rr1 = wuni(V.LS.rr1);
@@ -295,7 +302,7 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
     // point sources inside this warp's window, in list order (the later one
     // wins on a shared cell, as the reference's assignment, cu:545)
     int nsrc = 0;
-    if (FORM == kFormAny && V.n_src > 0) {
+    if (kSources && V.n_src > 0) {
         const double area = V.dx * V.dy;
         for (int base = 0; base < V.n_src; base += 32) {
             const int s = base + lane;
@@ -313,14 +320,21 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
                 if (off < kStreamMaxSrc) {
                     s_sr[off] = sr;
                     s_sc[off] = sc;
-                    s_q0[off] = (float)source_rate(*V.F, V.n_src, s, V.t0, area);
-                    s_q1[off] = (float)source_rate(*V.F, V.n_src, s, V.t1, area);
+                    s_q0[off] = __int_as_float(s);  // the source's index, until its rates replace it
                 } else {
                     A.too_many_sources = true;
                 }
             }
             nsrc += __popc(bal);
         }
+        // the rates at t and t + dt (FP64, long latencies): two lanes per source
+        __syncwarp();
+        static_assert(2 * kStreamMaxSrc <= 32, "one lane per rate");
+        const int e = lane >> 1;
+        const bool mine = e < min(nsrc, kStreamMaxSrc);
+        const int src = mine ? __float_as_int(s_q0[e]) : 0;
+        __syncwarp();
+        if (mine) (lane & 1 ? s_q1 : s_q0)[e] = (float)source_rate(*V.F, V.n_src, src, lane & 1 ? V.t1 : V.t0, area);
         __syncwarp();
         nsrc = min(nsrc, kStreamMaxSrc);
     }
@@ -330,6 +344,34 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
             if (s_sr[e] == row && s_sc[e] == gj) q = second ? s_q1[e] : s_q0[e];
         return q;
     };
+    // Rows are visited in order, so the warp keeps the next row that holds a source
+    // and the row loop one test per row, at its end, that looks up the sources of
+    // the rows continuity handles next (q_a of row r-2 at t, q_b of row r-3 at t +
+    // dt): a search in every row had made the warps with sources the last to finish.
+    int src_row = INT_MAX, src_prev = INT_MAX - 1;  // next source row; the row q_a was last for
+    float q_a = 0.f, q_b = 0.f;
+    auto next_source_row = [&](int after) -> int {
+        int n = INT_MAX;
+        for (int e = 0; e < nsrc; e++)
+            if (s_sr[e] > after) n = min(n, s_sr[e]);
+        return wuni(n);
+    };
+    auto sources_for = [&](int row) {  // row: r-2 of the next iteration
+        q_a = q_b = 0.f;
+        if (row >= min(src_row, src_prev)) {
+            if (row == src_prev + 1) q_b = source_at(src_prev, true);
+            src_prev = INT_MAX - 1;
+            if (row == src_row) {
+                q_a = source_at(row, false);
+                src_prev = row;
+                src_row = next_source_row(row);
+            }
+        }
+    };
+    if (kSources && nsrc > 0) {
+        src_row = next_source_row(R0 - 7);
+        sources_for(R0 - 6);
+    }
     auto storm_rate = [&](int row, bool on, float sx, float sy) -> float {
         if (!on) return 0.f;
         const float x = ((float)gj + 0.5f) * dx - sx;
@@ -552,7 +594,7 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
                 const bool hi = ho >= gt_ev;
                 const float pct = hi ? pct_hi : pct_lo;
                 const float evapo = hi ? u_ev0 : 0.f;
-                const float ql = nsrc ? source_at(r - 2, false) : 0.f;
+                const float ql = kSources ? q_a : 0.f;
                 float rr = storm ? storm_rate(r - 2, on0, sx0, sy0) : u_rr0;
                 if (RAINW) rr = rr * w_2;
                 if constexpr (FORM == kFormUniform && !RAINW) {  // the cell's forcing is one select of per-warp values
@@ -587,7 +629,7 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
                 const bool hi = ho >= gt_ev;
                 pct1 = hi ? pct_hi : pct_lo;
                 ev1 = hi ? u_ev1 : 0.f;
-                ql1 = nsrc ? source_at(f, true) : 0.f;
+                ql1 = kSources ? q_b : 0.f;
                 rr1 = storm ? storm_rate(f, on1, sx1, sy1) : u_rr1;
                 if (RAINW) rr1 = rr1 * w_3;
                 // compensated depth: the state is the FP32 pair h + remainder, and the
@@ -627,7 +669,7 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
                     A.out += us;
                 }
                 if (m3) {
-                    if constexpr (FORM == kFormUniform && !RAINW) {
+                    if constexpr (counts_rain(RAINW, FORM)) {
                         A.n_act++;
                         A.n_hi += h3 >= gt_ev ? 1 : 0;
                     } else {
@@ -660,6 +702,8 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
             }
         }
 
+        if (kSources) sources_for(r - 1);
+
         // ---- advance the rings ----
         h3 = h2; h2 = h1; h1 = h0; hL1 = hL0;
         n2 = n1; n1 = n0; nL1 = nL0;
@@ -676,20 +720,20 @@ __device__ __forceinline__ void stream_unit(const StreamView &V, const int ct, c
 }
 
 // Warp reduction of a StreamAcc: sums / max / any into lane 0's return.
-// UNIFORM: the uniform-forcing form's counts instead of the rate sums.
-template <bool UNIFORM>
+template <bool RAINW, int FORM>
 __device__ __forceinline__ void warp_reduce_acc(StreamAcc &A) {
-    if constexpr (UNIFORM) {
+    constexpr bool kCounts = counts_rain(RAINW, FORM), kSources = FORM == kFormSources || FORM == kFormAny;
+    if constexpr (kCounts) {
         A.n_act = __reduce_add_sync(0xffffffffu, A.n_act);
         A.n_hi = __reduce_add_sync(0xffffffffu, A.n_hi);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        if constexpr (!UNIFORM) {
+        if constexpr (!kCounts) {
             A.rain += __shfl_xor_sync(0xffffffffu, A.rain, o);
-            A.src += __shfl_xor_sync(0xffffffffu, A.src, o);
             A.ev += __shfl_xor_sync(0xffffffffu, A.ev, o);
         }
+        if constexpr (kSources) A.src += __shfl_xor_sync(0xffffffffu, A.src, o);
         A.out += __shfl_xor_sync(0xffffffffu, A.out, o);
         A.clamp += __shfl_xor_sync(0xffffffffu, A.clamp, o);
         A.cm = fmaxf(A.cm, __shfl_xor_sync(0xffffffffu, A.cm, o));
