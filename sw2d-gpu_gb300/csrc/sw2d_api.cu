@@ -12,7 +12,11 @@
 #include <cstring>
 #include <new>
 #include <string>
+#include <thread>
 #include <vector>
+
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <cuda_runtime.h>
 
@@ -881,6 +885,54 @@ int sw2d_advance(sw2d_handle *h, int64_t max_steps, double t_end, int64_t *steps
     return SW2D_OK;
 }
 
+namespace {
+
+// Brings the pages of a large output buffer in before a copy fills it, by a few
+// threads: a fresh buffer (an array just allocated by the caller) takes a page
+// fault per page, one after the other, when the copy first touches it -- 8192 x
+// 8192 float64 20.9 ms against 3.2 into a buffer in use, and 9.5 this way; 3000 x
+// 3000 4.1 and 2.7.  A buffer whose sampled pages are resident is left alone, and
+// so is one whose sampled pages cannot be written or whose system does not say
+// (MADV_POPULATE_WRITE): the copy then goes as it always did.  Only the first
+// byte of each page is written, which the copy overwrites.
+void touch_output(void *out, size_t bytes) {
+    constexpr int kPopulateWrite = 23;           // MADV_POPULATE_WRITE, Linux 5.14
+    constexpr size_t kLeast = (size_t)16 << 20;  // below, starting threads costs more than the faults
+    if (bytes < kLeast) return;
+    const long ps = sysconf(_SC_PAGESIZE);
+    if (ps <= 0) return;
+    const size_t page = (size_t)ps;
+    const uintptr_t lo = ((uintptr_t)out + page - 1) / page * page, hi = ((uintptr_t)out + bytes) / page * page;
+    if (hi <= lo) return;
+    const size_t pages = (hi - lo) / page;
+    constexpr int kSamples = 9;  // the first and last page among them
+    auto sample = [=](int k) { return (void *)(lo + (pages - 1) * k / (kSamples - 1) * page); };
+    int resident = 0;
+    for (int k = 0; k < kSamples; k++) {
+        unsigned char in = 0;
+        if (mincore(sample(k), page, &in) != 0) return;
+        resident += in & 1;
+    }
+    if (2 * resident > kSamples) return;
+    for (int k = 0; k < kSamples; k++)
+        if (madvise(sample(k), page, kPopulateWrite) != 0) return;
+    const unsigned hw = std::thread::hardware_concurrency();
+    const size_t n = hw < 2 ? 1 : (hw < 8 ? hw : 8);
+    auto touch = [=](size_t t) {
+        for (size_t k = pages * t / n; k < pages * (t + 1) / n; k++) *(volatile char *)(lo + k * page) = 0;
+    };
+    std::thread workers[8];
+    size_t started = 1;
+    try {
+        for (; started < n; started++) workers[started] = std::thread(touch, started);
+    } catch (...) {  // no thread: the copy takes the rest of the faults
+    }
+    touch(0);
+    for (size_t t = 1; t < started; t++) workers[t].join();
+}
+
+}  // namespace
+
 int sw2d_get_field(sw2d_handle *h, int32_t field, double *out) {
     if (!h || !out) return fail(h, SW2D_ERR_INVALID_ARG, "null argument");
     if (!h->have_state && field != SW2D_FIELD_ELEVATION) return fail(h, SW2D_ERR_STATE, "no state");
@@ -903,6 +955,7 @@ int sw2d_get_field(sw2d_handle *h, int32_t field, double *out) {
             CK(h, launch_velocity((const float *)h->h[b], (const float *)h->um[b], (const float *)h->vn[b], rows, cols,
                                   pitch, make_thr<float>(h->cfg).ge_th, h->stage, h->stage2, h->stream));
         const double *s = field == SW2D_FIELD_UU ? h->stage : h->stage2;
+        touch_output(out, (size_t)rows * cols * sizeof(double));
         CK(h, cudaMemcpyAsync(out, s, (size_t)rows * cols * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
         CK(h, cudaStreamSynchronize(h->stream));
         return SW2D_OK;
@@ -912,6 +965,7 @@ int sw2d_get_field(sw2d_handle *h, int32_t field, double *out) {
     }
     if (f64) CK(h, launch_unpack((const double *)src, (const double *)add, nr, nc, pitch, h->stage, h->stream));
     else CK(h, launch_unpack((const float *)src, (const float *)add, nr, nc, pitch, h->stage, h->stream));
+    touch_output(out, (size_t)nr * nc * sizeof(double));
     CK(h, cudaMemcpyAsync(out, h->stage, (size_t)nr * nc * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
     return SW2D_OK;
