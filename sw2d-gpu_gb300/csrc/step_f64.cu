@@ -66,7 +66,7 @@ cudaError_t prepare_step64(int th, int tw) {
     if (th == h && tw == w) {                                                                                   \
         const cudaError_t e2 = cudaFuncSetAttribute(step64_kernel<h, w, nt, mb>,                                \
                                                     cudaFuncAttributeMaxDynamicSharedMemorySize,                \
-                                                    (int)Step64Shape<h, w>::kSmem);                            \
+                                                    (int)Step64Shape<h, w>::smem(nt / 32));                    \
         if (e2 != cudaSuccess) return e2;                                                                       \
         return cudaFuncSetAttribute(step64_kernel<h, w, nt, mb>, cudaFuncAttributePreferredSharedMemoryCarveout, \
                                     (int)cudaSharedmemCarveoutMaxShared);                                       \
@@ -101,7 +101,7 @@ cudaError_t launch_step64(int th, int tw, int nblocks, int sms, const GridDesc &
 #define SW2D_L64(h, w, nt, mb)                                                                             \
     if (th == h && tw == w) {                                                                              \
         lc.blockDim = dim3(nt);                                                                            \
-        lc.dynamicSmemBytes = Step64Shape<h, w>::kSmem;                                                    \
+        lc.dynamicSmemBytes = Step64Shape<h, w>::smem(nt / 32);                                            \
         return cudaLaunchKernelEx(&lc, step64_kernel<h, w, nt, mb>, G, F, S, T, X, clk, ctl, slot);        \
     }
     SW2D_STEP64_TILES(SW2D_L64)

@@ -185,3 +185,22 @@ def test_step64_tile_rule(sw2d_mod):
                                  (64, 64, dict(tile_h=8, tile_w=32), "8,32")):
         with sw2d_mod.Solver(rows=rows, cols=cols, dx=1.0, dy=1.0, **kw) as g:
             assert g.describe().startswith("step_kernel<double,%s>" % name), g.describe()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tile", TILES)
+@pytest.mark.parametrize("shape", [(16, 32), (37, 70)])
+def test_step64_every_flux_at_once(oracle_mod, sw2d_mod, tile, shape):
+    """Deep water moving everywhere: all four fluxes of every element are
+    formed, so a warp's list is flushed before its last block of elements."""
+    rows, cols = shape
+    rng = np.random.default_rng(rows)
+    z = rng.uniform(0.0, 0.1, shape)
+    h = rng.uniform(2.0, 3.0, shape)
+    o, g = make_pair(oracle_mod, sw2d_mod, rows, cols, 4.0, z, h, n=rng.uniform(0.02, 0.1, shape), dt=0.1, tile=tile)
+    assert o.advance(20, 1e9) == g.advance(20, 1e9) == 20
+    a, b = o.state(), g.state()
+    assert np.count_nonzero(a["um"]) >= (rows - 1) * cols and np.count_nonzero(a["vn"]) >= rows * (cols - 1)
+    for k in ("h", "um", "vn"):
+        assert same(a[k], b[k]), (k, np.max(np.abs(a[k] - b[k])))
+    g.close()
