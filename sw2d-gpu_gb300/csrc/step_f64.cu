@@ -19,22 +19,33 @@ cudaError_t init_det_tables() {
 
 // Builds of the step kernel: (tile rows, tile columns, threads, minimum
 // resident CTAs per SM).  16 x 32 runs two CTAs of 512 threads per SM, whose
-// stages overlap: 313 us per iteration on a 1013 x 900 catchment, 447 with one
+// stages overlap: 312 us per iteration on a 1013 x 900 catchment, 447 with one
 // CTA of 768 (the stages then wait at each other's barriers), 358 with one CTA on
 // a 32 x 32 tile (less halo, same wait); 256 to 448 threads are within 3 %.
 //
-// The smaller tiles are for grids that would leave SMs without a CTA: a tile's
-// work runs on one SM, so a grid is cut into the smallest tiles that still give
-// one CTA per SM (step64_tile).  Measured with the first form of the kernel, us
-// per iteration, tiles 4x8 / 4x16 / 8x16 / 8x32 / 16x32: 64 x 64 23.8 / 27.0 /
-// 30.3 / 42.3 / 53.5; 117 x 131 48.8 / 42.8 / 34.5 / 47.5 / 60.2; 256 x 256 159 /
-// 106 / 79 / 72 / 69.5; 512 x 512 593 / 327 / 261 / 225 / 185 (the halo costs 2.3
-// times the faces of the tile at 4 x 8, 1.4 at 16 x 32); the final form runs 18.9,
-// 23.2, 43 and 106 on the tile the rule takes.  With one CTA per SM more threads
-// shorten the stages: 8 x 16 23.2 with 512 against 26.9 with 256, 8 x 32 30.6 with
-// 768 against 34.2 with 384.
-#define SW2D_STEP64_TILES(X) \
-    X(16, 32, 512, 2) X(8, 32, 768, 1) X(8, 16, 512, 1) X(4, 16, 256, 1) X(4, 8, 256, 1)
+// A tile's work runs on one SM, and an iteration takes as long as the SM with the
+// most of it: a grid of one CTA per SM, or of two, is cut into the smallest tiles
+// that still leave it so (step64_tile).  us per iteration, tiles 16x32 / 14x32 /
+// 12x32 / 10x32 / 8x32 / 6x32, the one that the rule takes in brackets:
+//   140 x 160  40.1 /  38.3  /  33.9  /  32.3  / 30.4 / (26.4)
+//   180 x 256  42.1 /  40.5  /  38.2  / (34.1) / 55.6 /  49.4
+//   200 x 256  43.6 /  40.2  / (38.4) /  55.3  / 56.6 /  50.0
+//   256 x 256  44.3 / (42.4) /  62.4  /  59.7  / 58.3 /  69.8
+// and, where two CTAs of 512 per SM hold the grid, 16x32 / 14x32: 256 x 512 63.5 /
+// (57.2), 270 x 480 60.6 / (57.2), 256 x 370 59.2 / (54.8), 270 x 300 55.6 /
+// (54.4); with few more CTAs of 16 x 32 than SMs most of these run alone, and
+// 14 x 32 is the slower: 256 x 300 (160 CTAs) (48.4) / 51.9, 656 x 128 (164) (45.0)
+// / 47.2; from 170 on it is the faster or within 4 % (672 x 128, 130 x 700).  The
+// narrow tiles, 8x16 / 4x16 / 4x8: 64 x 64 21.7 / 20.1 / (18.6), 80 x 100 22.2 /
+// (20.6) / 20.9, 117 x 131 (23.0) / 25.9 / 37.5.  Beyond two CTAs per SM the halo
+// decides (4 x 8 has 2.3 faces for each one of the tile, 14 x 32 1.5, 16 x 32
+// 1.4): 16x32 / 14x32 300 x 500 63.0 / 83.9, 400 x 400 79.2 / 82.5, 1013 x 900
+// 312 / 334.  With one CTA per SM more threads shorten the stages: 8 x 16 23.2
+// with 512 against 26.9 with 256, 8 x 32 30.6 with 768 against 34.2 with 384,
+// 10 x 32 33.1 with 768 against 34.8 with 512.
+#define SW2D_STEP64_TILES(X)                                                                        \
+    X(16, 32, 512, 2) X(14, 32, 512, 2) X(12, 32, 768, 1) X(10, 32, 768, 1) X(8, 32, 768, 1)        \
+    X(6, 32, 512, 1) X(8, 16, 512, 1) X(4, 16, 256, 1) X(4, 8, 256, 1)
 
 bool step64_tile_supported(int th, int tw) {
 #define SW2D_S64(h, w, nt, mb) \
@@ -44,17 +55,24 @@ bool step64_tile_supported(int th, int tw) {
     return false;
 }
 
-// The smallest tile with at most one CTA per SM, 16 x 32 beyond.
+// The smallest tile whose CTAs all have an SM to themselves; else the smallest of
+// which all are resident where two run per SM, if 16 x 32 would give more than a
+// twelfth of the SMs a second one; else 16 x 32.
 void step64_tile(int rows, int cols, int sms, int *th, int *tw) {
+    auto ctas = [&](int h, int w) { return (long long)((rows + h - 1) / h) * ((cols + w - 1) / w); };
     *th = 16;
     *tw = 32;
-    long long best = 16 * 32;
-#define SW2D_D64(h, w, nt, mb)                                                                       \
-    if (h * w < best && (long long)((rows + h - 1) / h) * ((cols + w - 1) / w) <= sms) {             \
-        best = h * w;                                                                                \
-        *th = h;                                                                                     \
-        *tw = w;                                                                                     \
+    int best = 16 * 32;
+#define SW2D_D64(h, w, nt, mb)                                        \
+    if (h * w < best && mb >= per_sm && ctas(h, w) <= per_sm * sms) { \
+        best = h * w;                                                 \
+        *th = h;                                                      \
+        *tw = w;                                                      \
     }
+    int per_sm = 1;
+    SW2D_STEP64_TILES(SW2D_D64)
+    if (best < 16 * 32 || ctas(16, 32) <= sms + sms / 12) return;
+    per_sm = 2;
     SW2D_STEP64_TILES(SW2D_D64)
 #undef SW2D_D64
 }

@@ -204,3 +204,23 @@ def test_step64_every_flux_at_once(oracle_mod, sw2d_mod, tile, shape):
     for k in ("h", "um", "vn"):
         assert same(a[k], b[k]), (k, np.max(np.abs(a[k] - b[k])))
     g.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tile", [(14, 32), (12, 32), (10, 32), (6, 32)])
+@pytest.mark.parametrize("shape", [(1, 33), (6, 32), (15, 31), (41, 66)])
+def test_step64_tiles_between_match_the_oracle(oracle_mod, sw2d_mod, tile, shape):
+    """The tile heights between 4 and 16, as above: film with NODATA cells,
+    storm, rain with evaporation and point sources; rows that the tile divides,
+    one less, one more."""
+    test_step64_tiles_match_the_oracle(oracle_mod, sw2d_mod, tile, shape)
+
+
+@pytest.mark.gpu
+def test_step64_tile_rule_fills_the_sms(sw2d_mod):
+    """Where no SM, or no SM more than two, CTAs: the smallest tile that leaves
+    it so (152 SMs)."""
+    for rows, cols, name in ((150, 150, "6,32"), (180, 256, "10,32"), (200, 256, "12,32"), (256, 256, "14,32"),
+                             (256, 512, "14,32"), (300, 500, "16,32"), (256, 300, "16,32"), (1013, 900, "16,32")):
+        with sw2d_mod.Solver(rows=rows, cols=cols, dx=1.0, dy=1.0) as g:
+            assert g.describe().startswith("step_kernel<double,%s>" % name), g.describe()
