@@ -7,16 +7,25 @@
 
 namespace sw2d {
 
+// The forms of a build: uniform rain as the build unrolls it, the others with the
+// row loop not unrolled: unrolled by 2, build 0 with both the storm and the
+// sources spilled 492 bytes, which in strips of more than a few rows cost more
+// than the pipelining saves; not unrolled it spills 28, with the sources alone 16
+// and with the storm alone 52.  us per iteration, 701 x 1237 / 1500 x 1500: storm
+// 55.5 / 115 -> 25.7 / 50.1, sources 54.7 / 108 -> 26.5 / 50.8, both 59.9 / 120 ->
+// 27.2 / 55.0, storm and rain factors 61.7 / 134 -> 28.0 / 56.4.
 cudaError_t prepare_stream_pipe(int variant) {
 #define SW2D_P(id, nw, mb, un)                                                                         \
     if (variant == id) {                                                                               \
-        const void *k[4] = {(const void *)stream_pipe_kernel<nw, mb, un, false, kFormUniform>,         \
-                            (const void *)stream_pipe_kernel<nw, mb, un, false, kFormAny>,             \
+        const void *k[6] = {(const void *)stream_pipe_kernel<nw, mb, un, false, kFormUniform>,         \
+                            (const void *)stream_pipe_kernel<nw, mb, 1, false, kFormStorm>,            \
+                            (const void *)stream_pipe_kernel<nw, mb, 1, false, kFormSources>,          \
+                            (const void *)stream_pipe_kernel<nw, mb, 1, false, kFormAny>,              \
                             (const void *)stream_pipe_kernel<nw, mb, un, true, kFormUniform>,          \
-                            (const void *)stream_pipe_kernel<nw, mb, un, true, kFormAny>};             \
-        for (int i = 0; i < 4; i++) {                                                                  \
-            cudaError_t e = cudaFuncSetAttribute(k[i], cudaFuncAttributePreferredSharedMemoryCarveout, \
-                                                 kStreamCarveoutPercent);                             \
+                            (const void *)stream_pipe_kernel<nw, mb, 1, true, kFormAny>};              \
+        for (const void *f : k) {                                                                      \
+            cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout,    \
+                                                 kStreamCarveoutPercent);                              \
             if (e != cudaSuccess) return e;                                                            \
         }                                                                                              \
         return cudaSuccess;                                                                            \
@@ -59,7 +68,7 @@ cudaError_t launch_stream_pipe(int variant, int nblocks, int tiles_w, int strip_
     P.plans = plans;
     P.words = words;
     P.flags = flags;
-    const bool gen = F.rain_kind == RAIN_STORM || G.n_src > 0;
+    const bool storm = F.rain_kind == RAIN_STORM, src = G.n_src > 0;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;  // every unit resident: the waits between units end
     attr[0].val.cooperative = 1;
@@ -73,20 +82,21 @@ cudaError_t launch_stream_pipe(int variant, int nblocks, int tiles_w, int strip_
     lc.attrs = attr;
     lc.numAttrs = 1;
     if (variant == kTmaVariant) variant = 0;
-#define SW2D_PL(id, nw, mb, un)                                                                            \
-    if (variant == id) {                                                                                 \
-        lc.blockDim = dim3(nw * 32);                                                                     \
-        if (S.rainw && gen)                                                                              \
-            return cudaLaunchKernelEx(&lc, stream_pipe_kernel<nw, mb, un, true, kFormAny>, G, F, S, T, clk, ctl, slot, sh, P);   \
-        else if (S.rainw)                                                                                \
-            return cudaLaunchKernelEx(&lc, stream_pipe_kernel<nw, mb, un, true, kFormUniform>, G, F, S, T, clk, ctl, slot, sh, P);  \
-        else if (gen)                                                                                    \
-            return cudaLaunchKernelEx(&lc, stream_pipe_kernel<nw, mb, un, false, kFormAny>, G, F, S, T, clk, ctl, slot, sh, P);  \
-        else                                                                                             \
-            return cudaLaunchKernelEx(&lc, stream_pipe_kernel<nw, mb, un, false, kFormUniform>, G, F, S, T, clk, ctl, slot, sh, P); \
+#define SW2D_PK(nw, mb, un, w, form) \
+    return cudaLaunchKernelEx(&lc, stream_pipe_kernel<nw, mb, un, w, form>, G, F, S, T, clk, ctl, slot, sh, P)
+#define SW2D_PL(id, nw, mb, un)                                     \
+    if (variant == id) {                                            \
+        lc.blockDim = dim3(nw * 32);                                \
+        if (S.rainw && (storm || src)) SW2D_PK(nw, mb, 1, true, kFormAny); \
+        if (S.rainw) SW2D_PK(nw, mb, un, true, kFormUniform);       \
+        if (storm && src) SW2D_PK(nw, mb, 1, false, kFormAny);      \
+        if (storm) SW2D_PK(nw, mb, 1, false, kFormStorm);           \
+        if (src) SW2D_PK(nw, mb, 1, false, kFormSources);           \
+        SW2D_PK(nw, mb, un, false, kFormUniform);                   \
     }
     SW2D_STREAM_VARIANTS(SW2D_PL)
 #undef SW2D_PL
+#undef SW2D_PK
     return cudaErrorInvalidValue;
 }
 

@@ -170,15 +170,14 @@ cudaError_t launch_one(sw2d_handle *h, int slot) {
                        make_thr<float>(h->cfg), h->d_clk, h->d_ctl, slot, h->stream);
 }
 
-// Whether advance runs several iterations per launch now: the pipelined form
-// with the storm or point sources compiled in spills at 96 registers and
-// measured 0.86-0.94x one launch per iteration on 256^2 to 1024^2, so the
-// library's own choice of it (not one the caller asked for) stands down
-// while that forcing is set.
+// Whether advance runs several iterations per launch now.  The library's own
+// choice of it (not one the caller asked for) stands down while a moving storm
+// is set: a storm's iterations gain little from it (us per iteration, one launch
+// each against 48 per launch: 128 x 128 18.9 / 17.5, 512 x 512 18.2 / 17.6, 1500 x
+// 1500 49.8 / 50.1).  Point sources stay with it: 21.5 / 19.0, 21.3 / 18.6, 701 x
+// 1237 29.7 / 26.5, 1500 x 1500 55.5 / 50.8; with rain factors too.
 bool pipe_now(const sw2d_handle *h) {
-    if (h->pipe_k <= 0) return false;
-    const bool gen = h->F.rain_kind == RAIN_STORM || h->G.n_src > 0;
-    return !(h->pipe_auto && gen);
+    return h->pipe_k > 0 && !(h->pipe_auto && h->F.rain_kind == RAIN_STORM);
 }
 
 int validate(const sw2d_config *c, std::string *why) {
@@ -319,8 +318,8 @@ int row_cost(long long warps_per_sm) { return warps_per_sm <= 8 ? 100 : (warps_p
 // finish first: a warp runs its rows plus 7 warm-up rows at row_cost, so a grid
 // that does not fill the GPU is cut into short strips (more warm-up rows in
 // all, but on warps that would otherwise be idle), down to one row.  us per
-// iteration, strips of 16 rows against the choice: 96 x 128 26.1 -> 14.1,
-// 256 x 256 26.2 -> 15.7, 512 x 512 25.3 -> 19.7.  0 when no height fits one
+// iteration, strips of 16 rows against the choice: 96 x 128 25.1 -> 12.7,
+// 256 x 256 25.3 -> 14.9, 512 x 512 24.3 -> 18.9.  0 when no height fits one
 // wave.
 int one_wave_strip(int rows, int tiles_w, long long sms, int ctas_per_sm, int warps, int least) {
     const long long tw = tiles_w > 0 ? tiles_w : 1, nw = warps;
