@@ -7,18 +7,20 @@
 
 namespace sw2d {
 
-// The forms of a build: uniform rain as the build unrolls it, the others with the
-// row loop not unrolled: unrolled by 2, build 0 with both the storm and the
-// sources spilled 492 bytes, which in strips of more than a few rows cost more
-// than the pipelining saves; not unrolled it spills 28, with the sources alone 16
-// and with the storm alone 52.  us per iteration, 701 x 1237 / 1500 x 1500: storm
-// 55.5 / 115 -> 25.7 / 50.1, sources 54.7 / 108 -> 26.5 / 50.8, both 59.9 / 120 ->
-// 27.2 / 55.0, storm and rain factors 61.7 / 134 -> 28.0 / 56.4.
+// The forms of a build: uniform rain and the storm as the build unrolls them, those
+// with the sources with the row loop not unrolled: unrolled by 2, build 0 with both
+// the storm and the sources spilled 492 bytes (412 with the sources alone), which in
+// strips of more than a few rows cost more than the pipelining saves; not unrolled
+// it spills 28 (16).  The storm alone spills 24 unrolled, 52 not (24.6 against 25.7
+// us at 701 x 1237).  us per iteration, one form for all of them unrolled by 2
+// against these, 701 x 1237 / 1500 x 1500: storm 55.5 / 115 -> 24.6 / 50.0, sources
+// 54.7 / 108 -> 26.6 / 51.0, both 59.9 / 120 -> 27.4 / 55.5, storm and rain factors
+// 61.7 / 134 -> 28.2 / 56.6.
 cudaError_t prepare_stream_pipe(int variant) {
 #define SW2D_P(id, nw, mb, un)                                                                         \
     if (variant == id) {                                                                               \
         const void *k[6] = {(const void *)stream_pipe_kernel<nw, mb, un, false, kFormUniform>,         \
-                            (const void *)stream_pipe_kernel<nw, mb, 1, false, kFormStorm>,            \
+                            (const void *)stream_pipe_kernel<nw, mb, un, false, kFormStorm>,           \
                             (const void *)stream_pipe_kernel<nw, mb, 1, false, kFormSources>,          \
                             (const void *)stream_pipe_kernel<nw, mb, 1, false, kFormAny>,              \
                             (const void *)stream_pipe_kernel<nw, mb, un, true, kFormUniform>,          \
@@ -84,15 +86,15 @@ cudaError_t launch_stream_pipe(int variant, int nblocks, int tiles_w, int strip_
     if (variant == kTmaVariant) variant = 0;
 #define SW2D_PK(nw, mb, un, w, form) \
     return cudaLaunchKernelEx(&lc, stream_pipe_kernel<nw, mb, un, w, form>, G, F, S, T, clk, ctl, slot, sh, P)
-#define SW2D_PL(id, nw, mb, un)                                     \
-    if (variant == id) {                                            \
-        lc.blockDim = dim3(nw * 32);                                \
+#define SW2D_PL(id, nw, mb, un)                                            \
+    if (variant == id) {                                                   \
+        lc.blockDim = dim3(nw * 32);                                       \
         if (S.rainw && (storm || src)) SW2D_PK(nw, mb, 1, true, kFormAny); \
-        if (S.rainw) SW2D_PK(nw, mb, un, true, kFormUniform);       \
-        if (storm && src) SW2D_PK(nw, mb, 1, false, kFormAny);      \
-        if (storm) SW2D_PK(nw, mb, 1, false, kFormStorm);           \
-        if (src) SW2D_PK(nw, mb, 1, false, kFormSources);           \
-        SW2D_PK(nw, mb, un, false, kFormUniform);                   \
+        if (S.rainw) SW2D_PK(nw, mb, un, true, kFormUniform);              \
+        if (storm && src) SW2D_PK(nw, mb, 1, false, kFormAny);             \
+        if (storm) SW2D_PK(nw, mb, un, false, kFormStorm);                 \
+        if (src) SW2D_PK(nw, mb, 1, false, kFormSources);                  \
+        SW2D_PK(nw, mb, un, false, kFormUniform);                          \
     }
     SW2D_STREAM_VARIANTS(SW2D_PL)
 #undef SW2D_PL

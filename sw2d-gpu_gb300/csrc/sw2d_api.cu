@@ -172,10 +172,11 @@ cudaError_t launch_one(sw2d_handle *h, int slot) {
 
 // Whether advance runs several iterations per launch now.  The library's own
 // choice of it (not one the caller asked for) stands down while a moving storm
-// is set: a storm's iterations gain little from it (us per iteration, one launch
-// each against 48 per launch: 128 x 128 18.9 / 17.5, 512 x 512 18.2 / 17.6, 1500 x
-// 1500 49.8 / 50.1).  Point sources stay with it: 21.5 / 19.0, 21.3 / 18.6, 701 x
-// 1237 29.7 / 26.5, 1500 x 1500 55.5 / 50.8; with rain factors too.
+// is set, as documented (sw2d.h); a caller can ask for it there, which gains up
+// to a tenth on small grids and nothing on the largest (us per iteration, one
+// launch each against 48 per launch: 128 x 128 19.0 / 17.0, 512 x 512 18.4 / 17.5,
+// 1500 x 1500 50.1 / 50.0).  Point sources stay with it: 21.5 / 19.0, 21.4 / 18.6,
+// 1500 x 1500 55.7 / 51.0; with rain factors too.
 bool pipe_now(const sw2d_handle *h) {
     return h->pipe_k > 0 && !(h->pipe_auto && h->F.rain_kind == RAIN_STORM);
 }
