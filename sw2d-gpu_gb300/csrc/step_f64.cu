@@ -110,7 +110,8 @@ cudaError_t launch_step64(int th, int tw, int nblocks, int sms, const GridDesc &
     // 91 against 72 us).
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = nblocks <= sms ? 1 : 0;
+    X.overlapped = nblocks <= sms;
+    attr[0].val.programmaticStreamSerializationAllowed = X.overlapped ? 1 : 0;
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3(nblocks);
     lc.stream = st;

@@ -15,10 +15,13 @@
 //     g n^2 of a face once per handle (the planes gnx, gny);
 //   * halves and quarters ride on exact powers of two folded into dt2/dx,
 //     dt2/dy and dt2 (the scaled product rounds as the unscaled one);
-//   * divisions and roots are the short correctly rounded forms of
-//     sw2d_f64math.cuh, divisions by dx and dy multiply by the rounded
-//     reciprocal and correct, the friction power leaves its exact steps to
-//     integer instructions and tables;
+//   * divisions, roots and the friction power's polynomials run in integer
+//     arithmetic (sw2d_f64math.cuh: a 53-bit result and its exact remainder),
+//     divisions by dx and dy multiply by the rounded reciprocal and correct;
+//   * what a face needs differs from face to face, and an FP64 instruction
+//     holds the pipe 64 cycles for 1 lane as for 32: faces and fluxes are
+//     sorted into lists first, and a cell's final depth is its provisional one
+//     where nothing changed it;
 //   * threshold and sign tests, clamps and maxima are integer comparisons of
 //     the bits;
 //   * the CFL bound is a maximum: an FP32 estimate of every face's wave speed
@@ -99,6 +102,7 @@ struct Step64Extra {
     double gn;          // g n^2 of the scalar n
     KnownDivisor dx, dy;
     float thf;          // T.ge_th in FP32
+    bool overlapped;    // launched as a programmatic dependent
 };
 
 constexpr int kStep64Arrays = 13;
@@ -188,10 +192,13 @@ __global__ void __launch_bounds__(NT, MINB)
     const int I0 = ti * TH - HN, J0 = tj * TW - HN;  // global index of smem (0,0)
 
     // ---- stage 0: stage the tile + halo in shared memory --------------------
-    // Launched as a programmatic dependent of the previous iteration: the
-    // static fields are read while that one drains, then its completion (and
-    // the visibility of its writes) is waited for
-    for (int idx = tid; idx < RN; idx += NT) {
+    // Launched as a programmatic dependent of the previous iteration (X.overlapped:
+    // at most one CTA per SM), the static fields are read while that one drains,
+    // then its completion (and the visibility of its writes) is waited for.
+    // Otherwise they are read with the state, after the plan: the launches of a
+    // replay past the end time then load nothing (an advance of one iteration and
+    // 47 such: 4.52 -> 3.84 ms at 2048 x 2048, 1.25 -> 1.05 at 1024 x 1024).
+    auto stage_static = [&](int idx) {
         const int r = idx / RW, c = idx - (idx / RW) * RW;
         const int gi = I0 + r, gj = J0 + c;
         const bool in = (unsigned)gi < (unsigned)rows && (unsigned)gj < (unsigned)cols;
@@ -199,7 +206,9 @@ __global__ void __launch_bounds__(NT, MINB)
         s_z[idx] = in ? S.z[gp] : 0.0;
         s_m[idx] = in ? S.mask[gp] : (uint8_t)0;
         s_tx[idx] = s_ty[idx] = 0;
-    }
+    };
+    if (X.overlapped)
+        for (int idx = tid; idx < RN; idx += NT) stage_static(idx);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const Clock &ci = clk[slot];
@@ -230,6 +239,7 @@ __global__ void __launch_bounds__(NT, MINB)
         const bool in_r = (unsigned)gi < (unsigned)rows, in_c = (unsigned)gj < (unsigned)cols;
         const size_t gp = (size_t)gi * pitch + gj;
         const double h = in_r && in_c ? Hin[gp] : 0.0;
+        if (!X.overlapped) stage_static(idx);
         s_h[idx] = h;
         s_eta[idx] = h + s_z[idx];  // this thread's own s_z
         s_umo[idx] = ((unsigned)gi <= (unsigned)rows && in_c) ? Uin[gp] : 0.0;
