@@ -42,7 +42,9 @@ cudaError_t init_det_tables() {
 // 1.4): 16x32 / 14x32 300 x 500 63.0 / 83.9, 400 x 400 79.2 / 82.5, 1013 x 900
 // 312 / 334.  With one CTA per SM more threads shorten the stages: 8 x 16 23.2
 // with 512 against 26.9 with 256, 8 x 32 30.6 with 768 against 34.2 with 384,
-// 10 x 32 33.1 with 768 against 34.8 with 512.
+// 10 x 32 33.1 with 768 against 34.8 with 512; 14 x 32 and 16 x 32 are the
+// exception (41.7 with 768 against 40.6 on 256 x 256, 43.5 against 42.3 on 230 x
+// 300: the next launch's CTAs, which start early, then no longer fit beside them).
 #define SW2D_STEP64_TILES(X)                                                                        \
     X(16, 32, 512, 2) X(14, 32, 512, 2) X(12, 32, 768, 1) X(10, 32, 768, 1) X(8, 32, 768, 1)        \
     X(6, 32, 512, 1) X(8, 16, 512, 1) X(4, 16, 256, 1) X(4, 8, 256, 1)
