@@ -125,9 +125,10 @@ SW2D_HD double d_half(double x) {
     return d_is_zero(x) ? x : 0.5 * x;
 }
 
-// Exponent field in [200, 1800): far from over- and underflow of anything the
-// fast forms below compute.
-SW2D_HD bool d_mid(double x) { return (d_hi(x) & 0x7ff00000u) - (200u << 20) < (1600u << 20); }
+// Exponent field in [524, 1524), 2^-499 to 2^500: the quotient of any two such
+// values has an exponent of at most 999 either way, far from over- and underflow,
+// as has a root.
+SW2D_HD bool d_mid(double x) { return (d_hi(x) & 0x7ff00000u) - (524u << 20) < (1000u << 20); }
 
 #ifdef __CUDACC__
 static __host__ __device__ __noinline__ double d_div_plain(double a, double b) { return a / b; }
