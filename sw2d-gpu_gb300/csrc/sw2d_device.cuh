@@ -433,6 +433,10 @@ __device__ __forceinline__ void accumulate_cmax(Clock &co, int bucket, double cm
     if (cmax > 0.0) atomicMax(&co.cmaxb[bucket], (unsigned long long)__double_as_longlong(cmax));
     if (bad) atomicOr(&co.nonfinite, 1u);
 }
+// A rate that n cells take.  None of them: nothing, also where the reference's
+// series formula has divided by zero (a record's own time) and the rate is infinite.
+__device__ __forceinline__ double counted_rate(int n, double rate) { return n ? (double)n * rate : 0.0; }
+
 __device__ __forceinline__ void accumulate_budgets(Clock &co, int bucket, const double v[B_N]) {
     for (int k = 0; k < B_N; k++)
         if (v[k] != 0.0) atomicAdd(&co.stepb[k][bucket], v[k]);

@@ -707,13 +707,13 @@ __global__ void __launch_bounds__(NT, MINB)
             c_hi += s_cnt[w][0];
             c_lo += s_cnt[w][1];
         }
-        if (uniform) acc[0] = rp1_hi * (double)c_hi + rp1_lo * (double)c_lo;
+        if (uniform) acc[0] = counted_rate(c_hi, rp1_hi) + counted_rate(c_lo, rp1_lo);
         const double area = G.dx * G.dy;
         const double scale = pl.d.dt2 * area;
         double v[B_N];
         v[B_RAIN] = acc[0] * scale;
         v[B_SRC] = acc[1] * scale;
-        v[B_EV] = LS.ev1 * (double)c_hi * scale;
+        v[B_EV] = counted_rate(c_hi, LS.ev1) * scale;
         v[B_OUT] = acc[2] * pl.d.dt2 * G.dy;
         v[B_CLAMP] = acc[3] * area;
         accumulate_budgets(clk[slot_out], blockIdx.x % kBuckets, v);
