@@ -49,6 +49,16 @@ cudaError_t init_det_tables() {
     X(16, 32, 512, 2) X(14, 32, 512, 2) X(12, 32, 768, 1) X(10, 32, 768, 1) X(8, 32, 768, 1)        \
     X(6, 32, 512, 1) X(8, 16, 512, 1) X(4, 16, 256, 1) X(4, 8, 256, 1)
 
+// The general build, for every grid of a handle that needs it: the largest tile.
+#define SW2D_STEP64_GENERAL step64_kernel<16, 32, 512, 2, true>
+
+bool step64_general(double ge_th, double gt_evmin, double g) {
+    // th = 0 and EV_WL_min < 0 are no positive constants; the FP32 estimates of the
+    // wave speeds hold for depths from 1e-20 m on and an ordinary g (a discharge that
+    // FP32 flushes to zero is then below their margin)
+    return !(ge_th >= 1e-20) || !(gt_evmin > 0.0) || !(g >= 1e-10 && g <= 1e10);
+}
+
 bool step64_tile_supported(int th, int tw) {
 #define SW2D_S64(h, w, nt, mb) \
     if (th == h && tw == w) return true;
@@ -79,18 +89,23 @@ void step64_tile(int rows, int cols, int sms, int *th, int *tw) {
 #undef SW2D_D64
 }
 
-cudaError_t prepare_step64(int th, int tw) {
+namespace {
+
+template <class Kernel>
+cudaError_t prepare_build(Kernel *k, size_t smem) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+}
+
+}  // namespace
+
+cudaError_t prepare_step64(int th, int tw, bool general) {
     const cudaError_t e = init_det_tables();
     if (e != cudaSuccess) return e;
-#define SW2D_P64(h, w, nt, mb)                                                                                  \
-    if (th == h && tw == w) {                                                                                   \
-        const cudaError_t e2 = cudaFuncSetAttribute(step64_kernel<h, w, nt, mb>,                                \
-                                                    cudaFuncAttributeMaxDynamicSharedMemorySize,                \
-                                                    (int)Step64Shape<h, w>::smem(nt / 32));                    \
-        if (e2 != cudaSuccess) return e2;                                                                       \
-        return cudaFuncSetAttribute(step64_kernel<h, w, nt, mb>, cudaFuncAttributePreferredSharedMemoryCarveout, \
-                                    (int)cudaSharedmemCarveoutMaxShared);                                       \
-    }
+    if (general) return prepare_build(SW2D_STEP64_GENERAL, Step64Shape<16, 32>::smem(16));
+#define SW2D_P64(h, w, nt, mb) \
+    if (th == h && tw == w) return prepare_build(step64_kernel<h, w, nt, mb>, Step64Shape<h, w>::smem(nt / 32));
     SW2D_STEP64_TILES(SW2D_P64)
 #undef SW2D_P64
     return cudaErrorInvalidValue;
@@ -119,6 +134,12 @@ cudaError_t launch_step64(int th, int tw, int nblocks, int sms, const GridDesc &
     lc.stream = st;
     lc.attrs = attr;
     lc.numAttrs = 1;
+    if (step64_general(T.ge_th, T.gt_evmin, G.sd.g)) {
+        if (th != 16 || tw != 32) return cudaErrorInvalidValue;
+        lc.blockDim = dim3(512);
+        lc.dynamicSmemBytes = Step64Shape<16, 32>::smem(16);
+        return cudaLaunchKernelEx(&lc, SW2D_STEP64_GENERAL, G, F, S, T, X, clk, ctl, slot);
+    }
 #define SW2D_L64(h, w, nt, mb)                                                                             \
     if (th == h && tw == w) {                                                                              \
         lc.blockDim = dim3(nt);                                                                            \

@@ -209,9 +209,20 @@ void grid_shape(const sw2d_config *c, int *pitch, size_t *plane) {
     *plane = plane_for(c->rows, *pitch);
 }
 
+// Whether an FP64 handle's thresholds need the step kernel's general build.
+bool needs_general(const sw2d_config &c) {
+    const Thr<double> t = make_thr<double>(c);
+    return c.precision == SW2D_PREC_F64 && step64_general(t.ge_th, t.gt_evmin, c.g);
+}
+
 // The tile of the FP64 and FP32 tile kernels: the caller's where there is a
 // build of it, the library's otherwise.
 void pick_tile(const sw2d_config *c, int sms, int *th, int *tw) {
+    if (needs_general(*c)) {
+        *th = 16;
+        *tw = 32;
+        return;
+    }
     *th = c->tile_h;
     *tw = c->tile_w;
     if (*th > 0 && *tw > 0 && tile_supported(c->precision, *th, *tw)) return;
@@ -478,7 +489,7 @@ int sw2d_create(const sw2d_config *cfg, sw2d_handle **out) {
     if (h->stream_kernel) {
         e = prepare_stream_step(h->variant);
     } else {
-        e = is_f64(h) ? prepare_step64(h->tile_h, h->tile_w) : prepare_step(h->tile_h, h->tile_w);
+        e = is_f64(h) ? prepare_step64(h->tile_h, h->tile_w, needs_general(*cfg)) : prepare_step(h->tile_h, h->tile_w);
     }
     if (e != cudaSuccess) return bail(SW2D_ERR_CUDA);
 

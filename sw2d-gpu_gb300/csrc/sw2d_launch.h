@@ -36,8 +36,9 @@ cudaError_t launch_step(int th, int tw, int nblocks, const GridDesc &G, const Fo
                         cudaStream_t st);
 
 // FP64 step kernel (step_f64.cu); sms: the device's SM count; gnx, gny: g n^2 per face (launch_pack_gn), or nullptr with a scalar n
-cudaError_t prepare_step64(int th, int tw);
+cudaError_t prepare_step64(int th, int tw, bool general);
 bool step64_tile_supported(int th, int tw);
+bool step64_general(double ge_th, double gt_evmin, double g);  // these need the general build, which has 16 x 32 tiles
 void step64_tile(int rows, int cols, int sms, int *th, int *tw);  // the library's tile for a grid
 cudaError_t launch_step64(int th, int tw, int nblocks, int sms, const GridDesc &G, const ForcingDesc &F,
                           const StateBufs<double> &S, const Thr<double> &T, const double *gnx, const double *gny,

@@ -142,7 +142,9 @@ __device__ __forceinline__ void append_back(uint16_t *end, int *count, bool keep
     if (keep) *(end - (base + __popc(bal & ((1u << lane) - 1u)))) = (uint16_t)item;
 }
 
-template <int TH, int TW, int NT, int MINB>
+// GENERAL: for thresholds that the bit comparisons and the FP32 estimates do not
+// cover (step64_general).
+template <int TH, int TW, int NT, int MINB, bool GENERAL = false>
 __global__ void __launch_bounds__(NT, MINB)
     step64_kernel(const GridDesc G, const ForcingDesc F, const StateBufs<double> S, const Thr<double> T,
                   const Step64Extra X, Clock *__restrict__ clk, const Control *__restrict__ ctl, const int slot) {
@@ -231,7 +233,10 @@ __global__ void __launch_bounds__(NT, MINB)
     const double dt2 = LS.dt2;
     const double dx = G.sd.dx, dy = G.sd.dy, g = G.sd.g;
     const unsigned long long gt_th = d_bits(T.gt_th), ge_th = d_bits(T.ge_th);
-    const unsigned long long gt_ev = d_bits(T.gt_evmin > 0.0 ? T.gt_evmin : 0.0);
+    const unsigned long long gt_ev = d_bits(T.gt_evmin);
+    // x >= th and x > EV_WL_min: on the bits where the constant is positive
+    auto wet = [&](double x) { return GENERAL ? x >= T.ge_th : d_ge_pos(x, ge_th); };
+    auto above_ev = [&](double x) { return GENERAL ? x >= T.gt_evmin : d_ge_pos(x, gt_ev); };
 
     for (int idx = tid; idx < RN; idx += NT) {
         const int r = idx / RW, c = idx - (idx / RW) * RW;
@@ -314,8 +319,8 @@ __global__ void __launch_bounds__(NT, MINB)
             if (gi == rows) hm = s_h[idx - RW];
             else if (gi == 0) hm = h;
             else hm = d_half(h + s_h[idx - RW]);
-            const double q = s_umo[idx];  // (at rest the division is left out)
-            s_uu[idx] = d_ge_pos(hm, ge_th) && !d_is_zero(q) ? d_div(q, hm) : 0.0;
+            const double q = s_umo[idx];  // (at rest the division is left out; with th = 0 it may be 0 / 0)
+            s_uu[idx] = wet(hm) && (GENERAL || !d_is_zero(q)) ? d_div(q, hm) : 0.0;
         }
         if (c >= 1) {
             double hn;
@@ -323,7 +328,7 @@ __global__ void __launch_bounds__(NT, MINB)
             else if (gj == 0) hn = h;
             else hn = d_half(h + s_h[idx - 1]);
             const double q = s_vno[idx];
-            s_vv[idx] = d_ge_pos(hn, ge_th) && !d_is_zero(q) ? d_div(q, hn) : 0.0;
+            s_vv[idx] = wet(hn) && (GENERAL || !d_is_zero(q)) ? d_div(q, hn) : 0.0;
         }
     }
 
@@ -341,7 +346,7 @@ __global__ void __launch_bounds__(NT, MINB)
         const bool in = k < FN && (unsigned)gi <= (unsigned)rows && (unsigned)gj < (unsigned)cols;
         if (in) {
             const double hb = s_h[p], zb = s_z[p], eb = s_eta[p];
-            const bool b_act = s_m[p] != 0, b_wet = d_ge_pos(hb, gt_th), b_ge = d_ge_pos(hb, ge_th);
+            const bool b_act = s_m[p] != 0, b_wet = d_ge_pos(hb, gt_th), b_ge = wet(hb);
             // cell "a" (north / west) of the face; p is "b"
             auto rule_of = [&](int pa) -> int {
                 const double ha = s_h[pa];
@@ -350,7 +355,7 @@ __global__ void __launch_bounds__(NT, MINB)
                 if (d_lt(eb, s_z[pa])) return a_wet ? 1 : 0;   // cu:130: b's surface below a's bed
                 if (d_lt(s_eta[pa], zb)) return b_wet ? 2 : 0;  // cu:138
                 // cu:149: exactly one side strictly wet; false for NaN
-                const bool a_dry = !d_ge_pos(ha, ge_th) && !d_is_nan(ha);
+                const bool a_dry = !wet(ha) && !d_is_nan(ha);
                 const bool b_dry = !b_ge && !d_is_nan(hb);
                 return (b_wet && a_dry) || (b_dry && a_wet) ? 3 : 4;
             };
@@ -411,7 +416,8 @@ __global__ void __launch_bounds__(NT, MINB)
             need[1] = y || s_ty[e - RW];
             need[2] = x || s_tx[e - 1];
             need[3] = y || s_ty[e - 1];
-            const bool u0 = d_is_zero(s_umo[e]), v0 = d_is_zero(s_vno[e]);
+            // (with th = 0 a velocity may be 0 / 0 where there is no discharge)
+            const bool u0 = !GENERAL && d_is_zero(s_umo[e]), v0 = !GENERAL && d_is_zero(s_vno[e]);
             if (need[0] && u0 && d_is_zero(s_umo[e - RW])) s_fx[e - RW] = 0.0, need[0] = false;
             if (need[1] && v0 && d_is_zero(s_vno[e - RW])) s_cv[e] = 0.0, need[1] = false;
             if (need[2] && u0 && d_is_zero(s_umo[e - 1])) s_cu[e] = 0.0, need[2] = false;
@@ -525,7 +531,7 @@ __global__ void __launch_bounds__(NT, MINB)
         bool dry = false;
         if (s_m[p]) {
             const double ho = s_h[p];
-            const bool hi = d_ge_pos(ho, gt_ev);
+            const bool hi = above_ev(ho);
             double ql = 0.0;
             for (int q = 0; q < nloc; q++)
                 if (s_srcp[q] == p) ql = s_srcq0[q];
@@ -536,7 +542,7 @@ __global__ void __launch_bounds__(NT, MINB)
                 rp = rr * (hi ? pct_hi : pct_lo);
             }
             hraw = balance(ho, s_rum[p], s_rum[p + RW], s_rvn[p], s_rvn[p + 1], ql, rp, hi ? LS.ev0 : 0.0, any_ev0);
-            dry = !d_ge_pos(d_clamp0(hraw), ge_th);  // cu:657
+            dry = !wet(d_clamp0(hraw));  // cu:657
         }
         s_hs[p] = hraw;
         s_dry[p] = dry;
@@ -574,7 +580,7 @@ __global__ void __launch_bounds__(NT, MINB)
         double ql = 0.0, rp = 0.0;
         if (act) {
             const double ho = s_h[p];
-            hi = d_ge_pos(ho, gt_ev);
+            hi = above_ev(ho);
             for (int q = 0; q < nloc; q++)
                 if (s_srcp[q] == p) ql = s_srcq1[q];
             rp = hi ? rp1_hi : rp1_lo;
@@ -620,7 +626,8 @@ __global__ void __launch_bounds__(NT, MINB)
     // is formed for every owned face between active cells (and the open south
     // faces).  The CTA's largest estimate among the faces certainly deeper than
     // th, less that margin, is a bar below the exact maximum: only faces whose
-    // estimate reaches it are evaluated in FP64.
+    // estimate reaches it are evaluated in FP64.  GENERAL evaluates every
+    // face.
     const float gf = G.sf.g, thf = X.thf;
     auto faces = [&](auto &&visit) {
         for (int k = tid; k < TH * TW; k += NT) {
@@ -639,12 +646,13 @@ __global__ void __launch_bounds__(NT, MINB)
     };
     constexpr float kMargin = 1.f / 131072.f;
     float sure = 0.f, est = 0.f;  // over faces certainly / possibly deeper than th
-    faces([&](double q, int p0, int p1) {
-        float hm;
-        const float e = estimate(q, p0, p1, hm);
-        if (hm >= thf * (1.f + kMargin)) sure = fmaxf(sure, e);
-        if (hm >= thf * (1.f - kMargin)) est = fmaxf(est, e);
-    });
+    if (!GENERAL)
+        faces([&](double q, int p0, int p1) {
+            float hm;
+            const float e = estimate(q, p0, p1, hm);
+            if (hm >= thf * (1.f + kMargin)) sure = fmaxf(sure, e);
+            if (hm >= thf * (1.f - kMargin)) est = fmaxf(est, e);
+        });
     const unsigned wmax = __reduce_max_sync(0xffffffffu, __float_as_uint(sure));
     if (lane == 0 && wmax) atomicMax(&s_est, wmax);
     const bool any_bad = __syncthreads_or(bad);
@@ -654,16 +662,17 @@ __global__ void __launch_bounds__(NT, MINB)
         // depth) is not evaluated again
         unsigned long long cm = 0ull, seen_q = 1ull, seen_0 = 0ull, seen_1 = 0ull;
         faces([&](double q, int p0, int p1) {
-            float hf;
-            const float e = estimate(q, p0, p1, hf);
-            if (!(e >= bar) || !(hf >= thf * (1.f - kMargin))) return;
+            if (!GENERAL) {
+                float hf;
+                if (!(estimate(q, p0, p1, hf) >= bar) || !(hf >= thf * (1.f - kMargin))) return;
+            }
             const double h0 = s_h[p0], h1 = s_h[p1];
             if ((d_bits(q) << 1) == seen_q && d_bits(h0) == seen_0 && d_bits(h1) == seen_1) return;
             seen_q = d_bits(q) << 1;
             seen_0 = d_bits(h0);
             seen_1 = d_bits(h1);
             const double hm = 0.50 * (h0 + h1);
-            if (!d_ge_pos(hm, ge_th)) return;
+            if (!wet(hm)) return;
             const double v = (d_is_zero(q) ? 0.0 : fabs(d_div(q, hm))) + d_sqrt(g * hm);
             if (!d_is_nan(v)) cm = d_bits(v) > cm ? d_bits(v) : cm;
         });
