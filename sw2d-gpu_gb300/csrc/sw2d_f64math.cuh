@@ -280,11 +280,12 @@ SW2D_HD double d_sqrt(double x) {
 
 // ---- double to float, for estimates only ---------------------------------------
 
-// |x| truncated to FP32 (0 below the normal range, inf above it, NaN stays NaN)
+// |x| truncated to FP32 (0 below the normal range, inf from 2^123 on, below the
+// divisors that __fdividef gives up on; NaN stays NaN)
 SW2D_HD float d_abs_float(double x) {
     const unsigned hi = d_hi(x) & 0x7fffffffu;
     const unsigned v = ((hi - 0x38000000u) << 3) | (d_lo(x) >> 29);
-    if (hi - 0x38100000u < 0x0fe00000u - 0x00100000u) return f_from_bits(v);
+    if (hi - 0x38100000u < 0x47a00000u - 0x38100000u) return f_from_bits(v);
     return hi < 0x38100000u ? 0.f : (hi >= 0x7ff00000u && d_is_nan(x) ? f_from_bits(0x7fc00000u) : f_from_bits(0x7f800000u));
 }
 

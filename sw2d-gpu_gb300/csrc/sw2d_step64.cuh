@@ -626,8 +626,9 @@ __global__ void __launch_bounds__(NT, MINB)
     // is formed for every owned face between active cells (and the open south
     // faces).  The CTA's largest estimate among the faces certainly deeper than
     // th, less that margin, is a bar below the exact maximum: only faces whose
-    // estimate reaches it are evaluated in FP64.  GENERAL evaluates every
-    // face.
+    // estimate reaches it are evaluated in FP64.  Estimates are compared as bits, so
+    // that one beyond FP32 (infinite or 0 x infinity, in a run that grows without
+    // bound) is the largest; it makes no bar.  GENERAL evaluates every face.
     const float gf = G.sf.g, thf = X.thf;
     auto faces = [&](auto &&visit) {
         for (int k = tid; k < TH * TW; k += NT) {
@@ -640,23 +641,24 @@ __global__ void __launch_bounds__(NT, MINB)
             if (gj > 0 && s_m[p - 1]) visit(s_vno[p], p, p - 1);
         }
     };
-    auto estimate = [&](double q, int p0, int p1, float &hm) -> float {
+    auto estimate = [&](double q, int p0, int p1, float &hm) -> unsigned {
         hm = 0.5f * (s_hf[p0] + s_hf[p1]);
-        return __fdividef(d_abs_float(q), hm) + __fsqrt_rn(gf * hm);
+        return __float_as_uint(__fdividef(d_abs_float(q), hm) + __fsqrt_rn(gf * hm));
     };
     constexpr float kMargin = 1.f / 131072.f;
-    float sure = 0.f, est = 0.f;  // over faces certainly / possibly deeper than th
+    constexpr unsigned kInfinite = 0x7f800000u;
+    unsigned sure = 0u, est = 0u;  // over faces certainly / possibly deeper than th
     if (!GENERAL)
         faces([&](double q, int p0, int p1) {
             float hm;
-            const float e = estimate(q, p0, p1, hm);
-            if (hm >= thf * (1.f + kMargin)) sure = fmaxf(sure, e);
-            if (hm >= thf * (1.f - kMargin)) est = fmaxf(est, e);
+            const unsigned e = estimate(q, p0, p1, hm);
+            if (hm >= thf * (1.f + kMargin)) sure = max(sure, e);
+            if (hm >= thf * (1.f - kMargin)) est = max(est, e);
         });
-    const unsigned wmax = __reduce_max_sync(0xffffffffu, __float_as_uint(sure));
+    const unsigned wmax = __reduce_max_sync(0xffffffffu, sure);
     if (lane == 0 && wmax) atomicMax(&s_est, wmax);
     const bool any_bad = __syncthreads_or(bad);
-    const float bar = __uint_as_float(s_est) * (1.f - kMargin);
+    const unsigned bar = s_est < kInfinite ? __float_as_uint(__uint_as_float(s_est) * (1.f - kMargin)) : 0u;
     if (est >= bar) {
         // a face with the values of the thread's last one (still water of one
         // depth) is not evaluated again
@@ -664,7 +666,7 @@ __global__ void __launch_bounds__(NT, MINB)
         faces([&](double q, int p0, int p1) {
             if (!GENERAL) {
                 float hf;
-                if (!(estimate(q, p0, p1, hf) >= bar) || !(hf >= thf * (1.f - kMargin))) return;
+                if (estimate(q, p0, p1, hf) < bar || !(hf >= thf * (1.f - kMargin))) return;
             }
             const double h0 = s_h[p0], h1 = s_h[p1];
             if ((d_bits(q) << 1) == seen_q && d_bits(h0) == seen_0 && d_bits(h1) == seen_1) return;

@@ -1,6 +1,7 @@
 """The FP64 kernel at the ends of what sw2d_create takes: no wet/dry threshold
-(th = 0) or a tiny one, a negative EV_WL_min, negative depths.  The state, the
-time steps and what is refused are the oracle's."""
+(th = 0) or a tiny one, a negative EV_WL_min, depths that are negative or
+beyond single precision.  The state, the time steps and what is refused are the
+oracle's."""
 import numpy as np
 import pytest
 
@@ -74,3 +75,20 @@ def test_negative_depths_and_evaporation_level(oracle_mod, sw2d_mod, evmin):
     for k in ("rain_in", "evap_out"):
         assert bg[k] == pytest.approx(bo[k], rel=1e-12, abs=1e-14), k
     g.close()
+
+
+@pytest.mark.parametrize("top", [1e30, 1e37, 1e38, 1e40, 1e80])
+def test_wave_speed_beyond_single_precision(oracle_mod, sw2d_mod, top):
+    """Deep and fast faces on which FP32 overflows beside ones on which it does
+    not: the CFL bound is the FP64 maximum."""
+    rng = np.random.default_rng(5)
+    shape = (20, 37)
+    for um_scale in (0.0, 1.0, 1e8, 1e30):
+        z = np.zeros(shape)
+        h = 10.0 ** rng.uniform(np.log10(top) - 3.0, np.log10(top), shape)
+        h[rng.random(shape) < 0.5] = 1.0
+        um = um_scale * rng.uniform(-1.0, 1.0, (shape[0] + 1, shape[1]))
+        o, g = _pair(oracle_mod, sw2d_mod, z, h, um=um, dt_mode=1, dt=1e-30, cfl=0.5)
+        assert o.advance(2) == g.advance(2) == 2
+        _equal(o, g)
+        g.close()
