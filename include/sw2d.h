@@ -133,10 +133,14 @@ typedef struct sw2d_handle sw2d_handle;
  * fixed dt).  Replaces the constants of cu:808-809 and cu:1130. */
 int sw2d_config_init(sw2d_config *cfg);
 
-/* Device bytes a handle with this config allocates (admission control). */
+/* Device bytes a handle with this config allocates (admission control),
+ * with a Manning raster: an FP64 handle without one holds 16 bytes per cell
+ * less (sw2d_set_static allocates them with the first raster). */
 int sw2d_device_bytes(const sw2d_config *cfg, int64_t *bytes);
 
-/* Creates a handle and allocates all device memory.
+/* Creates a handle and allocates its device memory; the per-cell fields that
+ * only some runs have (rain factors, an FP64 handle's roughness) are allocated
+ * when they are first set.
  * Replaces the cudaMalloc block cu:1163-1190 and the launch setup cu:1222-1235. */
 int sw2d_create(const sw2d_config *cfg, sw2d_handle **out);
 

@@ -50,7 +50,7 @@ struct sw2d_handle {
     cudaStream_t stream = nullptr;
     void *h[2] = {nullptr, nullptr}, *um[2] = {nullptr, nullptr}, *vn[2] = {nullptr, nullptr};
     void *z = nullptr, *nman = nullptr;  // nman: FP32 only
-    double *gnx = nullptr, *gny = nullptr;  // g n^2 per face (FP64 only; one allocation, gnx first)
+    double *gnx = nullptr, *gny = nullptr;  // g n^2 per face (FP64 only; one allocation at the first raster, gnx first)
     uint8_t *mask = nullptr;
     void *rainw = nullptr;  // spatial rain factors (allocated on first use)
     void *dzx = nullptr, *dzy = nullptr;  // bed differences across faces (streaming kernel)
@@ -417,7 +417,7 @@ int sw2d_device_bytes(const sw2d_config *c, int64_t *bytes) {
     const size_t rs = c->precision == SW2D_PREC_F64 ? 8 : 4;
     const bool stream = c->precision == SW2D_PREC_F32 && c->kernel != SW2D_KERNEL_TILE;
     // 2x(h, um, vn) + z, frame included, and: n (FP32), dzx, dzy, 2x remainder (streaming kernel), g n^2 of the
-    // two faces (FP64)
+    // two faces (FP64 with a raster)
     size_t total = plane * rs * (stream ? 12 : (rs == 8 ? 9 : 8));
     total += plane;                 // mask
     total += 2 * (size_t)(c->rows + 1) * (c->cols + 1) * sizeof(double);  // staging
@@ -462,14 +462,7 @@ int sw2d_create(const sw2d_config *cfg, sw2d_handle **out) {
             if (!alloc_field(a, h->real_size)) return bail(SW2D_ERR_OOM);
     }
     if (!alloc_field(&h->z, h->real_size) || !alloc_field((void **)&h->mask, 1)) return bail(SW2D_ERR_OOM);
-    if (is_f64(h)) {
-        void *p = nullptr;  // one allocation for both planes, filled by set_static before anything reads it
-        if (cudaMalloc(&p, 2 * h->plane * sizeof(double)) != cudaSuccess) return bail(SW2D_ERR_OOM);
-        h->gnx = static_cast<double *>(p) + h->origin;
-        h->gny = h->gnx + h->plane;
-    } else if (!alloc_field(&h->nman, h->real_size)) {
-        return bail(SW2D_ERR_OOM);
-    }
+    if (!is_f64(h) && !alloc_field(&h->nman, h->real_size)) return bail(SW2D_ERR_OOM);
     (void)fb;
     h->stage_elems = (size_t)(cfg->rows + 1) * (cfg->cols + 1);
     if (cudaMalloc((void **)&h->stage, h->stage_elems * sizeof(double)) != cudaSuccess) return bail(SW2D_ERR_OOM);
@@ -618,6 +611,13 @@ int sw2d_set_static(sw2d_handle *h, const double *z, const double *manning) {
     if (!h || !z) return fail(h, SW2D_ERR_INVALID_ARG, "z is null");
     const int rows = h->cfg.rows, cols = h->cfg.cols;
     const size_t n = (size_t)rows * cols;
+    if (is_f64(h) && manning && !h->gnx) {  // every face that is read is written below
+        void *p = nullptr;
+        CK(h, cudaSetDevice(h->cfg.device));
+        CK(h, cudaMalloc(&p, 2 * h->plane * sizeof(double)));
+        h->gnx = static_cast<double *>(p) + h->origin;
+        h->gny = h->gnx + h->plane;
+    }
     CK(h, cudaMemcpyAsync(h->stage, z, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     double *dn = nullptr;
     if (manning) {
