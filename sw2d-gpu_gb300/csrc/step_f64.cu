@@ -151,9 +151,10 @@ cudaError_t launch_step64(int th, int tw, int nblocks, int sms, const GridDesc &
     return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_pack_gn(const double *n, int rows, int cols, int pitch, double g, double *gnx, double *gny,
-                           cudaStream_t st) {
-    pack_gn_kernel<<<detail::grid_for((long long)rows * cols, 256), 256, 0, st>>>(n, rows, cols, pitch, g, gnx, gny);
+cudaError_t launch_pack_static_gn(const double *z, const double *n, int rows, int cols, int pitch, double nodata,
+                                  double g, double *zout, uint8_t *mask, double *gnx, double *gny, cudaStream_t st) {
+    const dim3 block(32, 8), grid((cols + 31) / 32, (unsigned)((rows + 7) / 8 < 65535 ? (rows + 7) / 8 : 65535));
+    pack_static_gn_kernel<<<grid, block, 0, st>>>(z, n, rows, cols, pitch, nodata, g, zout, mask, gnx, gny);
     return cudaGetLastError();
 }
 

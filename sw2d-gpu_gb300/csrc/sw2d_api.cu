@@ -624,11 +624,13 @@ int sw2d_set_static(sw2d_handle *h, const double *z, const double *manning) {
         CK(h, cudaMemcpyAsync(h->stage2, manning, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
         dn = h->stage2;
     }
-    if (is_f64(h)) {
-        CK(h, launch_pack_static(h->stage, dn, rows, cols, h->pitch, h->cfg.nodata, (double *)h->z, (double *)nullptr,
-                                 h->mask, h->stream));
-        if (dn) CK(h, launch_pack_gn(dn, rows, cols, h->pitch, h->cfg.g, h->gnx, h->gny, h->stream));
-    } else
+    if (is_f64(h) && dn)
+        CK(h, launch_pack_static_gn(h->stage, dn, rows, cols, h->pitch, h->cfg.nodata, h->cfg.g, (double *)h->z,
+                                    h->mask, h->gnx, h->gny, h->stream));
+    else if (is_f64(h))
+        CK(h, launch_pack_static(h->stage, nullptr, rows, cols, h->pitch, h->cfg.nodata, (double *)h->z,
+                                 (double *)nullptr, h->mask, h->stream));
+    else
         CK(h, launch_pack_static(h->stage, dn, rows, cols, h->pitch, h->cfg.nodata, (float *)h->z,
                                  dn ? (float *)h->nman : nullptr, h->mask, h->stream));
     if (h->stream_kernel)

@@ -35,7 +35,7 @@ cudaError_t launch_step(int th, int tw, int nblocks, const GridDesc &G, const Fo
                         const StateBufs<float> &S, const Thr<float> &T, Clock *clk, const Control *ctl, int slot,
                         cudaStream_t st);
 
-// FP64 step kernel (step_f64.cu); sms: the device's SM count; gnx, gny: g n^2 per face (launch_pack_gn), or nullptr with a scalar n
+// FP64 step kernel (step_f64.cu); sms: the device's SM count; gnx, gny: g n^2 per face (launch_pack_static_gn), or nullptr with a scalar n
 cudaError_t prepare_step64(int th, int tw, bool general);
 bool step64_tile_supported(int th, int tw);
 bool step64_general(double ge_th, double gt_evmin, double g);  // these need the general build, which has 16 x 32 tiles
@@ -43,8 +43,8 @@ void step64_tile(int rows, int cols, int sms, int *th, int *tw);  // the library
 cudaError_t launch_step64(int th, int tw, int nblocks, int sms, const GridDesc &G, const ForcingDesc &F,
                           const StateBufs<double> &S, const Thr<double> &T, const double *gnx, const double *gny,
                           Clock *clk, const Control *ctl, int slot, cudaStream_t st);
-cudaError_t launch_pack_gn(const double *n, int rows, int cols, int pitch, double g, double *gnx, double *gny,
-                           cudaStream_t st);
+cudaError_t launch_pack_static_gn(const double *z, const double *n, int rows, int cols, int pitch, double nodata,
+                                  double g, double *zout, uint8_t *mask, double *gnx, double *gny, cudaStream_t st);
 
 #define SW2D_DECLARE_LAUNCHERS(Real)                                                                          \
     cudaError_t launch_pack_static(const double *z, const double *n, int rows, int cols, int pitch,         \
