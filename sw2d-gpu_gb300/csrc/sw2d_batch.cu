@@ -36,6 +36,16 @@ constexpr int kBatchVariants = 3;
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// Scenarios of the same rows and strip rule, for choosing the strips.
+struct StripClass {
+    int rows, rule;  // rule: strip height by scenario size, or the caller's
+    bool own;        // the caller's
+    long long tiles; // column tiles of all of them
+    bool operator<(const StripClass &o) const {
+        return rows != o.rows ? rows < o.rows : (rule != o.rule ? rule < o.rule : own < o.own);
+    }
+};
+
 struct HostScenario {
     bool active = false;
     sw2d_config cfg{};
@@ -67,6 +77,12 @@ struct sw2d_batch {
     Clock *h_clk = nullptr;       // pinned
     std::vector<HostScenario> scen;
     std::vector<int2> units;
+    // the resident scenarios: slots in ascending order, and their classes; room for
+    // choosing their strips
+    std::vector<int> resident;
+    std::vector<StripClass> classes;
+    std::vector<std::pair<int, int>> order;
+    std::vector<std::pair<long long, long long>> done;
     long long launches = 0;
     int grid = 0, sms = 152;
     cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};
@@ -153,15 +169,32 @@ int capture(sw2d_batch *b, int parity) {
 
 int units_of(const HostScenario &h, int strip_h) { return h.tiles_w * ((h.cfg.rows + strip_h - 1) / strip_h); }
 
-// Rows of the strips in use when every scenario is cut at `sh` rows (0: the
-// size rule; a caller's height stays): rows of a strip -> number of strips.
-void strip_counts(const sw2d_batch *b, int sh, std::map<int, long long> &count) {
-    count.clear();
-    for (const HostScenario &h : b->scen) {
-        if (!h.active) continue;
-        const int s = h.own_strip || sh == 0 ? h.rule_strip : sh, full = h.cfg.rows / s, rest = h.cfg.rows % s;
-        if (full) count[s] += (long long)h.tiles_w * full;
-        if (rest) count[rest] += h.tiles_w;
+// The common heights that choose_strips tries beside the size rule, and the rows
+// of the strips in use when every scenario is cut at one height (0: the size rule;
+// a caller's height stays).  Strips taller than the tallest common height are the
+// callers' alone.
+constexpr int kHeights[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64, 96};
+constexpr int kTallest = 96;
+struct StripCounts {
+    long long of[kTallest + 1];       // strips of that many rows
+    std::map<int, long long> taller;  // rows -> strips
+    long long strips, steps;          // in all; their row steps, 7 of warm-up included
+};
+
+void strip_counts(const sw2d_batch *b, int sh, StripCounts &c) {
+    std::memset(c.of, 0, sizeof(c.of));
+    c.taller.clear();
+    c.strips = c.steps = 0;
+    auto add = [&](int rows, long long n) {
+        if (rows <= kTallest) c.of[rows] += n;
+        else c.taller[rows] += n;
+        c.strips += n;
+        c.steps += n * (rows + 7);
+    };
+    for (const StripClass &k : b->classes) {
+        const int s = k.own || sh == 0 ? k.rule : sh, full = k.rows / s, rest = k.rows % s;
+        if (full) add(s, k.tiles * full);
+        if (rest) add(rest, k.tiles);
     }
 }
 
@@ -172,31 +205,43 @@ void strip_counts(const sw2d_batch *b, int sh, std::map<int, long long> &count) 
 // build's 128 registers): 0.95 us up to 8 warps per SM, 1.04 at 9, 1.14 from 12
 // on; in the tail of several waves the warps still busy sit unevenly on the SMs,
 // and a row step stays at 1.11-1.14 us with 9 per SM on average.
-double iteration_length(const std::map<int, long long> &count, long long warps, long long sms) {
-    std::map<long long, long long> free_at;  // time -> warps that become free then
-    free_at[0] = warps;
-    long long used = 0;
-    for (auto it = count.rbegin(); it != count.rend(); ++it)
-        for (long long left = it->second; left > 0;) {
-            auto f = free_at.begin();
-            const long long t = f->first, k = f->second < left ? f->second : left;
-            if (k == f->second) free_at.erase(f);
-            else f->second -= k;
-            free_at[t + it->first + 7] += k;
+double iteration_length(const StripCounts &c, long long warps, long long sms,
+                        std::vector<std::pair<long long, long long>> &done) {
+    // (time, warps free from then on), the earliest last; the warps that have had no
+    // strip yet are counted apart
+    done.clear();
+    long long idle = warps;
+    auto take = [&](int rows, long long left) {
+        while (left > 0) {
+            long long t = 0, k = 0;
+            if (idle > 0) {
+                k = idle < left ? idle : left;
+                idle -= k;
+            } else {
+                t = done.back().first;
+                k = done.back().second < left ? done.back().second : left;
+                done.back().second -= k;
+                if (done.back().second == 0) done.pop_back();
+            }
             left -= k;
+            const long long end = t + rows + 7;
+            auto at = std::lower_bound(done.begin(), done.end(), end,
+                                       [](const std::pair<long long, long long> &x, long long y) { return x.first > y; });
+            if (at != done.end() && at->first == end) at->second += k;
+            else done.insert(at, {end, k});
         }
-    for (auto &f : free_at) used += f.first > 0 ? f.second : 0;
-    long long strips = 0;
-    for (auto &c : count) strips += c.second;
-    const bool one_wave = strips <= warps;
+    };
+    for (auto it = c.taller.rbegin(); it != c.taller.rend(); ++it) take(it->first, it->second);
+    for (int rows = kTallest; rows > 0; rows--)
+        if (c.of[rows]) take(rows, c.of[rows]);
+    const bool one_wave = c.strips <= warps;
+    const long long light = (one_wave ? 8 : 4) * sms;
     double len = 0.0;
-    long long t = 0, busy = used;
-    for (auto &f : free_at) {
-        if (f.first == 0) continue;
-        const long long light = (one_wave ? 8 : 4) * sms;
-        len += (double)(f.first - t) * (busy <= light ? 100 : (one_wave && busy <= 10 * sms ? 110 : 120));
-        t = f.first;
-        busy -= f.second;
+    long long t = 0, busy = warps - idle;
+    for (auto f = done.rbegin(); f != done.rend(); ++f) {
+        len += (double)(f->first - t) * (busy <= light ? 100 : (one_wave && busy <= 10 * sms ? 110 : 120));
+        t = f->first;
+        busy -= f->second;
     }
     return len;
 }
@@ -208,60 +253,79 @@ double iteration_length(const std::map<int, long long> &count, long long warps, 
 // size rule against the choice: 8 scenarios of 64 .. 128 cells a side 35.7 ->
 // 20.1, 40 of 64 .. 300 58.5 -> 47, 100 of 128 .. 1024 561 -> 519.  A scenario's
 // state does not depend on the strips, nor, with the counted rain, do its
-// budgets beyond the order of their sums.
-void choose_strips(sw2d_batch *b) {
+// budgets beyond the order of their sums.  The resident scenarios are counted in
+// classes of equal rows (b->classes), and heights that cannot win by their tallest
+// strip or by their work alone are not scheduled.  0: the size rule.
+int choose_strips(sw2d_batch *b) {
     const long long warps = (long long)b->grid * batch_warps(b->cfg.variant);
-    std::map<int, long long> count;
-    int best_sh = 0;
-    double best = 0.0;
-    for (int sh : {0, 1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64, 96}) {
+    StripCounts count;
+    strip_counts(b, 0, count);
+    // a common height has to be clearly better than the rule: the estimate is
+    // good to about 10 % (a mix of heights fills the queue's tail better than
+    // it says: 24 scenarios of 128 .. 1024 run in 160 us under the rule, 170
+    // at 48 rows and 189 at 96, estimated 164, 162 and 161)
+    double best = 0.93 * iteration_length(count, warps, b->sms, b->done);
+    int best_sh = 0, tallest = 0;  // grid to cut at a common height
+    for (const StripClass &k : b->classes)
+        if (!k.own) tallest = std::max(tallest, k.rows);
+    for (int sh : kHeights) {
+        if (100.0 * (std::min(sh, tallest) + 7) >= best) break;  // nor can the ones above
         strip_counts(b, sh, count);
-        long long units = 0, steps = 0;
-        for (auto &c : count) {
-            units += c.second;
-            steps += c.second * (c.first + 7);
-        }
-        if (sh > 0 && (units > b->cfg.max_units || 120.0 * (double)steps >= best * (double)warps)) continue;
-        const double len = iteration_length(count, warps, b->sms);
-        // a common height has to be clearly better than the rule: the estimate is
-        // good to about 10 % (a mix of heights fills the queue's tail better than
-        // it says: 24 scenarios of 128 .. 1024 run in 160 us under the rule, 170
-        // at 48 rows and 189 at 96, estimated 164, 162 and 161)
-        if (sh == 0) best = 0.93 * len;
-        else if (len < best) best = len, best_sh = sh;
+        if (count.strips > b->cfg.max_units || 120.0 * (double)count.steps >= best * (double)warps) continue;
+        const double len = iteration_length(count, warps, b->sms, b->done);
+        if (len < best) best = len, best_sh = sh;
     }
-    for (HostScenario &h : b->scen) {
-        if (!h.active) continue;
-        h.strip_h = h.own_strip || best_sh == 0 ? h.rule_strip : best_sh;
-        h.nunits = units_of(h, h.strip_h);
-    }
+    return best_sh;
 }
 
-// The unit table of the resident scenarios, and the strips in use in their
-// descriptors; in stream order, so between launches.
-int upload_units(sw2d_batch *b) {
+// The class of a scenario gains (or loses) its column tiles.
+void count_scenario(sw2d_batch *b, const HostScenario &h, int sign) {
+    const StripClass k{h.cfg.rows, h.rule_strip, h.own_strip, 0};
+    auto at = std::lower_bound(b->classes.begin(), b->classes.end(), k);
+    if (at == b->classes.end() || k < *at) at = b->classes.insert(at, k);
+    at->tiles += sign * h.tiles_w;
+    if (at->tiles == 0) b->classes.erase(at);
+}
+
+// The strips and the unit table of the resident scenarios (those in b->resident)
+// on the host.  Sending them is send_units.
+int plan_units(sw2d_batch *b) {
     long long rule = 0;
-    for (const HostScenario &h : b->scen)
-        if (h.active) rule += units_of(h, h.rule_strip);
+    for (const StripClass &k : b->classes) rule += k.tiles * ((k.rows + k.rule - 1) / k.rule);
     if (rule > b->cfg.max_units) return bfail(b, SW2D_ERR_INVALID_ARG, "unit table full: raise max_units");
-    // the longest strips first: a launch ends when its last unit does, and a
-    // 64-row strip that the queue hands out last leaves the other warps idle
-    b->units.clear();
     try {  // no exception crosses the C ABI
-        choose_strips(b);
-        std::vector<int> order;
-        for (size_t s = 0; s < b->scen.size(); s++)
-            if (b->scen[s].active) order.push_back((int)s);
-        auto rows_of = [&](int s) { return std::min(b->scen[s].strip_h, b->scen[s].cfg.rows); };
-        std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return rows_of(x) > rows_of(y); });
-        for (int s : order)
-            for (int u = 0; u < b->scen[s].nunits; u++) b->units.push_back(make_int2(s, u));
+        const int common = choose_strips(b);
+        b->order.clear();
+        size_t total = 0;
+        for (int s : b->resident) {
+            HostScenario &h = b->scen[s];
+            h.strip_h = h.own_strip || common == 0 ? h.rule_strip : common;
+            h.nunits = units_of(h, h.strip_h);
+            total += h.nunits;
+            b->order.push_back({-std::min(h.strip_h, h.cfg.rows), s});
+        }
+        // the longest strips first: a launch ends when its last unit does, and a
+        // 64-row strip that the queue hands out last leaves the other warps idle
+        if (!std::is_sorted(b->order.begin(), b->order.end())) std::sort(b->order.begin(), b->order.end());
+        b->units.resize(total);
+        int2 *unit = b->units.data();
+        for (const std::pair<int, int> &o : b->order) {
+            const int n = b->scen[o.second].nunits;
+            for (int u = 0; u < n; u++) unit[u] = make_int2(o.second, u);
+            unit += n;
+        }
     } catch (...) {
         return bfail(b, SW2D_ERR_OOM, "host memory for the unit table");
     }
-    for (size_t s = 0; s < b->scen.size(); s++) {
+    return SW2D_OK;
+}
+
+// Sends the unit table, and the strips that changed to their descriptors; in
+// stream order, so between launches.
+int send_units(sw2d_batch *b) {
+    for (int s : b->resident) {
         HostScenario &h = b->scen[s];
-        if (!h.active || (h.dev.strip_h == h.strip_h && h.dev.nunits == h.nunits)) continue;
+        if (h.dev.strip_h == h.strip_h && h.dev.nunits == h.nunits) continue;
         h.dev.strip_h = h.strip_h;
         h.dev.nunits = h.nunits;
         // strip_h and nunits are neighbours in the descriptor
@@ -273,7 +337,24 @@ int upload_units(sw2d_batch *b) {
                                b->stream));
     const int n = (int)b->units.size();
     BCK(b, cudaMemcpyAsync(&b->d_hdr->n_units, &n, sizeof(int), cudaMemcpyHostToDevice, b->stream));
-    BCK(b, cudaStreamSynchronize(b->stream));  // the host vector and n must outlive the copies
+    BCK(b, cudaStreamSynchronize(b->stream));  // the host vectors and n must outlive the copies
+    return SW2D_OK;
+}
+
+// The lists of resident scenarios with slot s put in or taken out.
+int list_scenario(sw2d_batch *b, int s, bool in) {
+    try {
+        if (in) {
+            count_scenario(b, b->scen[s], 1);
+            b->resident.insert(std::lower_bound(b->resident.begin(), b->resident.end(), s), s);
+        } else {
+            count_scenario(b, b->scen[s], -1);
+            b->resident.erase(std::lower_bound(b->resident.begin(), b->resident.end(), s));
+        }
+    } catch (...) {
+        return bfail(b, SW2D_ERR_OOM, "host memory for the scenario lists");
+    }
+    b->scen[s].active = in;
     return SW2D_OK;
 }
 
@@ -554,27 +635,30 @@ int sw2d_batch_add(sw2d_batch *b, const sw2d_config *cfg, const double *z, const
     if (vrc) return vrc;
     d.status = b->d_status + slot;
     d.tiles_w = h.tiles_w;
+    int rc = list_scenario(b, slot, true);
+    if (!rc && (rc = plan_units(b)) != SW2D_OK) list_scenario(b, slot, false);
     d.strip_h = h.strip_h;
     d.nunits = h.nunits;
-    BCK(b, cudaMemcpyAsync(b->d_scen + slot, &d, sizeof(ScenarioDev), cudaMemcpyHostToDevice, b->stream));
-    // clock: the current launch parity holds this state
-    const int cur = (int)(b->launches % 3);
-    Clock c0;
-    std::memset(&c0, 0, sizeof(c0));
-    *b->h_clk = c0;
-    BCK(b, cudaMemcpyAsync(clk + cur, b->h_clk, sizeof(Clock), cudaMemcpyHostToDevice, b->stream));
-    BCK(b, launch_cmax(d.h[0], d.um[0], d.vn[0], m_dev, cfg->rows, cfg->cols, h.pitch, G.south_open, d.T.ge_th,
-                       cfg->g, &clk[cur].cmax_bits, b->stream));
-    plan_kernel<<<1, 32, 0, b->stream>>>(G, F, clk, &b->d_scen[slot].ctl, cur);
-    BCK(b, cudaGetLastError());
-    ScenarioStatus s0;
-    std::memset(&s0, 0, sizeof(s0));
-    s0.running = 1;
-    BCK(b, cudaMemcpyAsync(b->d_status + slot, &s0, sizeof(s0), cudaMemcpyHostToDevice, b->stream));
-    h.active = true;
-    int rc = upload_units(b);  // synchronises: the host-side sources above are safe to reuse
-    if (rc) {  // the unit table is full: the scenario is not admitted and its memory goes back
-        h.active = false;
+    auto send = [&]() -> int {
+        BCK(b, cudaMemcpyAsync(b->d_scen + slot, &d, sizeof(ScenarioDev), cudaMemcpyHostToDevice, b->stream));
+        // clock: the current launch parity holds this state
+        const int cur = (int)(b->launches % 3);
+        Clock c0;
+        std::memset(&c0, 0, sizeof(c0));
+        *b->h_clk = c0;
+        BCK(b, cudaMemcpyAsync(clk + cur, b->h_clk, sizeof(Clock), cudaMemcpyHostToDevice, b->stream));
+        BCK(b, launch_cmax(d.h[0], d.um[0], d.vn[0], m_dev, cfg->rows, cfg->cols, h.pitch, G.south_open, d.T.ge_th,
+                           cfg->g, &clk[cur].cmax_bits, b->stream));
+        plan_kernel<<<1, 32, 0, b->stream>>>(G, F, clk, &b->d_scen[slot].ctl, cur);
+        BCK(b, cudaGetLastError());
+        ScenarioStatus s0;
+        std::memset(&s0, 0, sizeof(s0));
+        s0.running = 1;
+        BCK(b, cudaMemcpyAsync(b->d_status + slot, &s0, sizeof(s0), cudaMemcpyHostToDevice, b->stream));
+        return send_units(b);  // synchronises: the host-side sources above are safe to reuse
+    };
+    if (!rc && (rc = send()) != SW2D_OK) list_scenario(b, slot, false);
+    if (rc) {  // e.g. the unit table is full: the scenario is not admitted and its memory goes back
         cudaFreeAsync(h.block, b->stream);
         h.block = nullptr;
         b->bytes_in_use -= (int64_t)h.bytes;
@@ -706,8 +790,9 @@ int sw2d_batch_remove(sw2d_batch *b, int32_t id) {
     if (!b || id < 0 || id >= (int)b->scen.size() || !b->scen[id].active)
         return bfail(b, SW2D_ERR_INVALID_ARG, "bad scenario id");
     HostScenario &h = b->scen[id];
-    h.active = false;
-    int rc = upload_units(b);  // the next launch no longer sees the scenario
+    int rc = list_scenario(b, id, false);
+    if (!rc) rc = plan_units(b);
+    if (!rc) rc = send_units(b);  // the next launch no longer sees the scenario
     if (rc) return rc;
     BCK(b, cudaFreeAsync(h.block, b->stream));
     h.block = nullptr;
