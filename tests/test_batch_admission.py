@@ -1,5 +1,6 @@
 """Admitting and removing a scenario beside many resident ones: the strips are
-chosen anew each time, in a time that does not grow with the residents."""
+chosen anew each time, in a time that does not grow with the residents, and the
+heights of all of them reach the device at once."""
 import time
 
 import numpy as np
@@ -32,6 +33,23 @@ def test_cost_does_not_grow_with_the_residents(sw2d_mod):
                     ids.append(_add(sw2d_mod, b))
                 best[residents] = min(best.get(residents, 1.0), time.perf_counter() - t)
     assert best[900] < 1.35 * best[30], best
+
+
+def test_changed_heights_reach_all_residents_in_one_copy(sw2d_mod):
+    """Two large scenarios leave and the others' height changes: 20 times as long for
+    900 residents as for 20 with a copy for each."""
+    best = {}
+    for residents in (20, 900):
+        with sw2d_mod.Batch(max_scenarios=1024) as b:
+            for _ in range(residents):
+                _add(sw2d_mod, b)
+            for _ in range(7):
+                large = [_add(sw2d_mod, b, side=700) for _ in range(2)]
+                t = time.perf_counter()
+                for sid in large:
+                    b.remove(sid)
+                best[residents] = min(best.get(residents, 1.0), time.perf_counter() - t)
+    assert best[900] < 6.0 * best[20], best
 
 
 def test_every_resident_takes_the_new_heights(sw2d_mod):
