@@ -58,6 +58,7 @@ BATCH_STRIPS = (0, 64, 96)
 BATCH_CLASS = "batch"
 STEPS_PER_LAUNCH = (1, 24, 48, 96)  # fixed time step: iterations per launch tried by tune_fixed
 FIXED_VARIANTS = (0, 2)
+PIPE_MIN_STRIP = 8  # rows of the shortest strip that sw2d_create takes for several iterations per launch
 
 
 def fixed_class(rows: int, cols: int) -> str:
@@ -209,10 +210,19 @@ def tune_fixed(rows: int, cols: int, device: int = 0, cache: Optional[Cache] = N
     return entry
 
 
+def pipelined_strip(rows: int, strip_h: int) -> bool:
+    """Whether strips of strip_h rows can take several iterations per launch: the
+    shortest of them (the rows are split evenly) has PIPE_MIN_STRIP rows."""
+    strips = -(-rows // strip_h) if strip_h > 0 else 1
+    return strips == 1 or rows // strips >= PIPE_MIN_STRIP
+
+
 def apply(cfg, cache: Optional[Cache] = None, device: int = 0):
     """Fills cfg.strip_h / cfg.variant from the cache (FP32 only), and under
     the fixed time step cfg.steps_per_launch when tune_fixed has run for the
-    size class (its entry wins there); returns cfg."""
+    size class (its entry wins there); returns cfg.  A cached height that is too
+    short for several iterations per launch -- tune() times one launch per
+    iteration -- is left to the library where the fixed step may take several."""
     import sw2d
     if cfg.precision != sw2d.PREC_F32:
         return cfg
@@ -222,14 +232,14 @@ def apply(cfg, cache: Optional[Cache] = None, device: int = 0):
     if cfg.dt_mode == sw2d.DT_FIXED:
         fixed = c.get(gpu, fixed_class(cfg.rows, cfg.cols))
         if fixed:
-            cfg.strip_h = int(fixed["strip_h"])
-            cfg.variant = int(fixed["variant"])
             if cfg.steps_per_launch == 0:
                 cfg.steps_per_launch = int(fixed["steps_per_launch"])
-            return cfg
+            hit = fixed
     if hit:
         cfg.strip_h = int(hit["strip_h"])
         cfg.variant = int(hit["variant"])
+        if cfg.dt_mode == sw2d.DT_FIXED and cfg.steps_per_launch != 1 and not pipelined_strip(cfg.rows, cfg.strip_h):
+            cfg.strip_h = 0
     return cfg
 
 
