@@ -250,7 +250,10 @@ int sw2d_launch_count(sw2d_handle *h, int64_t *launches);
 
 /* One line naming the step kernel build and the decomposition the handle
  * runs, e.g. "stream_step_kernel<2,10,2> forcing=uniform strip_h=52 units=3040
- * ctas=1520 steps_per_launch=1 strip_skew=20"
+ * ctas=1520 steps_per_launch=1 strip_skew=20 form=uniform" or
+ * "step_kernel<double,16,32> ctas=1856 build=step64_kernel<16,32,512,2>": form
+ * is the forcing that the build carries (uniform, storm, sources, any; +skip:
+ * the build for short strips), build the FP64 kernel
  * (written NUL-terminated, truncated to `n` bytes).  No reference
  * counterpart: the reference's launch shape is fixed at cu:1222-1235. */
 int sw2d_describe(const sw2d_handle *h, char *buf, int32_t n);

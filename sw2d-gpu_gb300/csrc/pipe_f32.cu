@@ -8,7 +8,7 @@
 namespace sw2d {
 
 // The forms of a build: uniform rain and the storm as the build unrolls them, those
-// with the sources with the row loop not unrolled: unrolled by 2, build 0 with both
+// with the sources with the row loop not unrolled (pipe_unroll): unrolled by 2, build 0 with both
 // the storm and the sources spilled 492 bytes (412 with the sources alone), which in
 // strips of more than a few rows cost more than the pipelining saves; not unrolled
 // it spills 28 (16).  The storm alone spills 24 unrolled, 52 not (24.6 against 25.7
@@ -17,14 +17,12 @@ namespace sw2d {
 // 54.7 / 108 -> 26.6 / 51.0, both 59.9 / 120 -> 27.4 / 55.5, storm and rain factors
 // 61.7 / 134 -> 28.2 / 56.6.
 cudaError_t prepare_stream_pipe(int variant) {
+#define SW2D_PF(nw, mb, un, w, f) ((const void *)stream_pipe_kernel<nw, mb, pipe_unroll(un, f), w, f>)
 #define SW2D_P(id, nw, mb, un)                                                                         \
     if (variant == id) {                                                                               \
-        const void *k[6] = {(const void *)stream_pipe_kernel<nw, mb, un, false, kFormUniform>,         \
-                            (const void *)stream_pipe_kernel<nw, mb, un, false, kFormStorm>,           \
-                            (const void *)stream_pipe_kernel<nw, mb, 1, false, kFormSources>,          \
-                            (const void *)stream_pipe_kernel<nw, mb, 1, false, kFormAny>,              \
-                            (const void *)stream_pipe_kernel<nw, mb, un, true, kFormUniform>,          \
-                            (const void *)stream_pipe_kernel<nw, mb, 1, true, kFormAny>};              \
+        const void *k[6] = {SW2D_PF(nw, mb, un, false, kFormUniform), SW2D_PF(nw, mb, un, false, kFormStorm),      \
+                            SW2D_PF(nw, mb, un, false, kFormSources), SW2D_PF(nw, mb, un, false, kFormAny),        \
+                            SW2D_PF(nw, mb, un, true, kFormUniform), SW2D_PF(nw, mb, un, true, kFormAny)};         \
         for (const void *f : k) {                                                                      \
             cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout,    \
                                                  kStreamCarveoutPercent);                              \
@@ -34,6 +32,7 @@ cudaError_t prepare_stream_pipe(int variant) {
     }
     SW2D_STREAM_VARIANTS(SW2D_P)
 #undef SW2D_P
+#undef SW2D_PF
     return cudaErrorInvalidValue;
 }
 
@@ -70,7 +69,8 @@ cudaError_t launch_stream_pipe(int variant, int nblocks, int tiles_w, int strip_
     P.plans = plans;
     P.words = words;
     P.flags = flags;
-    const bool storm = F.rain_kind == RAIN_STORM, src = G.n_src > 0;
+    const bool rainw = S.rainw != nullptr;
+    const int form = stream_form(F.rain_kind == RAIN_STORM, G.n_src > 0, rainw);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;  // every unit resident: the waits between units end
     attr[0].val.cooperative = 1;
@@ -84,17 +84,17 @@ cudaError_t launch_stream_pipe(int variant, int nblocks, int tiles_w, int strip_
     lc.attrs = attr;
     lc.numAttrs = 1;
     if (variant == kTmaVariant) variant = 0;
-#define SW2D_PK(nw, mb, un, w, form) \
-    return cudaLaunchKernelEx(&lc, stream_pipe_kernel<nw, mb, un, w, form>, G, F, S, T, clk, ctl, slot, sh, P)
-#define SW2D_PL(id, nw, mb, un)                                            \
-    if (variant == id) {                                                   \
-        lc.blockDim = dim3(nw * 32);                                       \
-        if (S.rainw && (storm || src)) SW2D_PK(nw, mb, 1, true, kFormAny); \
-        if (S.rainw) SW2D_PK(nw, mb, un, true, kFormUniform);              \
-        if (storm && src) SW2D_PK(nw, mb, 1, false, kFormAny);             \
-        if (storm) SW2D_PK(nw, mb, un, false, kFormStorm);                 \
-        if (src) SW2D_PK(nw, mb, 1, false, kFormSources);                  \
-        SW2D_PK(nw, mb, un, false, kFormUniform);                          \
+#define SW2D_PK(nw, mb, un, w, f) \
+    return cudaLaunchKernelEx(&lc, stream_pipe_kernel<nw, mb, pipe_unroll(un, f), w, f>, G, F, S, T, clk, ctl, slot, sh, P)
+#define SW2D_PL(id, nw, mb, un)                                              \
+    if (variant == id) {                                                     \
+        lc.blockDim = dim3(nw * 32);                                         \
+        if (rainw && form == kFormAny) SW2D_PK(nw, mb, un, true, kFormAny);  \
+        if (rainw) SW2D_PK(nw, mb, un, true, kFormUniform);                  \
+        if (form == kFormAny) SW2D_PK(nw, mb, un, false, kFormAny);          \
+        if (form == kFormStorm) SW2D_PK(nw, mb, un, false, kFormStorm);      \
+        if (form == kFormSources) SW2D_PK(nw, mb, un, false, kFormSources);  \
+        SW2D_PK(nw, mb, un, false, kFormUniform);                            \
     }
     SW2D_STREAM_VARIANTS(SW2D_PL)
 #undef SW2D_PL

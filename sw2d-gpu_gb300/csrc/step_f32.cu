@@ -95,6 +95,24 @@ const char *stream_variant_name(int variant) {
     return "stream_step_kernel<?>";
 }
 
+std::string stream_build_name(int variant, int strip_h, bool storm, bool sources, bool rainw, bool pipelined,
+                              std::string *form) {
+    static const char *const names[4] = {"uniform", "storm", "sources", "any"};
+    const int f = stream_form(storm, sources, rainw);
+    *form = names[f];
+    if (variant == kTmaVariant && (pipelined || rainw || f != kFormUniform)) variant = 0;
+    if (!pipelined) {
+        if (stream_skips(variant, strip_h, f, rainw)) *form += "+skip";
+        return stream_variant_name(variant);
+    }
+#define SW2D_N(id, nw, mb, un)                                                            \
+    if (variant == id)                                                                    \
+        return "stream_pipe_kernel<" #nw "," #mb "," + std::to_string(pipe_unroll(un, f)) + ">";
+    SW2D_STREAM_VARIANTS(SW2D_N)
+#undef SW2D_N
+    return "stream_pipe_kernel<?>";
+}
+
 int stream_ctas_per_sm(int variant) {
     int n = 0;
     if (variant == kTmaVariant)
@@ -155,11 +173,8 @@ cudaError_t launch_stream_step(int variant, int nblocks, int tiles_w, int strip_
                                const GridDesc &G, const ForcingDesc &F, const StateBufs<float> &S,
                                const Thr<float> &T, Clock *clk, const Control *ctl, int slot, cudaStream_t st) {
     const StreamShape sh = stream_shape(G.rows, tiles_w, strip_h, units, false, skew);
-    // the build that carries the forcing that is set and no other
-    const bool storm = F.rain_kind == RAIN_STORM;
-    const bool src = G.n_src > 0;
-    const int form = S.rainw ? (src || storm ? kFormAny : kFormUniform)
-                             : (storm ? (src ? kFormAny : kFormStorm) : (src ? kFormSources : kFormUniform));
+    const bool rainw = S.rainw != nullptr;
+    const int form = stream_form(F.rain_kind == RAIN_STORM, G.n_src > 0, rainw);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -170,7 +185,7 @@ cudaError_t launch_stream_step(int variant, int nblocks, int tiles_w, int strip_
     lc.attrs = attr;
     lc.numAttrs = 1;
     if (variant == kTmaVariant) {
-        if (!S.rainw && form == kFormUniform) {
+        if (!rainw && form == kFormUniform) {
             TmaMaps M;
             std::memset(&M, 0, sizeof(M));
             bool ok = true;
@@ -198,19 +213,19 @@ cudaError_t launch_stream_step(int variant, int nblocks, int tiles_w, int strip_
     // (13), 78.2 / 81.4 (52); sources 17.3 / 15.5 (1), 40.2 / 39.4 (13), 93.6 / 95.1
     // (52); rain factors 14.1 / 13.4 (1), 33.2 / 33.0 (13), 39.2 / 39.6 (16), 98 / 103
     // (52).
-    if (variant == 0 && strip_h <= (form == kFormUniform && !S.rainw ? 6 : 13)) {
+    if (stream_skips(variant, strip_h, form, rainw)) {
         lc.blockDim = dim3(64);
-        if (S.rainw && form == kFormUniform) SW2D_LK(2, 10, 2, true, kFormUniform, true);
-        if (!S.rainw && form == kFormStorm) SW2D_LK(2, 10, 2, false, kFormStorm, true);
-        if (!S.rainw && form == kFormSources) SW2D_LK(2, 10, 2, false, kFormSources, true);
-        if (!S.rainw && form == kFormAny) SW2D_LK(2, 10, 2, false, kFormAny, true);
-        if (!S.rainw) SW2D_LK(2, 10, 2, false, kFormUniform, true);
+        if (rainw) SW2D_LK(2, 10, 2, true, kFormUniform, true);
+        if (form == kFormStorm) SW2D_LK(2, 10, 2, false, kFormStorm, true);
+        if (form == kFormSources) SW2D_LK(2, 10, 2, false, kFormSources, true);
+        if (form == kFormAny) SW2D_LK(2, 10, 2, false, kFormAny, true);
+        SW2D_LK(2, 10, 2, false, kFormUniform, true);
     }
 #define SW2D_L(id, nw, mb, un)                                                      \
     if (variant == id) {                                                            \
         lc.blockDim = dim3(nw * 32);                                                \
-        if (S.rainw && form == kFormAny) SW2D_LK(nw, mb, un, true, kFormAny, false); \
-        if (S.rainw) SW2D_LK(nw, mb, un, true, kFormUniform, false);                \
+        if (rainw && form == kFormAny) SW2D_LK(nw, mb, un, true, kFormAny, false);  \
+        if (rainw) SW2D_LK(nw, mb, un, true, kFormUniform, false);                  \
         if (form == kFormStorm) SW2D_LK(nw, mb, un, false, kFormStorm, false);      \
         if (form == kFormSources) SW2D_LK(nw, mb, un, false, kFormSources, false);  \
         if (form == kFormAny) SW2D_LK(nw, mb, un, false, kFormAny, false);          \

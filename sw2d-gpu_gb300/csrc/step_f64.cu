@@ -67,6 +67,15 @@ bool step64_tile_supported(int th, int tw) {
     return false;
 }
 
+std::string step64_build_name(int th, int tw, bool general) {
+    if (general) return "step64_kernel<16,32,512,2,general>";
+#define SW2D_S64(h, w, nt, mb) \
+    if (th == h && tw == w) return "step64_kernel<" #h "," #w "," #nt "," #mb ">";
+    SW2D_STEP64_TILES(SW2D_S64)
+#undef SW2D_S64
+    return "step64_kernel<?>";
+}
+
 // The smallest tile whose CTAs all have an SM to themselves; else the smallest of
 // which all are resident where two run per SM, if 16 x 32 would give more than a
 // twelfth of the SMs a second one; else 16 x 32.

@@ -1169,25 +1169,27 @@ int sw2d_launch_count(sw2d_handle *h, int64_t *launches) {
 
 int sw2d_describe(const sw2d_handle *h, char *buf, int32_t n) {
     if (!h || !buf || n <= 0) return SW2D_ERR_INVALID_ARG;
-    if (h->stream_kernel) {
-        // the forcing build the launcher picks (step_f32.cu): storm and point
-        // sources, per-cell rain factors, or neither
-        const bool gen = h->F.rain_kind == RAIN_STORM || h->G.n_src > 0;
-        if (pipe_now(h))
-            snprintf(buf, (size_t)n, "stream_pipe_kernel%s forcing=%s%s strip_h=%d units=%d ctas=%d steps_per_launch=%d",
-                     std::strchr(stream_variant_name(h->variant), '<'), gen ? "storm/sources" : "uniform",
-                     h->use_rainw ? "+rain_weights" : "", h->strip_h, h->stream_units, h->nblocks, h->pipe_k);
-        else {
-            char skew_s[32] = "";
-            if (h->strip_skew) snprintf(skew_s, sizeof(skew_s), " strip_skew=%d", h->strip_skew);
-            snprintf(buf, (size_t)n, "%s forcing=%s%s strip_h=%d units=%d ctas=%d steps_per_launch=1%s",
-                     stream_variant_name(h->variant), gen ? "storm/sources" : "uniform",
-                     h->use_rainw ? "+rain_weights" : "", h->strip_h, h->stream_units, h->nblocks, skew_s);
+    std::string line;
+    try {  // no exception crosses the C ABI
+        if (h->stream_kernel) {
+            const bool storm = h->F.rain_kind == RAIN_STORM, sources = h->G.n_src > 0, pipelined = pipe_now(h);
+            std::string form;
+            line = stream_build_name(h->variant, h->strip_h, storm, sources, h->use_rainw, pipelined, &form);
+            line += std::string(" forcing=") + (storm || sources ? "storm/sources" : "uniform") +
+                    (h->use_rainw ? "+rain_weights" : "") + " strip_h=" + std::to_string(h->strip_h) +
+                    " units=" + std::to_string(h->stream_units) + " ctas=" + std::to_string(h->nblocks) +
+                    " steps_per_launch=" + std::to_string(pipelined ? h->pipe_k : 1);
+            if (!pipelined && h->strip_skew) line += " strip_skew=" + std::to_string(h->strip_skew);
+            line += " form=" + form;
+        } else {
+            line = std::string("step_kernel<") + (is_f64(h) ? "double" : "float") + "," + std::to_string(h->tile_h) +
+                   "," + std::to_string(h->tile_w) + "> ctas=" + std::to_string(h->nblocks);
+            if (is_f64(h)) line += " build=" + step64_build_name(h->tile_h, h->tile_w, needs_general(h->cfg));
         }
+    } catch (...) {
+        return SW2D_ERR_OOM;
     }
-    else
-        snprintf(buf, (size_t)n, "step_kernel<%s,%d,%d> ctas=%d", is_f64(h) ? "double" : "float", h->tile_h,
-                 h->tile_w, h->nblocks);
+    snprintf(buf, (size_t)n, "%s", line.c_str());
     return SW2D_OK;
 }
 

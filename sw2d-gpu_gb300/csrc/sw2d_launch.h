@@ -3,6 +3,8 @@
 // FMA contraction), the FP32 set in step_f32.cu (fast math).
 #pragma once
 
+#include <string>
+
 #include "sw2d_device.cuh"
 
 namespace sw2d {
@@ -38,6 +40,7 @@ cudaError_t launch_step(int th, int tw, int nblocks, const GridDesc &G, const Fo
 // FP64 step kernel (step_f64.cu); sms: the device's SM count; gnx, gny: g n^2 per face (launch_pack_static_gn), or nullptr with a scalar n
 cudaError_t prepare_step64(int th, int tw, bool general);
 bool step64_tile_supported(int th, int tw);
+std::string step64_build_name(int th, int tw, bool general);
 bool step64_general(double ge_th, double gt_evmin, double g);  // these need the general build, which has 16 x 32 tiles
 void step64_tile(int rows, int cols, int sms, int *th, int *tw);  // the library's tile for a grid
 cudaError_t launch_step64(int th, int tw, int nblocks, int sms, const GridDesc &G, const ForcingDesc &F,
@@ -76,8 +79,11 @@ SW2D_DECLARE_LAUNCHERS(float)
 int stream_out_cols();
 int stream_variants();
 int stream_warps(int variant);
-int stream_ctas_per_sm(int variant);
-const char *stream_variant_name(int variant);  // "stream_step_kernel<warps,minB,unroll>"  // resident CTAs per SM (occupancy), 0 on error
+int stream_ctas_per_sm(int variant);  // resident CTAs per SM (occupancy), 0 on error
+const char *stream_variant_name(int variant);  // "stream_step_kernel<warps,minB,unroll>"
+// the build that runs under a forcing, and its form: "uniform", "storm", "sources" or "any", "+skip" for short strips
+std::string stream_build_name(int variant, int strip_h, bool storm, bool sources, bool rainw, bool pipelined,
+                              std::string *form);
 cudaError_t prepare_stream_step(int variant);
 // skew: percent by which strip heights fall from the first strip to the last (0 = even).
 cudaError_t launch_stream_step(int variant, int nblocks, int tiles_w, int strip_h, int units, int skew,

@@ -54,4 +54,19 @@ constexpr int kTmaVariant = 6;
 // Attributes of a build's pipelined forms (pipe_f32.cu)
 cudaError_t prepare_stream_pipe(int variant);
 
+// The form that carries the forcing that is set and, but with rain factors, no other.
+inline int stream_form(bool storm, bool sources, bool rainw) {
+    if (rainw) return storm || sources ? kFormAny : kFormUniform;
+    return storm ? (sources ? kFormAny : kFormStorm) : (sources ? kFormSources : kFormUniform);
+}
+
+// Whether strips of strip_h rows run the form's SKIP build (launch_stream_step).
+inline bool stream_skips(int variant, int strip_h, int form, bool rainw) {
+    return variant == 0 && !(rainw && form == kFormAny) && strip_h <= (form == kFormUniform && !rainw ? 6 : 13);
+}
+
+// The unrolling of a form's pipelined row loop in a build that unrolls by `un`
+// (prepare_stream_pipe).
+constexpr int pipe_unroll(int un, int form) { return form == kFormSources || form == kFormAny ? 1 : un; }
+
 }  // namespace sw2d
