@@ -149,8 +149,7 @@ __global__ void __launch_bounds__(NWARP * 32, MINB) batch_step_kernel(const Batc
                 const float rate_lo = lane == B_RAIN ? L.rr1 * S.G.sf.pct_lo : 0.f;
                 const float sum = lane == B_OUT ? A.out : (lane == B_CLAMP ? A.clamp : 0.f);
                 const double per = lane == B_CLAMP ? area : dt2 * (lane == B_OUT ? S.G.dy : area);
-                const double v = (double)sum + counted_rate(A.n_hi, (double)rate) +
-                                 counted_rate(A.n_act - A.n_hi, (double)rate_lo);
+                const double v = (double)sum + counted_rate(A.n_hi, rate) + counted_rate(A.n_act - A.n_hi, rate_lo);
                 if (v != 0.0) atomicAdd(&S.clk[slot_out].stepb[lane][ue.y % kBuckets], v * per);
             }
         }

@@ -436,6 +436,8 @@ __device__ __forceinline__ void accumulate_cmax(Clock &co, int bucket, double cm
 // A rate that n cells take.  None of them: nothing, also where the reference's
 // series formula has divided by zero (a record's own time) and the rate is infinite.
 __device__ __forceinline__ double counted_rate(int n, double rate) { return n ? (double)n * rate : 0.0; }
+// (an FP32 select costs the iteration's last warp less than one of FP64)
+__device__ __forceinline__ double counted_rate(int n, float rate) { return (double)n * (double)(n ? rate : 0.f); }
 
 __device__ __forceinline__ void accumulate_budgets(Clock &co, int bucket, const double v[B_N]) {
     for (int k = 0; k < B_N; k++)

@@ -190,11 +190,10 @@ __device__ __forceinline__ void acc_clear(StreamAcc &A) {
 // sums, with the FP32 rates the unit applied.
 __device__ __forceinline__ double acc_rain(double sum, int n_act, int n_hi, const LaunchScalars<float> &LS,
                                            const GridScalars<float> &GS) {
-    return sum + counted_rate(n_hi, (double)(LS.rr1 * GS.pct_hi)) +
-           counted_rate(n_act - n_hi, (double)(LS.rr1 * GS.pct_lo));
+    return sum + counted_rate(n_hi, LS.rr1 * GS.pct_hi) + counted_rate(n_act - n_hi, LS.rr1 * GS.pct_lo);
 }
 __device__ __forceinline__ double acc_ev(double sum, int n_hi, const LaunchScalars<float> &LS) {
-    return sum + counted_rate(n_hi, (double)LS.ev1);
+    return sum + counted_rate(n_hi, LS.ev1);
 }
 
 // Advances column tile `ct`, rows r0 .. r1-1 (a strip) of the
