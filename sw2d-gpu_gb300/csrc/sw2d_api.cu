@@ -331,8 +331,9 @@ int row_cost(long long warps_per_sm) { return warps_per_sm <= 8 ? 100 : (warps_p
 // that does not fill the GPU is cut into short strips (more warm-up rows in
 // all, but on warps that would otherwise be idle), down to one row.  us per
 // iteration, strips of 16 rows against the choice: 96 x 128 25.1 -> 12.7,
-// 256 x 256 25.3 -> 14.9, 512 x 512 24.3 -> 18.9.  0 when no height fits one
-// wave.
+// 256 x 256 25.3 -> 14.9, 512 x 512 24.3 -> 18.9.  That is for a handle with the
+// GPU to itself: 8 handles of 512 x 512 at once take 48.6 us with strips of 16 rows
+// and 62.6 with these (sw2d.h says so).  0 when no height fits one wave.
 int one_wave_strip(int rows, int tiles_w, long long sms, int ctas_per_sm, int warps, int least) {
     const long long tw = tiles_w > 0 ? tiles_w : 1, nw = warps;
     long long best = 0;
