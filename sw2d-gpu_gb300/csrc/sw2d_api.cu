@@ -510,8 +510,8 @@ int sw2d_create(const sw2d_config *cfg, sw2d_handle **out) {
             // strips split the rows evenly: the shortest has rows / strips rows
             const bool tall = strips == 1 || (strips > 1 && cfg->rows / strips >= stream_pipe_min_strip());
             // the library's choice: pipelined where one wave holds the grid in
-            // short strips (measured on GB300: 1.12-1.30x faster than one launch
-            // per iteration up to 1024^2, whose iterations are mostly the
+            // short strips (measured on GB300: 1.11-1.22x faster than one launch
+            // per iteration up to 1500^2, whose iterations are mostly the
             // grid-wide drain; about even with 52-row strips at 2048^2, slower
             // with the long strips one wave needs beyond)
             const bool worth = cfg->steps_per_launch > 1 || psh <= kAutoPipeMaxStrip;
@@ -904,8 +904,8 @@ namespace {
 // Brings the pages of a large output buffer in before a copy fills it, by a few
 // threads: a fresh buffer (an array just allocated by the caller) takes a page
 // fault per page, one after the other, when the copy first touches it -- 8192 x
-// 8192 float64 20.9 ms against 3.2 into a buffer in use, and 9.5 this way; 3000 x
-// 3000 4.1 and 2.7.  A buffer whose sampled pages are resident is left alone, and
+// 8192 float64 20.9 ms against 3.2 into a buffer in use, and 8.7 this way; 3000 x
+// 3000 4.1 and 2.6.  A buffer whose sampled pages are resident is left alone, and
 // so is one whose sampled pages cannot be written or whose system does not say
 // (MADV_POPULATE_WRITE): the copy then goes as it always did.  Only the first
 // byte of each page is written, which the copy overwrites.

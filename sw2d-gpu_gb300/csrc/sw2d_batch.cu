@@ -265,7 +265,9 @@ int choose_strips(sw2d_batch *b) {
     // a common height has to be clearly better than the rule: the estimate is
     // good to about 10 % (a mix of heights fills the queue's tail better than
     // it says: 24 scenarios of 128 .. 1024 run in 160 us under the rule, 170
-    // at 48 rows and 189 at 96, estimated 164, 162 and 161)
+    // at 48 rows and 189 at 96, estimated 164, 162 and 161).  With that margin none of
+    // 49 ensembles of 1 to 200 scenarios of 64 .. 1024 cells a side ran slower than
+    // under the rule's heights and a queue alone: 0.40 to 1.00 of the time.
     double best = 0.93 * iteration_length(count, warps, b->sms, b->done);
     int best_sh = 0, tallest = 0;  // grid to cut at a common height
     for (const StripClass &k : b->classes)

@@ -4,11 +4,13 @@
 // Each scenario keeps its own state, static fields, forcing, CFL time step
 // and clock (three rotating slots, as a single-scenario handle).  The work of
 // one launch is the list of (scenario, column tile, row strip) units of every
-// scenario in the batch; a fixed grid of CTAs pulls units from a queue head
-// (one atomic per unit), so scenarios of 64 x 64 and 2048 x 2048 cells share
-// the GPU without load imbalance.  A scenario's units take a ticket when they
-// finish; the last one finalises that scenario's clock slot (time, budgets,
-// CFL bound, the plan of its next iteration) -- no warp ever waits.
+// scenario in the batch, the longest first; each warp of a fixed grid of CTAs
+// starts on the unit of its own index and pulls further ones from a queue head
+// (one atomic each), so scenarios of 64 x 64 and 2048 x 2048 cells share the GPU
+// without load imbalance.  A scenario's units take a ticket when they finish; the
+// last one finalises that scenario's clock slot (time, CFL bound, the plan of its
+// next iteration), whose budgets the first one of the next launch folds -- no warp
+// ever waits.
 //
 // The unit table, its length and the scenario descriptors live in device
 // memory, so the CUDA graph of launches stays valid while scenarios are

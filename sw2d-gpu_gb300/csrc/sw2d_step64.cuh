@@ -30,8 +30,8 @@
 //   * rain and evaporation are counted per cell and multiplied once per CTA
 //     where they are uniform; sums that are zero in a whole warp are skipped.
 //
-// The last scaling differs from the unscaled expression only where a product
-// leaves the normal range (below 1e-300).
+// The scaled products differ from the unscaled ones only where one of them leaves the
+// normal range: below 1e-300, or above 4e307 (a quarter of the largest number).
 #pragma once
 
 #include "sw2d_device.cuh"

@@ -50,8 +50,8 @@ def wave_strips(rows: int, cols: int, sms: int = 152, waves=(1, 2, 3, 4), warps_
 
 
 BATCH_VARIANTS = (0, 1, 2)
-# rows per warp for every scenario of a batch (0: by scenario size, 16/32/64
-# rows); taller strips repeat fewer warm-up rows, which pays on a large
+# rows per warp for every scenario of a batch (0: the library's choice for the
+# scenarios resident); taller strips repeat fewer warm-up rows, which pays on a large
 # ensemble (measured on GB300, 64 scenarios of 128-1024 cells a side: 4.85e10
 # cell-updates/s by size, 4.98e10 with 64 rows, 5.02e10 with 96)
 BATCH_STRIPS = (0, 64, 96)
