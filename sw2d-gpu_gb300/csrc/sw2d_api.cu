@@ -870,6 +870,9 @@ int sw2d_advance(sw2d_handle *h, int64_t max_steps, double t_end, int64_t *steps
                 int rc = capture_graph(h);
                 if (rc) return rc;
             }
+            // the graph starts from clock slot 0; pipelined launches before it may have
+            // left the state in another
+            for (; h->launches % 3 != 0; h->launches++, h->kernels++) CK(h, launch_one(h, (int)(h->launches % 3)));
             CK(h, cudaGraphLaunch(h->graph, h->stream));
             h->launches += kChunk;
             h->kernels += kChunk;
