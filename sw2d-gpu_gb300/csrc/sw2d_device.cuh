@@ -201,7 +201,7 @@ __device__ inline double compat_series(const double *v, int n, double dtv, doubl
     if (t <= 1.00) return v[0] * t;
     int it = (int)(t / dtv);
     int a = it < n ? it : n - 1;
-    int b = it + 1 < n ? it + 1 : n - 1;
+    int b = it < n - 1 ? it + 1 : n - 1;  // (it is INT_MAX where t / dtv is beyond it)
     return v[a] + (v[b] - v[a]) / (dtv * __dsub_rn(t, __dmul_rn(dtv, (double)it)));
 }
 
@@ -240,7 +240,7 @@ __device__ inline double source_rate(const ForcingDesc &F, int n_src, int s, dou
     } else {
         int it = (int)d_div(t, F.dtoq);
         int a = it < F.n_qrec ? it : F.n_qrec - 1;
-        int b = it + 1 < F.n_qrec ? it + 1 : F.n_qrec - 1;
+        int b = it < F.n_qrec - 1 ? it + 1 : F.n_qrec - 1;  // as in compat_series
         double qa = F.src_q[(size_t)a * n_src + s];
         double qb = F.src_q[(size_t)b * n_src + s];
         q = qa + d_div(qb - qa, F.dtoq * __dsub_rn(t, __dmul_rn(F.dtoq, (double)it)));
