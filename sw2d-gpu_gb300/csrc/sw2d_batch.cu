@@ -74,7 +74,7 @@ struct sw2d_batch {
     size_t stage_elems = 0;
     double *d_partial = nullptr;
     double *h_partial = nullptr;  // pinned
-    Clock *h_clk = nullptr;       // pinned
+    Clock *h_clk = nullptr;       // pinned, three
     std::vector<HostScenario> scen;
     std::vector<int2> units;
     // the resident scenarios: slots in ascending order, and their classes; room for
@@ -448,7 +448,7 @@ int sw2d_batch_create(const sw2d_batch_config *cfg, sw2d_batch **out) {
         return bail(SW2D_ERR_OOM);
     if (cudaMallocHost((void **)&b->h_status, (size_t)cfg->max_scenarios * sizeof(ScenarioStatus)) != cudaSuccess ||
         cudaMallocHost((void **)&b->h_partial, kVolumeBlocks * sizeof(double)) != cudaSuccess ||
-        cudaMallocHost((void **)&b->h_clk, sizeof(Clock)) != cudaSuccess)
+        cudaMallocHost((void **)&b->h_clk, 3 * sizeof(Clock)) != cudaSuccess)
         return bail(SW2D_ERR_OOM);
     cudaMemset(b->d_hdr, 0, sizeof(BatchHeader));
     cudaMemset(b->d_scen, 0, (size_t)cfg->max_scenarios * sizeof(ScenarioDev));
@@ -742,13 +742,32 @@ int sw2d_batch_poll(sw2d_batch *b, int32_t *ids, int32_t *running, double *t, in
     return SW2D_OK;
 }
 
+// The scenario's current clock into *b->h_clk; waits.
 static int read_current_clock(sw2d_batch *b, const HostScenario &h) {
     const int cur = (int)(b->launches % 3);
-    // the last launch left its budgets to fold (a fold happens once)
-    fold_kernel<<<1, 32, 0, b->stream>>>(h.dev.clk, cur, (cur + 2) % 3);
-    BCK(b, cudaGetLastError());
     BCK(b, cudaMemcpyAsync(b->h_clk, h.dev.clk + cur, sizeof(Clock), cudaMemcpyDeviceToHost, b->stream));
     BCK(b, cudaStreamSynchronize(b->stream));
+    return SW2D_OK;
+}
+
+// The same with its budgets, which the last launch leaves for the next one to fold:
+// folded here from the copies of the clock slots, in fold_slot_warp's order (a fold
+// kernel before the copy took 11 us of each read).
+static int read_current_budgets(sw2d_batch *b, const HostScenario &h, Clock *out) {
+    const int cur = (int)(b->launches % 3);
+    BCK(b, cudaMemcpyAsync(b->h_clk, h.dev.clk, 3 * sizeof(Clock), cudaMemcpyDeviceToHost, b->stream));
+    BCK(b, cudaStreamSynchronize(b->stream));
+    Clock &c = *out;
+    c = b->h_clk[cur];
+    if (!c.fold_pending) return SW2D_OK;
+    for (int k = 0; k < B_N; k++) {
+        double v[kBuckets];
+        for (int q = 0; q < kBuckets; q++) v[q] = c.stepb[k][q];
+        for (int o = kBuckets / 2; o > 0; o >>= 1)
+            for (int q = 0; q < o; q++) v[q] += v[q + o];
+        c.step[k] = v[0];
+    }
+    fold_totals(b->h_clk[(cur + 2) % 3], c);
     return SW2D_OK;
 }
 
@@ -781,9 +800,9 @@ int sw2d_batch_get_budget(sw2d_batch *b, int32_t id, sw2d_budget *out) {
     if (!b || !out || id < 0 || id >= (int)b->scen.size() || !b->scen[id].active)
         return bfail(b, SW2D_ERR_INVALID_ARG, "bad scenario id");
     const HostScenario &h = b->scen[id];
-    int rc = read_current_clock(b, h);
+    Clock k;
+    int rc = read_current_budgets(b, h, &k);
     if (rc) return rc;
-    const Clock k = *b->h_clk;
     double vol = 0.0;
     rc = scenario_volume(b, h, k.buf, &vol);
     if (rc) return rc;

@@ -399,7 +399,7 @@ __device__ inline void clear_slot_accumulators_warp(const int lane, Clock &c) {
     }
 }
 
-__device__ inline void fold_totals(const Clock &ci, Clock &co) {
+__host__ __device__ inline void fold_totals(const Clock &ci, Clock &co) {
     for (int k = 0; k < B_N; k++) {  // Kahan: running total += previous iteration's sum
         double s = ci.tot_s[k], c = ci.tot_c[k];
         double y = ci.step[k] - c;
