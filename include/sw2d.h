@@ -304,7 +304,8 @@ int sw2d_batch_add(sw2d_batch *b, const sw2d_config *cfg, const double *z, const
                    const double *depth, int32_t rain_kind, const double *rain, int32_t n_rain, double rain_dt,
                    double t_end, int32_t *id);
 /* Enqueues `launches` iterations of every admitted scenario (finished ones
- * idle).  With running != NULL, waits and returns how many still run. */
+ * idle).  With running != NULL, waits and returns how many still run; the next
+ * call then suits its work split to those (as after sw2d_batch_poll). */
 int sw2d_batch_advance(sw2d_batch *b, int32_t launches, int32_t *running);
 /* Status of the admitted scenarios (waits for queued work): up to cap
  * entries of id, running flag, simulated time and iterations; *n = count. */

@@ -52,7 +52,8 @@ struct HostScenario {
     int pitch = 0, tiles_w = 0;
     int rule_strip = 0;    // strip height by scenario size, or the caller's
     bool own_strip = false;  // rule_strip is the caller's
-    int strip_h = 0, nunits = 0;  // in use (choose_strips)
+    int strip_h = 0, nunits = 0;  // in use (plan_units)
+    bool finished = false;   // its status said so; it has one unit, which carries its clock on
     bool raster = false;
     void *block = nullptr;
     size_t bytes = 0;
@@ -80,7 +81,9 @@ struct sw2d_batch {
     // the resident scenarios: slots in ascending order, and their classes; room for
     // choosing their strips
     std::vector<int> resident;
-    std::vector<StripClass> classes;
+    std::vector<StripClass> classes;  // of those that run
+    int finished = 0;                 // resident scenarios that do not
+    bool stale = false;               // scenarios have finished since the last plan_units
     std::vector<std::pair<int, int>> order;
     std::vector<std::pair<long long, long long>> done;
     std::vector<int3> strips;
@@ -275,7 +278,7 @@ int choose_strips(sw2d_batch *b) {
     for (int sh : kHeights) {
         if (100.0 * (std::min(sh, tallest) + 7) >= best) break;  // nor can the ones above
         strip_counts(b, sh, count);
-        if (count.strips > b->cfg.max_units || 120.0 * (double)count.steps >= best * (double)warps) continue;
+        if (count.strips + b->finished > b->cfg.max_units || 120.0 * (double)count.steps >= best * (double)warps) continue;
         const double len = iteration_length(count, warps, b->sms, b->done);
         if (len < best) best = len, best_sh = sh;
     }
@@ -295,7 +298,7 @@ void count_scenario(sw2d_batch *b, const HostScenario &h, int sign) {
 // on the host.  Sending them is send_units.
 int plan_units(sw2d_batch *b) {
     long long rule = 0;
-    for (const StripClass &k : b->classes) rule += k.tiles * ((k.rows + k.rule - 1) / k.rule);
+    for (int s : b->resident) rule += units_of(b->scen[s], b->scen[s].rule_strip);
     if (rule > b->cfg.max_units) return bfail(b, SW2D_ERR_INVALID_ARG, "unit table full: raise max_units");
     try {  // no exception crosses the C ABI
         const int common = choose_strips(b);
@@ -303,10 +306,14 @@ int plan_units(sw2d_batch *b) {
         size_t total = 0;
         for (int s : b->resident) {
             HostScenario &h = b->scen[s];
-            h.strip_h = h.own_strip || common == 0 ? h.rule_strip : common;
-            h.nunits = units_of(h, h.strip_h);
+            if (h.finished) {
+                h.nunits = 1;
+            } else {
+                h.strip_h = h.own_strip || common == 0 ? h.rule_strip : common;
+                h.nunits = units_of(h, h.strip_h);
+            }
             total += h.nunits;
-            b->order.push_back({-std::min(h.strip_h, h.cfg.rows), s});
+            b->order.push_back({h.finished ? 0 : -std::min(h.strip_h, h.cfg.rows), s});
         }
         // the longest strips first: a launch ends when its last unit does, and a
         // 64-row strip that the queue hands out last leaves the other warps idle
@@ -321,6 +328,7 @@ int plan_units(sw2d_batch *b) {
     } catch (...) {
         return bfail(b, SW2D_ERR_OOM, "host memory for the unit table");
     }
+    b->stale = false;
     return SW2D_OK;
 }
 
@@ -357,6 +365,26 @@ int send_units(sw2d_batch *b) {
     return SW2D_OK;
 }
 
+// Waits for the statuses and notes the scenarios that have finished: an end time does
+// not move, so they never run again. The next advance cuts the others for themselves
+// and gives these one unit each. us per launch of 300 scenarios of 64 .. 128 cells a
+// side, 90 % of them finished: 77 with the heights chosen for all of them, 48.8 with
+// the size rule, 27 this way.
+int read_status(sw2d_batch *b) {
+    BCK(b, cudaMemcpyAsync(b->h_status, b->d_status, b->scen.size() * sizeof(ScenarioStatus), cudaMemcpyDeviceToHost,
+                           b->stream));
+    BCK(b, cudaStreamSynchronize(b->stream));
+    for (int s : b->resident) {
+        HostScenario &h = b->scen[s];
+        if (h.finished || b->h_status[s].running) continue;
+        count_scenario(b, h, -1);  // its class exists: nothing is allocated
+        h.finished = true;
+        b->finished++;
+        b->stale = true;
+    }
+    return SW2D_OK;
+}
+
 // The lists of resident scenarios with slot s put in or taken out.
 int list_scenario(sw2d_batch *b, int s, bool in) {
     try {
@@ -364,7 +392,8 @@ int list_scenario(sw2d_batch *b, int s, bool in) {
             count_scenario(b, b->scen[s], 1);
             b->resident.insert(std::lower_bound(b->resident.begin(), b->resident.end(), s), s);
         } else {
-            count_scenario(b, b->scen[s], -1);
+            if (b->scen[s].finished) b->finished--;
+            else count_scenario(b, b->scen[s], -1);
             b->resident.erase(std::lower_bound(b->resident.begin(), b->resident.end(), s));
         }
     } catch (...) {
@@ -691,6 +720,11 @@ int sw2d_batch_add(sw2d_batch *b, const sw2d_config *cfg, const double *z, const
 int sw2d_batch_advance(sw2d_batch *b, int32_t launches, int32_t *running) {
     if (!b || launches < 0) return bfail(b, SW2D_ERR_INVALID_ARG, "bad arguments");
     BCK(b, cudaSetDevice(b->cfg.device));
+    if (b->stale && launches > 0) {
+        int rc = plan_units(b);
+        if (!rc) rc = send_units(b);
+        if (rc) return rc;
+    }
     int left = launches;
     while (left > 0) {
         const int parity = (int)(b->launches % 3);
@@ -709,13 +743,9 @@ int sw2d_batch_advance(sw2d_batch *b, int32_t launches, int32_t *running) {
         }
     }
     if (running) {
-        BCK(b, cudaMemcpyAsync(b->h_status, b->d_status, b->scen.size() * sizeof(ScenarioStatus),
-                               cudaMemcpyDeviceToHost, b->stream));
-        BCK(b, cudaStreamSynchronize(b->stream));
-        int n = 0;
-        for (size_t s = 0; s < b->scen.size(); s++)
-            if (b->scen[s].active && b->h_status[s].running) n++;
-        *running = n;
+        int rc = read_status(b);
+        if (rc) return rc;
+        *running = (int)b->resident.size() - b->finished;
     }
     return SW2D_OK;
 }
@@ -723,14 +753,12 @@ int sw2d_batch_advance(sw2d_batch *b, int32_t launches, int32_t *running) {
 int sw2d_batch_poll(sw2d_batch *b, int32_t *ids, int32_t *running, double *t, int64_t *steps, int32_t cap,
                     int32_t *n) {
     if (!b || !n) return bfail(b, SW2D_ERR_INVALID_ARG, "null argument");
-    BCK(b, cudaMemcpyAsync(b->h_status, b->d_status, b->scen.size() * sizeof(ScenarioStatus), cudaMemcpyDeviceToHost,
-                           b->stream));
-    BCK(b, cudaStreamSynchronize(b->stream));
+    int rc = read_status(b);
+    if (rc) return rc;
     int k = 0;
-    for (size_t s = 0; s < b->scen.size(); s++) {
-        if (!b->scen[s].active) continue;
+    for (int s : b->resident) {
         if (k < cap) {
-            if (ids) ids[k] = (int32_t)s;
+            if (ids) ids[k] = s;
             if (running) running[k] = b->h_status[s].running;
             if (t) t[k] = b->h_status[s].t;
             if (steps) steps[k] = b->h_status[s].steps;
