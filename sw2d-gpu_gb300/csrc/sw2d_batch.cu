@@ -82,6 +82,7 @@ struct sw2d_batch {
     // choosing their strips
     std::vector<int> resident;
     std::vector<StripClass> classes;  // of those that run
+    long long rule_units = 0;         // units of all residents by the size rule
     int finished = 0;                 // resident scenarios that do not
     bool stale = false;               // scenarios have finished since the last plan_units
     std::vector<std::pair<int, int>> order;
@@ -297,9 +298,7 @@ void count_scenario(sw2d_batch *b, const HostScenario &h, int sign) {
 // The strips and the unit table of the resident scenarios (those in b->resident)
 // on the host.  Sending them is send_units.
 int plan_units(sw2d_batch *b) {
-    long long rule = 0;
-    for (int s : b->resident) rule += units_of(b->scen[s], b->scen[s].rule_strip);
-    if (rule > b->cfg.max_units) return bfail(b, SW2D_ERR_INVALID_ARG, "unit table full: raise max_units");
+    if (b->rule_units > b->cfg.max_units) return bfail(b, SW2D_ERR_INVALID_ARG, "unit table full: raise max_units");
     try {  // no exception crosses the C ABI
         const int common = choose_strips(b);
         b->order.clear();
@@ -385,22 +384,22 @@ int read_status(sw2d_batch *b) {
     return SW2D_OK;
 }
 
-// The lists of resident scenarios with slot s put in or taken out.
-int list_scenario(sw2d_batch *b, int s, bool in) {
-    try {
-        if (in) {
-            count_scenario(b, b->scen[s], 1);
-            b->resident.insert(std::lower_bound(b->resident.begin(), b->resident.end(), s), s);
-        } else {
-            if (b->scen[s].finished) b->finished--;
-            else count_scenario(b, b->scen[s], -1);
-            b->resident.erase(std::lower_bound(b->resident.begin(), b->resident.end(), s));
-        }
-    } catch (...) {
-        return bfail(b, SW2D_ERR_OOM, "host memory for the scenario lists");
+// The lists of resident scenarios with slot s put in or taken out (they have room for
+// every slot: nothing is allocated).
+void list_scenario(sw2d_batch *b, int s, bool in) {
+    HostScenario &h = b->scen[s];
+    const auto at = std::lower_bound(b->resident.begin(), b->resident.end(), s);
+    if (in) {
+        count_scenario(b, h, 1);
+        b->resident.insert(at, s);
+    } else {
+        if (h.finished) b->finished--;
+        else count_scenario(b, h, -1);
+        b->resident.erase(at);
     }
-    b->scen[s].active = in;
-    return SW2D_OK;
+    const int units = units_of(h, h.rule_strip);
+    b->rule_units += in ? units : -units;
+    h.active = in;
 }
 
 // rows per warp: the scenario's own setting (autotuned), the batch's, or by size
@@ -485,6 +484,8 @@ int sw2d_batch_create(const sw2d_batch_config *cfg, sw2d_batch **out) {
     try {
         b->scen.resize(cfg->max_scenarios);
         b->strips.resize(cfg->max_scenarios);
+        b->resident.reserve(cfg->max_scenarios);
+        b->classes.reserve(cfg->max_scenarios);
     } catch (...) {
         return bail(SW2D_ERR_OOM);
     }
@@ -683,8 +684,9 @@ int sw2d_batch_add(sw2d_batch *b, const sw2d_config *cfg, const double *z, const
     if (vrc) return vrc;
     d.status = b->d_status + slot;
     d.tiles_w = h.tiles_w;
-    int rc = list_scenario(b, slot, true);
-    if (!rc && (rc = plan_units(b)) != SW2D_OK) list_scenario(b, slot, false);
+    list_scenario(b, slot, true);
+    int rc = plan_units(b);
+    if (rc) list_scenario(b, slot, false);
     d.strip_h = h.strip_h;
     d.nunits = h.nunits;
     auto send = [&]() -> int {
@@ -856,8 +858,8 @@ int sw2d_batch_remove(sw2d_batch *b, int32_t id) {
     if (!b || id < 0 || id >= (int)b->scen.size() || !b->scen[id].active)
         return bfail(b, SW2D_ERR_INVALID_ARG, "bad scenario id");
     HostScenario &h = b->scen[id];
-    int rc = list_scenario(b, id, false);
-    if (!rc) rc = plan_units(b);
+    list_scenario(b, id, false);
+    int rc = plan_units(b);
     if (!rc) rc = send_units(b);  // the next launch no longer sees the scenario
     if (rc) return rc;
     BCK(b, cudaFreeAsync(h.block, b->stream));
